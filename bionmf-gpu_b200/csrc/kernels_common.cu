@@ -246,48 +246,114 @@ __global__ void k_conv_compare(const uint32_t *__restrict__ labels, uint32_t *__
 // ---------------------------------------------------------------------------
 // FP64 objectives over V (n x m, ld ldv) and W (n x kp), H (m x kp):
 // out[0] = ||V||^2, out[1] = ||V - WH||^2, out[2] = KL(V || WH).
-__global__ void k_objective(const float *__restrict__ V, size_t ldv, const float *__restrict__ W,
-                            const float *__restrict__ H, uint32_t n, uint32_t m, uint32_t kp, uint32_t k,
-                            double *__restrict__ part, double *__restrict__ out, uint32_t *__restrict__ ticket)
+//
+// Bound by the FP64 pipe (64 FMA per cycle and SM): k multiply-adds an element
+// for WH and, for the divergence, a division and a logarithm (about 45 more).
+// A CTA takes 64 x 64 tiles of V in turn; 32 columns at a time of the tile's
+// rows of W and H are converted to FP64 once, in shared memory, and each
+// thread forms 4 x 4 elements of WH from them, so an element costs half a
+// shared load per multiply-add and no conversion.  (One thread per element
+// with both rows read and converted from global memory was bound by the
+// conversions and by the division of the element index: 1344 us for
+// 12007 x 1501 at k = 20.)  WHAT selects the
+// sums: OBJ_DOTS leaves out the division and the logarithm.  Thread, CTA and
+// grid sums have fixed orders.
+enum { OBJ_DOTS = 1, OBJ_KL = 2 };
+constexpr int OBJ_T = 64;    // tile edge
+constexpr int OBJ_KC = 32;   // rank columns per shared-memory chunk
+
+template <int WHAT>
+__global__ void __launch_bounds__(256) k_objective(const float *__restrict__ V, size_t ldv, const float *__restrict__ W,
+                                                   const float *__restrict__ H, uint32_t n, uint32_t m, uint32_t kp,
+                                                   uint32_t k, double *__restrict__ part, double *__restrict__ out,
+                                                   uint32_t *__restrict__ ticket)
 {
-    __shared__ double red[3][256];
+    __shared__ __align__(16) double sW[OBJ_KC][OBJ_T + 2];   // [column][row]; 16-byte rows for the paired loads
+    __shared__ __align__(16) double sH[OBJ_KC][OBJ_T + 2];
+    __shared__ double red[3][8];
     __shared__ bool is_last;
+    uint32_t const tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    uint32_t const tcols = (m + OBJ_T - 1) / OBJ_T, trows = (n + OBJ_T - 1) / OBJ_T;
+    uint64_t const tiles = (uint64_t)tcols * trows;
     double sv = 0.0, sd = 0.0, kl = 0.0;
-    size_t const total = (size_t)n * m;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        uint32_t const i = (uint32_t)(e / m), j = (uint32_t)(e % m);
-        const float *w = W + (size_t)i * kp;
-        const float *h = H + (size_t)j * kp;
-        double wh = 0.0;
-        for (uint32_t c = 0; c < k; c++)
-            wh += (double)w[c] * (double)h[c];
-        double const v = V[(size_t)i * ldv + j];
-        sv += v * v;
-        sd += (v - wh) * (v - wh);
-        kl += (v > 0.0 ? v * log(v / wh) : 0.0) - v + wh;
+    for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        uint32_t const i0 = (uint32_t)(t / tcols) * OBJ_T, j0 = (uint32_t)(t % tcols) * OBJ_T;
+        // this thread's 4 x 4 elements of V; the leading dimension is a multiple of 32, so a
+        // float4 starting below m lies in its row
+        float4 v[4];
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            uint32_t const i = i0 + ty * 4 + p, j = j0 + tx * 4;
+            v[p] = (i < n && j < m) ? __ldcs(reinterpret_cast<const float4 *>(V + (size_t)i * ldv + j))
+                                    : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        double wh[4][4] = {};
+        for (uint32_t c0 = 0; c0 < k; c0 += OBJ_KC) {
+            uint32_t const kc = min((uint32_t)OBJ_KC, k - c0);
+            __syncthreads();   // the previous chunk's readers are done
+            for (uint32_t e = tid; e < OBJ_T * kc; e += 256) {
+                uint32_t const r = e / kc, c = e % kc;
+                sW[c][r] = i0 + r < n ? (double)W[(size_t)(i0 + r) * kp + c0 + c] : 0.0;
+                sH[c][r] = j0 + r < m ? (double)H[(size_t)(j0 + r) * kp + c0 + c] : 0.0;
+            }
+            __syncthreads();
+#pragma unroll 4
+            for (uint32_t c = 0; c < kc; c++) {
+                double2 const wa = *reinterpret_cast<const double2 *>(&sW[c][ty * 4]);
+                double2 const wb = *reinterpret_cast<const double2 *>(&sW[c][ty * 4 + 2]);
+                double2 const ha = *reinterpret_cast<const double2 *>(&sH[c][tx * 4]);
+                double2 const hb = *reinterpret_cast<const double2 *>(&sH[c][tx * 4 + 2]);
+                double const w[4] = {wa.x, wa.y, wb.x, wb.y}, h[4] = {ha.x, ha.y, hb.x, hb.y};
+#pragma unroll
+                for (int p = 0; p < 4; p++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) wh[p][q] += w[p] * h[q];
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 4; p++) {
+            if (i0 + ty * 4 + p >= n) continue;
+            float const vs[4] = {v[p].x, v[p].y, v[p].z, v[p].w};
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if (j0 + tx * 4 + q >= m) continue;
+                double const x = (double)vs[q], y = wh[p][q];
+                if (WHAT & OBJ_DOTS) {
+                    sv += x * x;
+                    sd += (x - y) * (x - y);
+                }
+                if (WHAT & OBJ_KL) kl += (x > 0.0 ? x * log(x / y) : 0.0) - x + y;
+            }
+        }
     }
-    red[0][threadIdx.x] = sv;
-    red[1][threadIdx.x] = sd;
-    red[2][threadIdx.x] = kl;
+    double s[3] = {sv, sd, kl};
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], off);
+        if (tid % 32 == 0) red[q][tid / 32] = s[q];
+    }
     __syncthreads();
-    for (uint32_t s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            for (int q = 0; q < 3; q++) red[q][threadIdx.x] += red[q][threadIdx.x + s];
-        __syncthreads();
+    if (tid < 3) {
+        double u = 0.0;
+        for (int w = 0; w < 8; w++) u += red[tid][w];
+        part[(size_t)blockIdx.x * 3 + tid] = u;
     }
-    if (threadIdx.x < 3) part[(size_t)blockIdx.x * 3 + threadIdx.x] = red[threadIdx.x][0];
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
+    if (tid == 0) is_last = (atomicAdd(ticket, 1u) == gridDim.x - 1);
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    if (threadIdx.x < 3) {
-        double t = 0.0;
-        for (uint32_t b = 0; b < gridDim.x; b++) t += __ldcg(&part[(size_t)b * 3 + threadIdx.x]);
-        out[threadIdx.x] = t;
+    // the CTAs' sums: warp q adds sum q, lane l the CTAs l, l + 32, ... in order, then a shuffle tree
+    if (tid < 96) {
+        double u = 0.0;
+        for (uint32_t b = tid % 32; b < gridDim.x; b += 32) u += __ldcg(&part[(size_t)b * 3 + tid / 32]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) u += __shfl_xor_sync(0xffffffffu, u, off);
+        if (tid % 32 == 0) out[tid / 32] = u;
     }
-    if (threadIdx.x == 0) *ticket = 0u;
+    if (tid == 0) *ticket = 0u;
 }
 
 inline unsigned grid_for(size_t items, unsigned block, unsigned cap)
@@ -393,21 +459,34 @@ int nmfb_reset_conv(nmfb_ctx *ctx, uint32_t stop_threshold)
     return NMFB_OK;
 }
 
-int nmfb_objectives_rows(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, double out[3])
+static int objectives_rows(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, int what, double out[3])
 {
-    unsigned const grid = 4u * (unsigned)ctx->sm_count;
-    k_objective<<<grid, 256, 0, ctx->stream>>>(V, ctx->ldv, W, ctx->dH, rows, ctx->m, ctx->kp, ctx->k, ctx->dObj,
-                                              ctx->dObj + 3 * 1024, ctx->dObjTicket);
+    // four CTAs per SM by registers and shared memory; dObj holds the partials of 1024
+    uint64_t const tiles = (uint64_t)((ctx->m + OBJ_T - 1) / OBJ_T) * ((rows + OBJ_T - 1) / OBJ_T);
+    uint64_t grid = 4u * (uint64_t)ctx->sm_count;
+    if (grid > tiles) grid = tiles;
+    if (grid > 1024) grid = 1024;
+    auto const kern = what == OBJ_DOTS ? k_objective<OBJ_DOTS> : what == OBJ_KL ? k_objective<OBJ_KL>
+                                                                                : k_objective<OBJ_DOTS | OBJ_KL>;
+    kern<<<(unsigned)grid, 256, 0, ctx->stream>>>(V, ctx->ldv, W, ctx->dH, rows, ctx->m, ctx->kp, ctx->k, ctx->dObj,
+                                                 ctx->dObj + 3 * 1024, ctx->dObjTicket);
     NMFB_LAUNCH_CHECK(ctx);
     NMFB_CUDA_TRY(ctx, cudaMemcpyAsync(out, ctx->dObj + 3 * 1024, 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
     NMFB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     return NMFB_OK;
 }
 
+int nmfb_objectives_rows(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, double out[3])
+{
+    return objectives_rows(ctx, V, W, rows, OBJ_DOTS | OBJ_KL, out);
+}
+
 int nmfb_objectives(nmfb_ctx *ctx, double *dot_V, double *dot_VWH, double *kl)
 {
     double host[3];
-    int const rc = ctx->splan ? nmfb_stream_objectives(ctx, host) : nmfb_objectives_rows(ctx, ctx->dV, ctx->dW, ctx->n, host);
+    int const what = (dot_V || dot_VWH ? OBJ_DOTS : 0) | (kl ? OBJ_KL : 0);
+    int const rc = ctx->splan ? nmfb_stream_objectives(ctx, host)
+                              : objectives_rows(ctx, ctx->dV, ctx->dW, ctx->n, what ? what : OBJ_DOTS | OBJ_KL, host);
     if (rc) return rc;
     if (dot_V) *dot_V = host[0];
     if (dot_VWH) *dot_VWH = host[1];
