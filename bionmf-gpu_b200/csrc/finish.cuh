@@ -22,11 +22,11 @@ constexpr uint32_t FIN_RB = 32;    // rows of X per k_finish CTA
 // k_finish's launch shape for a factor of `rows` rows: KP / 4 threads per row
 // of a 32-row set, RPT row sets per CTA (each thread takes one row of each),
 // and enough CTAs to cover every 64-row block of the split copies (rows past
-// the end get zeros there).  RPT > 1 when there are few splits: more loads in
+// the end get zeros there).  RPT > 1 when there are few partials: more loads in
 // flight per thread, fewer waves of CTAs.
 template <int KP>
 constexpr int fin_threads() { return (int)FIN_RB * (KP / 4); }
-inline uint32_t fin_rpt(uint32_t nsplit) { return nsplit <= 2 ? 4u : nsplit <= 4 ? 2u : 1u; }
+inline uint32_t fin_rpt(uint32_t slots) { return slots <= 2 ? 4u : slots <= 4 ? 2u : 1u; }
 inline uint32_t fin_blocks(uint32_t rows, uint32_t rpt)
 {
     uint32_t const rows64 = (rows + 63u) / 64u * 64u;
@@ -44,7 +44,7 @@ __device__ __forceinline__ uint32_t fin_bf16x2(float first, float second)
 // Finish of a half-iteration, one CTA per FIN_RB = 32 rows of X, KP / 4 threads
 // per row (four consecutive columns each), right after the fused kernel
 // (k_fused_half, LAYOUT 0, or k_fused_bf16, LAYOUT 1):
-//   Xaux = the split partials summed in split order; X = X * Xaux / accY
+//   Xaux = the partials of its row block summed in slot order; X = X * Xaux / accY
 //   (matrix_mul_div, src/GPU_kernels.cu:1885-2058: product first, then the
 //   division, correctly rounded) with the EPS adjust when asked (kernel_adjust,
 //   :2338-2345); then X's split copies in the arm's layout (LAYOUT 0:
@@ -58,9 +58,10 @@ __device__ __forceinline__ uint32_t fin_bf16x2(float first, float second)
 //   dependent memory round trips short: the kernel is latency-bound, its traffic
 //   (the partials, X and its copies) small.
 struct FinishArgs {
-    uint32_t O, nsplit, k;
+    uint32_t O, k;
+    nmfb_tc::TileSplit ts;
     int adjust;
-    const float *part;    // [split][O][KP]
+    const float *part;    // [slot][O][KP] (TileSplit::slot)
     float *X;
     const float *accY;    // column sums of Y (KP)
     float *xhi, *xT;      // LAYOUT 0: X's split copies (the FP32 arm's SplitLayout of X's rows)
@@ -105,21 +106,25 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
         xv[r] = in[r] ? *reinterpret_cast<const float4 *>(a.X + (size_t)o[r] * KP + c0)   // independent of the partials
                       : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
-    // Xaux: each row's split partials in split order, QB splits of every row in flight
-    for (uint32_t q = 0; q < a.nsplit; q += QB) {
+    // Xaux: each row's partials in slot order, QB slots of every row in flight (the
+    // row sets of a CTA lie in one row block: BO is a multiple of FIN_RB RPT)
+    static_assert(BO % ((int)FIN_RB * RPT) == 0, "row sets of a CTA in one row block");
+    uint32_t const ob = blk * (FIN_RB * RPT) / BO;
+    uint32_t const nslot = a.ts.nslot(ob);
+    for (uint32_t q = 0; q < nslot; q += QB) {
         float4 v[RPT][QB];
 #pragma unroll
         for (int r = 0; r < RPT; r++)
 #pragma unroll
             for (int j = 0; j < QB; j++)
-                v[r][j] = (in[r] && q + j < a.nsplit)
+                v[r][j] = (in[r] && q + j < nslot)
                               ? __ldcg(reinterpret_cast<const float4 *>(a.part + (size_t)o[r] * KP + c0 + (q + j) * qs))
                               : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int r = 0; r < RPT; r++)
 #pragma unroll
             for (int j = 0; j < QB; j++)
-                if (q + j < a.nsplit) {
+                if (q + j < nslot) {
                     x[r][0] += v[r][j].x;
                     x[r][1] += v[r][j].y;
                     x[r][2] += v[r][j].z;
@@ -159,9 +164,13 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
                 }
                 size_t const e = (size_t)o[r] * KP + c0;
                 *reinterpret_cast<float4 *>(a.xhi + e) = make_float4(h[0], h[1], h[2], h[3]);
-                *reinterpret_cast<uint2 *>(a.xBl + e) = make_uint2(fin_bf16x2(l[0], l[1]), fin_bf16x2(l[2], l[3]));
-                *reinterpret_cast<uint2 *>(a.xB + e) =
-                    make_uint2(fin_bf16x2(x[r][0], x[r][1]), fin_bf16x2(x[r][2], x[r][3]));
+                if (KP == 16) {   // the FP32 lo part in place of bf16(lo) | bf16(x)
+                    *reinterpret_cast<float4 *>(reinterpret_cast<float *>(a.xBl) + e) = make_float4(l[0], l[1], l[2], l[3]);
+                } else {
+                    *reinterpret_cast<uint2 *>(a.xBl + e) = make_uint2(fin_bf16x2(l[0], l[1]), fin_bf16x2(l[2], l[3]));
+                    *reinterpret_cast<uint2 *>(a.xB + e) =
+                        make_uint2(fin_bf16x2(x[r][0], x[r][1]), fin_bf16x2(x[r][2], x[r][3]));
+                }
             }
         } else if (in[r]) {
             // hi = bf16(x), lo = bf16(x - hi), both rounded to nearest (k_split_bf16)
@@ -264,11 +273,11 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
 }
 
 // k_finish for the factor of a.O rows, with the row sets per thread that its
-// split count calls for (the block count is fin_blocks(a.O, fin_rpt(a.nsplit))).
+// partial count calls for (the block count is fin_blocks(a.O, fin_rpt(a.ts.slots))).
 template <int KP, int BR, int LAYOUT>
 void fin_launch(const FinishArgs &a, cudaStream_t s)
 {
-    uint32_t const rpt = fin_rpt(a.nsplit), nb = fin_blocks(a.O, rpt);
+    uint32_t const rpt = fin_rpt(a.ts.slots), nb = fin_blocks(a.O, rpt);
     if (rpt == 4)
         k_finish<KP, BR, LAYOUT, 4><<<nb, fin_threads<KP>(), 0, s>>>(a);
     else if (rpt == 2)

@@ -13,6 +13,58 @@ constexpr uint32_t TMEM_COLS = 512;
 constexpr int SMEM_LIMIT = 232448; // max dynamic shared memory per block on sm_100
 constexpr unsigned long long WAIT_LIMIT_NS = 1000000000ull;
 
+// How a half-iteration's tiles are dealt out.  Tile g is reduction tile g % tb
+// of row block g / tb (BO output rows); CTA b takes tiles [b tpc, (b + 1) tpc).
+// A row block's sum is then spread over the CTAs first(ob) .. last(ob); each
+// writes a partial at the end of its run and every `run` reduction tiles (a
+// chain of FP32 additions no longer than that), and k_finish adds the partials
+// in tile order: a fixed order for given sizes and SM count.
+struct TileSplit {
+    uint32_t tb, total, tpc;   // tiles per row block, of all row blocks, per CTA
+    uint32_t run;              // longest sum of tiles in one partial
+    uint32_t slots;            // most partials of a row block
+    __host__ __device__ uint32_t ctas() const { return (total + tpc - 1) / tpc; }
+    __host__ __device__ uint32_t first(uint32_t ob) const { return ob * tb / tpc; }
+    __host__ __device__ uint32_t last(uint32_t ob) const { return (ob * tb + tb - 1) / tpc; }
+    // Partial that CTA b's sum of row block ob up to reduction tile c goes to, and the
+    // number of them.  A CTA's tiles that start on a multiple of `run` (not 0) leave
+    // the slot before their first one unused; the CTA writes zeros there.
+    __host__ __device__ uint32_t slot(uint32_t ob, uint32_t b, uint32_t c) const { return c / run + (b - first(ob)); }
+    __host__ __device__ uint32_t nslot(uint32_t ob) const { return slot(ob, last(ob), tb - 1) + 1; }
+};
+
+// Equal runs of tiles for `sms` CTAs.  With few tiles per CTA the runs are made
+// longer where that saves k_finish more than it costs here: k_finish reads the
+// partials of a row eight at a time, about 0.8 tile times a batch (0.8 us).
+// Sums of 128 tiles where the partials of all O rows fit `part_rows` rows,
+// longer ones otherwise (one partial per CTA and row block always fits:
+// slots <= sms / row blocks + 3).
+inline TileSplit plan_tiles(uint32_t O, uint32_t R, uint32_t br, uint32_t sms, size_t part_rows)
+{
+    TileSplit s;
+    uint32_t const oblocks = (O + BO - 1) / BO;
+    s.tb = (R + br - 1) / br;
+    s.total = oblocks * s.tb;
+    auto const slots = [&](uint32_t tpc) {
+        uint32_t const most = (s.tb - 1) / tpc + 2;   // CTAs of a row block that starts inside a run
+        return (most < s.tb ? most : s.tb) + (s.tb - 1) / s.run;
+    };
+    s.run = 128;
+    uint32_t const even = (s.total + sms - 1) / sms;
+    s.tpc = even;
+    uint32_t best = 0xffffffffu;
+    for (uint32_t tpc = even; tpc <= even + 8 && tpc <= s.tb; tpc++) {
+        uint32_t const cost = 10 * tpc + 8 * ((slots(tpc) + 7) / 8);   // tenths of a tile time
+        if (cost < best) {
+            best = cost;
+            s.tpc = tpc;
+        }
+    }
+    while ((size_t)slots(s.tpc) * O > part_rows && s.run < s.tb) s.run *= 2;
+    s.slots = slots(s.tpc);
+    return s;
+}
+
 // PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -100,6 +152,27 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
     return true;
 }
 
+// Time limit of a polling loop: expired() is called once per fruitless poll and
+// reset() whenever the loop got on.  %globaltimer is read every 64th fruitless
+// poll only (every one for limits below 10 us): in the MMA issuer's loop a read
+// per tile costs as much as issuing MMAs.
+struct PollLimit {
+    unsigned long long limit, t0;
+    uint32_t polls, mask;
+    __device__ __forceinline__ explicit PollLimit(unsigned long long limit_ns)
+        : limit(limit_ns), t0(0), polls(0), mask(limit_ns < 10000 ? 0u : 63u)
+    {
+    }
+    __device__ __forceinline__ void reset() { polls = 0; }
+    __device__ __forceinline__ bool expired()
+    {
+        if (++polls & mask) return false;
+        unsigned long long const now = globaltimer();
+        if (polls == mask + 1) t0 = now;
+        return now - t0 > limit;
+    }
+};
+
 // Drain wait, used after a role has stopped (normally or on abort): waits for
 // a phase of asynchronous work this thread issued itself (a TMA load's
 // complete_tx, an MMA commit) to land, ignoring the abort flag, for at most
@@ -142,13 +215,68 @@ __device__ __forceinline__ void mma_drain(uint64_t *bar)
     mbar_drain(bar, 0);
 }
 
-__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t acc)
+// The MMA issuer runs as a whole warp on warp-uniform values and only the MMAs
+// and commits themselves are left to one elected lane (always the same one):
+// tcgen05.mma takes its descriptors and addresses from uniform registers, and
+// an issuer that had branched to a single lane first spent more time moving
+// operands there, one by one, than the tensor core on the MMAs (a tile's 20
+// MMAs took about 2000 cycles to issue, against 1020 to execute).
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok));
+    return ok != 0;
+}
+// Warp-wide probe and bounded wait of a phase (as mbar_wait).  Every branch of
+// the wait is on a vote, so the lanes leave it together: the .aligned tensor-
+// memory instructions that follow need a converged warp, and lanes that left a
+// wait one by one need not be (a vote after the wait does not converge them).
+__device__ __forceinline__ bool mbar_test_warp(uint64_t *bar, uint32_t parity)
+{
+    return __all_sync(0xffffffffu, mbar_test(bar, parity));
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile uint32_t *abort_flag,
+                                               uint32_t *err, uint32_t code, unsigned long long limit_ns)
+{
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+    PollLimit limit(limit_ns);
+    for (;;) {
+        if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+        bool const stop = *abort_flag != 0, late = limit.expired();
+        if (__any_sync(0xffffffffu, stop || late)) {
+            if (!stop && threadIdx.x % 32 == 0) {
+                *abort_flag = 1;
+                atomicExch(err, code);
+            }
+            return false;
+        }
+    }
+}
+// A value that is the same in all lanes, in a uniform register.
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __reduce_max_sync(0xffffffffu, x); }
+
+// Shared-memory descriptor with its start address moved on by `off` 16-byte units
+// (no carry out of the address field: every operand lies below 256 KB).
+__device__ __forceinline__ uint64_t desc_at(uint64_t base, uint32_t off)
+{
+    uint64_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"((uint32_t)base + off), "r"((uint32_t)(base >> 32)));
+    return d;
+}
+
+// D (tensor memory) = or += A (tensor memory) x B (shared memory), kind::tf32.
+template <bool ACC>
+__device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
         : "memory");
 }
 
@@ -210,6 +338,16 @@ __device__ __forceinline__ void tmem_wait_ld_dep(uint32_t (&r)[32])
           "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
           "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]), "+r"(r[23]),
           "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]), "+r"(r[30]), "+r"(r[31])
+        :
+        : "memory");
+}
+// The same for a 16-column load.
+__device__ __forceinline__ void tmem_wait_ld_dep16(uint32_t (&r)[32])
+{
+    asm volatile(
+        "tcgen05.wait::ld.sync.aligned;"
+        : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+          "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
         :
         : "memory");
 }

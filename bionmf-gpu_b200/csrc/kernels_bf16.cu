@@ -36,6 +36,8 @@
 //
 // Warp roles (768 threads): 0 = V producer, 1 = MMA issuer / TMEM owner,
 // 2 = X and Y producer, 3 = idle, 4..19 = R warps, 20..23 = accumulator warps.
+// Persistent like the FP32 arm: every CTA takes an equal run of the list of all
+// row blocks' tiles (TileSplit), loading X anew where the run enters a row block.
 // Every wait is bounded (1 s); on expiry the kernel records an error word that
 // the host turns into NMFB_ETIMEOUT.  No TMA multicast is used.
 #include "nmfb_internal.cuh"
@@ -58,13 +60,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t acc)
+template <bool ACC>
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(acc)
+        "l"(adesc), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
         : "memory");
 }
 
@@ -116,8 +119,8 @@ struct MapsB {
 
 struct ArgsB {
     uint32_t O, R;
-    uint32_t tiles_per_split, nsplit;
-    float *part;
+    TileSplit ts;
+    float *part;                 // [slot][O][KP]
     uint32_t *err;
     const ConvState *st;
     unsigned long long wait_ns;  // limit of every bounded wait (%globaltimer ns)
@@ -186,18 +189,17 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     uint64_t *const accrdy = rempty + G::NRB;        // [2]    MMA2 commit -> accumulator warps
     uint64_t *const accfree = accrdy + 2;            // [2]    accumulator warps -> MMA2
     uint64_t *const xfull = accfree + 2;             // [1]    TMA -> MMA1
-    uint64_t *const mdrain = xfull + 1;              // [1]    issuer's final commit (drain)
+    uint64_t *const xfree = xfull + 1;               // [1]    last MMA1 of a row block -> X producer
+    uint64_t *const mdrain = xfree + 1;              // [1]    issuer's final commit (drain)
     uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(mdrain + 1);
     volatile uint32_t *const abort_flag = tmem_slot + 1;
 
-    uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    uint32_t const oblk = blockIdx.x / args.nsplit;
-    uint32_t const split = blockIdx.x % args.nsplit;
-    uint32_t const o0 = oblk * BO;
-    uint32_t const T_all = (args.R + BR - 1) / BR;
-    uint32_t const t_begin = split * args.tiles_per_split;
-    uint32_t const t_end = min(T_all, t_begin + args.tiles_per_split);
-    uint32_t const T = t_end > t_begin ? t_end - t_begin : 0;
+    uint32_t const warp = uniform(threadIdx.x / 32), lane = threadIdx.x % 32;
+    // This CTA's run of tiles [g0, g0 + T) of the (row block, reduction tile) list.
+    uint32_t const TB = args.ts.tb;
+    uint32_t const g0 = blockIdx.x * args.ts.tpc;
+    uint32_t const T = min(args.ts.total - g0, args.ts.tpc);
+    uint32_t const ob0 = g0 / TB, c00 = g0 - ob0 * TB;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < G::VST; s++) {
@@ -218,6 +220,7 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             mbar_init(&accfree[b], 4);
         }
         mbar_init(xfull, 1);
+        mbar_init(xfree, 1);
         mbar_init(mdrain, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -233,28 +236,26 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     tc_fence_after();
     uint32_t const tmem = *tmem_slot;
 
-    if (T == 0) {
-        // idle
-    } else if (warp == 0) {
+    if (warp == 0) {
         // ------------------------------------------------------------ V producer
         if (lane == 0) {
             uint64_t const pol = policy_evict_first();
-            uint32_t issued = 0;
-            for (uint32_t t = 0; t < T; t++) {
+            uint32_t issued = 0, ob = ob0, c = c00;
+            for (uint32_t t = 0; t < T; t++, ob += (c + 1 == TB), c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::VST;
                 if (t >= (uint32_t)G::VST &&
                     !mbar_wait(&vempty[s], ((t / G::VST) - 1) & 1, abort_flag, args.err, 21u, args.wait_ns))
                     break;
                 issued = t + 1;
                 unsigned char *sv = sV + s * G::VBYTES;
-                int const r0 = (int)((t_begin + t) * BR);
+                int const r0 = (int)(c * BR), o0 = (int)(ob * BO);
                 mbar_expect_tx(&vfull[s], G::VBYTES);
                 if (HSIDE) {
-                    tma_load_2d(sv, &maps.v, &vfull[s], (int)o0, r0, pol);     // V[r0:r0+BR][o0:o0+128]
+                    tma_load_2d(sv, &maps.v, &vfull[s], o0, r0, pol);          // V[r0:r0+BR][o0:o0+128]
                 } else {
 #pragma unroll
                     for (int b = 0; b < BR / 32; b++)                          // V[o0:o0+128][r0+32b : +32]
-                        tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, (int)o0, pol);
+                        tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, o0, pol);
                 }
             }
             // drain: the last load into every stage has landed
@@ -265,25 +266,30 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         // ------------------------------------------------------------ X and Y producer
         if (lane == 0) {
             uint64_t const pol = policy_evict_last();
-            mbar_expect_tx(xfull, (SPLIT ? 2 : 1) * G::XBYTES);
-            tma_load_2d(sX, &maps.xh, xfull, 0, (int)o0, pol);
-            if (SPLIT) tma_load_2d(sX + G::XBYTES, &maps.xl, xfull, 0, (int)o0, pol);
-            uint32_t issued = 0;
-            for (uint32_t t = 0; t < T; t++) {
+            uint32_t issued = 0, xs = 0, c = c00;   // xs: row blocks whose X has been requested
+            for (uint32_t t = 0; t < T; t++, c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::YST;
                 if (t >= (uint32_t)G::YST &&
                     !mbar_wait(&yempty[s], ((t / G::YST) - 1) & 1, abort_flag, args.err, 22u, args.wait_ns))
                     break;
                 issued = t + 1;
                 unsigned char *sy = sY + s * G::YSTAGE;
-                int const r0 = (int)((t_begin + t) * BR);
+                int const r0 = (int)(c * BR);
                 mbar_expect_tx(&yfull[s], (SPLIT ? 2 : 1) * G::YBYTES + G::YTROWS * 128);
                 tma_load_2d(sy, &maps.yh, &yfull[s], 0, r0, pol);
                 if (SPLIT) tma_load_2d(sy + G::YBYTES, &maps.yl, &yfull[s], 0, r0, pol);
-                tma_load_2d(sy + 2 * G::YBYTES, &maps.yt, &yfull[s], 0, (int)((t_begin + t) * 2 * KP), pol);
+                tma_load_2d(sy + 2 * G::YBYTES, &maps.yt, &yfull[s], 0, (int)(c * 2 * KP), pol);
+                if (t == 0 || c == 0) {   // X of the row block, once MMA1 has read the previous one's
+                    if (xs > 0 && !mbar_wait(xfree, (xs - 1) & 1, abort_flag, args.err, 29u, args.wait_ns)) break;
+                    int const o0 = (int)((ob0 + xs) * BO);
+                    mbar_expect_tx(xfull, (SPLIT ? 2 : 1) * G::XBYTES);
+                    tma_load_2d(sX, &maps.xh, xfull, 0, o0, pol);
+                    if (SPLIT) tma_load_2d(sX + G::XBYTES, &maps.xl, xfull, 0, o0, pol);
+                    xs++;
+                }
             }
-            // drain: X and the last load into every Y stage have landed
-            mbar_drain(xfull, 0);
+            // drain: the last X and the last load into every Y stage have landed
+            if (xs > 0) mbar_drain(xfull, (xs - 1) & 1);
             for (uint32_t t = issued > (uint32_t)G::YST ? issued - G::YST : 0; t < issued; t++)
                 mbar_drain(&yfull[t % G::YST], (t / G::YST) & 1);
         }
@@ -291,82 +297,97 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         // ------------------------------------------------------------ MMA issuer
         //   MMA2(n2): needs R(n2) in shared memory and, for n2 >= 2, Acc[n2 % 2]
         //             read by the accumulator warps (tile n2-2);
-        //   MMA1(n1): needs Y(n1) and a free D buffer (n1 < n2 + NDB).
+        //   MMA1(n1): needs Y(n1), a free D buffer (n1 < n2 + NDB) and, for the
+        //             first tile of a row block, its X; the last one's releases X.
         // MMA2(t) is the last reader of Y stage t % YST and R stage t % NRB.
-        if (lane == 0) {
-            constexpr uint32_t IDESC1 = idesc_bf16(BO, BR);
-            constexpr uint32_t IDESC2 = idesc_bf16(BO, KP);
-            constexpr uint32_t IDESC2W = idesc_bf16(BO, 2 * KP);
-            uint64_t const dXh = smem_desc(smem_u32(sX), 16, 8 * G::ROWB, G::LAYOUT);
-            uint64_t const dXl = dXh + (G::XBYTES >> 4);
-            uint64_t const dY0 = smem_desc(smem_u32(sY), 16, 8 * G::ROWB, G::LAYOUT);
-            uint64_t const dYT0 = smem_desc(smem_u32(sY + 2 * G::YBYTES), 16, 1024, 2u);
-            uint64_t const dR0 = smem_desc(smem_u32(sR), 16, 1024, 2u);
-            bool ok = mbar_wait(xfull, 0, abort_flag, args.err, 23u, args.wait_ns);
-            tc_fence_after();
-            uint32_t n1 = 0, n2 = 0;
-            unsigned long long last = globaltimer();
-            while (ok && n2 < T) {
-                bool progressed = false;
-                if (n2 < n1 && mbar_test(&rfull[n2 % G::NRB], (n2 / G::NRB) & 1) &&
-                    (n2 < 2 || mbar_test(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
-                    tc_fence_after();
-                    uint32_t const ys = n2 % G::YST, rs = n2 % G::NRB, bp = n2 & 1;
-                    uint64_t const dYT = dYT0 + ((ys * G::YSTAGE) >> 4);
-                    uint64_t const dR = dR0 + ((rs * G::RSTAGE) >> 4);
-                    uint32_t const dacc = tmem + bp * G::ACCW;
+        constexpr uint32_t IDESC1 = idesc_bf16(BO, BR);
+        constexpr uint32_t IDESC2 = idesc_bf16(BO, KP);
+        constexpr uint32_t IDESC2W = idesc_bf16(BO, 2 * KP);
+        uint32_t const sy_u32 = base_u32 + 2 * G::XBYTES, sr_u32 = sy_u32 + G::YST * G::YSTAGE;
+        uint64_t const dX = smem_desc(base_u32, 16, 8 * G::ROWB, G::LAYOUT);   // Xh, then Xl
+        uint64_t const dY0 = smem_desc(sy_u32, 16, 8 * G::ROWB, G::LAYOUT);
+        uint64_t const dYT0 = smem_desc(sy_u32 + 2 * G::YBYTES, 16, 1024, 2u);
+        uint64_t const dR0 = smem_desc(sr_u32, 16, 1024, 2u);
+        uint32_t const tm = uniform(tmem);
+        bool ok = true, x_ok = false;
+        uint32_t n1 = 0, n2 = 0, c1 = c00, xs = 0;   // c1: reduction tile of n1; xs: its row block, from the CTA's first
+        PollLimit limit(args.wait_ns);
+        while (ok && n2 < T) {
+            bool progressed = false;
+            if (n2 < n1 && mbar_test_warp(&rfull[n2 % G::NRB], (n2 / G::NRB) & 1) &&
+                (n2 < 2 || mbar_test_warp(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
+                tc_fence_after();
+                uint32_t const ys = n2 % G::YST, rs = n2 % G::NRB, bp = n2 & 1;
+                uint32_t const oyt = ys * (G::YSTAGE >> 4), orr = rs * (G::RSTAGE >> 4);
+                uint32_t const dacc = tm + bp * G::ACCW;
+                if (elect_one()) {
+                    // Acc[0:2KP] (+)= Rh [Y^T_hi; Y^T_lo];  Acc[0:KP] += Rl Y^T_hi  (MODE 2), or
+                    // Acc (+)= Rh Y^T_hi
+                    mma_bf16<false>(dacc, desc_at(dR0, orr), desc_at(dYT0, oyt), SPLIT2 ? IDESC2W : IDESC2);
+                    if (SPLIT2) mma_bf16<true>(dacc, desc_at(dR0, orr + (G::RBYTES >> 4)), desc_at(dYT0, oyt), IDESC2);
 #pragma unroll
-                    for (int ks = 0; ks < BR / 16; ks++) {
-                        if (SPLIT2) {
-                            // Acc[0:2KP] (+)= Rh [Y^T_hi; Y^T_lo];  Acc[0:KP] += Rl Y^T_hi
-                            mma_bf16(dacc, dR + ks * 2, dYT + ks * 2, IDESC2W, ks > 0 ? 1u : 0u);
-                            mma_bf16(dacc, dR + (G::RBYTES >> 4) + ks * 2, dYT + ks * 2, IDESC2, 1u);
-                        } else {
-                            mma_bf16(dacc, dR + ks * 2, dYT + ks * 2, IDESC2, ks > 0 ? 1u : 0u);
-                        }
+                    for (int ks = 1; ks < BR / 16; ks++) {
+                        mma_bf16<true>(dacc, desc_at(dR0, orr + ks * 2), desc_at(dYT0, oyt + ks * 2),
+                                       SPLIT2 ? IDESC2W : IDESC2);
+                        if (SPLIT2)
+                            mma_bf16<true>(dacc, desc_at(dR0, orr + (G::RBYTES >> 4) + ks * 2),
+                                           desc_at(dYT0, oyt + ks * 2), IDESC2);
                     }
                     tc_commit(&accrdy[bp]);
                     tc_commit(&yempty[ys]);
                     tc_commit(&rempty[rs]);
-                    n2++;
-                    progressed = true;
                 }
-                if (n1 < T && n1 < n2 + G::NDB && mbar_test(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
-                    tc_fence_after();
-                    uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
-                    uint64_t const dYh = dY0 + ((s * G::YSTAGE) >> 4);
-                    uint64_t const dYl = dYh + (G::YBYTES >> 4);
-                    uint32_t const dcol = tmem + G::DB0 + db * BR;
+                n2++;
+                progressed = true;
+            }
+            if (n1 < T && !x_ok) x_ok = mbar_test_warp(xfull, xs & 1);
+            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
+                tc_fence_after();
+                uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
+                uint32_t const oy = s * (G::YSTAGE >> 4);
+                uint32_t const dcol = tm + G::DB0 + db * BR;
+                bool const last = c1 + 1 == TB;   // the row block's last tile
+                if (elect_one()) {
                     // D = Xl Yh^T + Xh Yl^T + Xh Yh^T (split arms; small terms first), K = KP in steps of 16.
 #pragma unroll
                     for (int tt = 0; tt < NTERMS; tt++) {
                         int const term = NTERMS - 1 - tt;   // 2: Xl*Yh, 1: Xh*Yl, 0: Xh*Yh
-                        uint64_t const xa = (term == 2) ? dXl : dXh;
-                        uint64_t const yb = (term == 1) ? dYl : dYh;
+                        uint32_t const xo = (term == 2) ? (G::XBYTES >> 4) : 0;
+                        uint32_t const yo = oy + ((term == 1) ? (G::YBYTES >> 4) : 0);
+                        if (tt == 0)
+                            mma_bf16<false>(dcol, desc_at(dX, xo), desc_at(dY0, yo), IDESC1);
+                        else
+                            mma_bf16<true>(dcol, desc_at(dX, xo), desc_at(dY0, yo), IDESC1);
 #pragma unroll
-                        for (int ks = 0; ks < KP / 16; ks++)
-                            mma_bf16(dcol, xa + ks * 2, yb + ks * 2, IDESC1, (tt > 0 || ks > 0) ? 1u : 0u);
+                        for (int ks = 1; ks < KP / 16; ks++)
+                            mma_bf16<true>(dcol, desc_at(dX, xo + ks * 2), desc_at(dY0, yo + ks * 2), IDESC1);
                     }
                     tc_commit(&dfull[db]);
-                    n1++;
-                    progressed = true;
+                    if (last) tc_commit(xfree);
                 }
-                if (progressed) {
-                    last = globaltimer();
-                } else if (*abort_flag) {
+                n1++;
+                c1 = last ? 0 : c1 + 1;
+                xs += last;
+                x_ok = !last;
+                progressed = true;
+            }
+            if (progressed) {
+                limit.reset();
+            } else {
+                bool const stop = *abort_flag != 0, late = limit.expired();
+                if (__any_sync(0xffffffffu, stop || late)) {
+                    if (!stop && lane == 0) {
+                        *abort_flag = 1;
+                        atomicExch(args.err, 24u);
+                    }
                     ok = false;
-                } else if (globaltimer() - last > args.wait_ns) {
-                    *abort_flag = 1;
-                    atomicExch(args.err, 24u);
-                    ok = false;
-                } else {
-                    __nanosleep(64);
                 }
             }
-            // drain: every MMA issued above has completed before the CTA frees
-            // the shared and tensor memory it reads and writes
-            mma_drain(mdrain);
         }
+        // drain: every MMA issued above has completed before the CTA frees
+        // the shared and tensor memory it reads and writes
+        if (elect_one()) mma_drain(mdrain);
+        __syncwarp();
     } else if (warp >= 4 && warp < 4 + NR) {
         // ------------------------------------------------------------ R warps
         // Two teams of NR/2 warps take alternate tiles (team 0 even, team 1 odd), so
@@ -382,15 +403,16 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
         for (uint32_t t = team; t < T; t += 2) {
             uint32_t const s = t % G::VST, b = t % G::NDB, rs = t % G::NRB;
-            if (!mbar_wait(&dfull[b], (t / G::NDB) & 1, abort_flag, args.err, 25u, args.wait_ns)) break;
-            if (!mbar_wait(&vfull[s], (t / G::VST) & 1, abort_flag, args.err, 26u, args.wait_ns)) break;
+            uint32_t const c = (c00 + t) % TB;              // reduction tile
+            if (!mbar_wait_warp(&dfull[b], (t / G::NDB) & 1, abort_flag, args.err, 25u, args.wait_ns)) break;
+            if (!mbar_wait_warp(&vfull[s], (t / G::VST) & 1, abort_flag, args.err, 26u, args.wait_ns)) break;
             if (t >= (uint32_t)G::NRB &&
-                !mbar_wait(&rempty[rs], ((t / G::NRB) - 1) & 1, abort_flag, args.err, 27u, args.wait_ns))
+                !mbar_wait_warp(&rempty[rs], ((t / G::NRB) - 1) & 1, abort_flag, args.err, 27u, args.wait_ns))
                 break;
             tc_fence_after();
             const unsigned char *sv = sV + s * G::VBYTES;
-            bool const edge = (t_begin + t + 1) * BR > args.R;   // the partial last reduction tile
-            int const valid = (int)(args.R - (t_begin + t) * BR);          // its columns before R
+            bool const edge = (c + 1) * BR > args.R;        // the partial last reduction tile
+            int const valid = (int)(args.R - c * BR);       // its columns before R
 #pragma unroll 1
             for (int ch = 0; ch < CW / 16; ch++) {
                 int const col0 = grp * CW + ch * 16;
@@ -415,10 +437,6 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                         v[4 * c + 2] = x.z;
                         v[4 * c + 3] = x.w;
                     }
-                }
-                if (ch == CW / 16 - 1) {
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&vempty[s]);
                 }
                 tmem_wait_ld_dep(d);
                 if (edge) {
@@ -457,7 +475,10 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&rfull[rs]);
+            if (lane == 0) {
+                mbar_arrive(&vempty[s]);   // the values of V have been used (see the FP32 kernel)
+                mbar_arrive(&rfull[rs]);
+            }
         }
     } else if (warp >= 4 + NR) {
         // ------------------------------------------------------------ accumulator warps
@@ -467,44 +488,46 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         float sum[KP];
 #pragma unroll
         for (int c = 0; c < KP; c++) sum[c] = 0.0f;
-        bool ok = true;
-        for (uint32_t t = 0; ok && t < T; t++) {
+        uint32_t ob = ob0, c1 = c00;   // row block and reduction tile of t
+        bool gap_done = c00 == 0 || c00 % args.ts.run != 0;
+        for (uint32_t t = 0; t < T; t++) {
             uint32_t const bp = t & 1;
-            if (!mbar_wait(&accrdy[bp], (t >> 1) & 1, abort_flag, args.err, 28u, args.wait_ns)) {
-                ok = false;
-                break;
-            }
+            if (!mbar_wait_warp(&accrdy[bp], (t >> 1) & 1, abort_flag, args.err, 28u, args.wait_ns)) break;
             tc_fence_after();
 #pragma unroll
-            for (int part = 0; part < (SPLIT2 ? 2 : 1); part++) {
+            for (int c0 = 0; c0 < KP; c0 += 16) {
+                uint32_t a[32], a2[32];
+                tmem_ld16(lane_addr + bp * G::ACCW + c0, a);
+                if (SPLIT2) tmem_ld16(lane_addr + bp * G::ACCW + KP + c0, a2);
+                tmem_wait_ld_dep16(a);
+                if (SPLIT2) tmem_wait_ld_dep16(a2);
 #pragma unroll
-                for (int c0 = 0; c0 < KP; c0 += 16) {
-                    uint32_t a[32];
-                    tmem_ld16(lane_addr + bp * G::ACCW + part * KP + c0, a);
-                    tmem_wait_ld_dep(a);
-#pragma unroll
-                    for (int c = 0; c < 16; c++) sum[c0 + c] += __uint_as_float(a[c]);
-                }
+                for (int c = 0; c < 16; c++)
+                    sum[c0 + c] += SPLIT2 ? __uint_as_float(a[c]) + __uint_as_float(a2[c]) : __uint_as_float(a[c]);
             }
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&accfree[bp]);
-        }
-        if (ok) {
-            uint32_t const o = o0 + row;
-            if (o < args.O) {
-                float *dst = args.part + ((size_t)split * args.O + o) * KP;
+            bool const done = c1 + 1 == TB;   // the row block's last tile
+            if (done || t + 1 == T || (c1 + 1) % args.ts.run == 0) {   // a partial of the row block
+                uint32_t const o = ob * BO + row;
+                if (o < args.O) {
+                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP;
 #pragma unroll
-                for (int c = 0; c < KP; c += 4)
-                    *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                    for (int c = 0; c < KP; c += 4)
+                        *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                    if (!gap_done) {   // the unused slot (TileSplit::slot)
+                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP;
+#pragma unroll
+                        for (int c = 0; c < KP; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                }
+                gap_done = true;
+#pragma unroll
+                for (int c = 0; c < KP; c++) sum[c] = 0.0f;
             }
-        }
-    }
-    if (T == 0 && warp >= 4 + NR) {
-        uint32_t const o = o0 + (warp & 3) * 32 + lane;
-        if (o < args.O) {
-            float *dst = args.part + ((size_t)split * args.O + o) * KP;
-            for (int c = 0; c < KP; c++) dst[c] = 0.0f;
+            c1 = done ? 0 : c1 + 1;
+            ob += done;
         }
     }
     tc_fence_before();
@@ -574,35 +597,19 @@ int set_attrs_b(nmfb_ctx *ctx)
 }
 
 template <bool HSIDE, int KP, int MODE>
-int launch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err)
+int launch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
 {
     using G = GeoB<KP, MODE>;
     constexpr int BR = G::BR;
     uint32_t const O = HSIDE ? ctx->m : ctx->n;
     uint32_t const R = HSIDE ? ctx->n : ctx->m;
-    uint32_t const oblocks = (O + BO - 1) / BO;
-    uint32_t const T = (R + BR - 1) / BR;
-    // Same wave model as the FP32 arm: minimise waves x (tiles per split + fill).
-    uint32_t tps = T, best = 0xffffffffu;
-    for (uint32_t want = 1; want <= NMFB_MAX_SPLIT && want <= T; want++) {
-        uint32_t const t_ps = (T + want - 1) / want;
-        uint32_t const ns = (T + t_ps - 1) / t_ps;
-        if ((size_t)ns * O * KP > ctx->part_items) break;
-        uint32_t const waves = (oblocks * ns + (uint32_t)ctx->sm_count - 1) / (uint32_t)ctx->sm_count;
-        uint32_t const cost = waves * (t_ps + 3);
-        if (cost < best) {
-            best = cost;
-            tps = t_ps;
-        }
-    }
-    uint32_t const nsplit = (T + tps - 1) / tps;
-    if ((size_t)nsplit * O * KP > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arm: partial buffer too small (%u splits)", nsplit);
+    ts = plan_tiles(O, R, BR, (uint32_t)ctx->sm_count, ctx->part_items / KP);
+    if ((size_t)ts.slots * O * KP > ctx->part_items)
+        return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arm: partial buffer too small (%u slots)", ts.slots);
     ArgsB args;
     args.O = O;
     args.R = R;
-    args.tiles_per_split = tps;
-    args.nsplit = nsplit;
+    args.ts = ts;
     args.part = ctx->dPart;
     args.err = err;
     args.st = ctx->dState;
@@ -610,29 +617,28 @@ int launch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err)
     int const main = HSIDE ? 0 : 1;
     int rc = nmfb_prof_begin(ctx, main);
     if (rc) return rc;
-    k_fused_bf16<HSIDE, KP, MODE><<<oblocks * nsplit, G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
+    k_fused_bf16<HSIDE, KP, MODE><<<ts.ctas(), G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
     NMFB_LAUNCH_CHECK(ctx);
-    if ((rc = nmfb_prof_end(ctx, main))) return rc;
-    return (int)nsplit;
+    return nmfb_prof_end(ctx, main);
 }
 
 template <bool HSIDE, int KP>
-int dispatch_kp(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err)
+int dispatch_kp(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
 {
     switch (ctx->arm) {
-    case NMFB_ARM_BF16: return launch_b<HSIDE, KP, 0>(ctx, maps, err);
-    case NMFB_ARM_SPLIT_BF16: return launch_b<HSIDE, KP, 1>(ctx, maps, err);
-    default: return launch_b<HSIDE, KP, 2>(ctx, maps, err);
+    case NMFB_ARM_BF16: return launch_b<HSIDE, KP, 0>(ctx, maps, err, ts);
+    case NMFB_ARM_SPLIT_BF16: return launch_b<HSIDE, KP, 1>(ctx, maps, err, ts);
+    default: return launch_b<HSIDE, KP, 2>(ctx, maps, err, ts);
     }
 }
 
 template <bool HSIDE>
-int dispatch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err)
+int dispatch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
 {
     switch (ctx->kp) {
-    case 16: return dispatch_kp<HSIDE, 16>(ctx, maps, err);
-    case 32: return dispatch_kp<HSIDE, 32>(ctx, maps, err);
-    case 64: return dispatch_kp<HSIDE, 64>(ctx, maps, err);
+    case 16: return dispatch_kp<HSIDE, 16>(ctx, maps, err, ts);
+    case 32: return dispatch_kp<HSIDE, 32>(ctx, maps, err, ts);
+    case 64: return dispatch_kp<HSIDE, 64>(ctx, maps, err, ts);
     default: return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arms: unsupported padded rank %u", ctx->kp);
     }
 }
@@ -695,18 +701,18 @@ int prepare_b(nmfb_ctx *ctx, bool w)
 }
 
 template <int KP>
-int launch_finish_b(nmfb_ctx *ctx, bool is_H, uint32_t nsplit, int adjust)
+int launch_finish_b(nmfb_ctx *ctx, bool is_H, const TileSplit &ts, int adjust)
 {
     PlanB *plan = (PlanB *)ctx->bplan;
     uint32_t const O = is_H ? ctx->m : ctx->n;
-    uint32_t const fblocks = fin_blocks(O, fin_rpt(nsplit));
+    uint32_t const fblocks = fin_blocks(O, fin_rpt(ts.slots));
     if (fblocks > plan->csoff || (fblocks + FIN_ECH - 1) / FIN_ECH + 1 > plan->nticks)
         return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arms: column-sum buffers too small");
     __nv_bfloat16 *xs = is_H ? plan->hsplit : plan->wsplit;
     size_t const sz = (size_t)O * KP;
     FinishArgs fa = {};
     fa.O = O;
-    fa.nsplit = nsplit;
+    fa.ts = ts;
     fa.k = ctx->k;
     fa.adjust = adjust;
     fa.part = ctx->dPart;
@@ -739,12 +745,13 @@ int bf16_half(nmfb_ctx *ctx, bool is_H, int adjust)
     if ((rc = nmfb_prof_begin(ctx, whole))) return rc;
     if (!ctx->fz_ok[is_H ? 0 : 1] && (rc = prepare_b(ctx, is_H))) return rc;    // Y
     if (!ctx->fz_ok[is_H ? 1 : 0] && (rc = prepare_b(ctx, !is_H))) return rc;   // X
-    int const nsplit = is_H ? dispatch_b<true>(ctx, plan->mapsH, plan->dErr) : dispatch_b<false>(ctx, plan->mapsW, plan->dErr);
-    if (nsplit < 0) return nsplit;
+    TileSplit ts;
+    if ((rc = is_H ? dispatch_b<true>(ctx, plan->mapsH, plan->dErr, ts) : dispatch_b<false>(ctx, plan->mapsW, plan->dErr, ts)))
+        return rc;
     switch (ctx->kp) {
-    case 16: rc = launch_finish_b<16>(ctx, is_H, (uint32_t)nsplit, adjust); break;
-    case 32: rc = launch_finish_b<32>(ctx, is_H, (uint32_t)nsplit, adjust); break;
-    default: rc = launch_finish_b<64>(ctx, is_H, (uint32_t)nsplit, adjust); break;
+    case 16: rc = launch_finish_b<16>(ctx, is_H, ts, adjust); break;
+    case 32: rc = launch_finish_b<32>(ctx, is_H, ts, adjust); break;
+    default: rc = launch_finish_b<64>(ctx, is_H, ts, adjust); break;
     }
     if (rc) return rc;
     ctx->fz_ok[is_H ? 1 : 0] = 1;

@@ -15,7 +15,8 @@
 //              producer TMA-loads them per tile.  X (128 rows per CTA) is split
 //              once per CTA by the accumulator warps.
 //   MMA1     : D (TMEM, 128 x BR) = Xh Yh^T                    (kind::tf32, k-steps of 8)
-//              + [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T (kind::f16, K = 2 KP, k-steps of 16).
+//              + [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T (kind::f16, K = 2 KP, k-steps of 16),
+//              or at KP = 16 + Xh Yl^T + Xl Yh^T (kind::tf32).
 //   epilogue : R = V / D in FP32 registers (V times an approximate reciprocal,
 //              <= 1.5 ulp; the reference uses fdividef);  R = Rh + Rl with
 //              Rh = TF32(R) written back over D and bf16(Rl) packed into a
@@ -70,16 +71,16 @@ __host__ __device__ constexpr uint32_t idesc_bf16xf32(uint32_t M, uint32_t N)
     return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-// kind::f16 MMA with A from tensor memory (two BF16 per 32-bit column, the
+// D = or += A B, kind::f16, with A from tensor memory (two BF16 per 32-bit column, the
 // lower K index in the low half) and B from shared memory.
-__device__ __forceinline__ void mma_ts_bf16(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
-                                            uint32_t acc)
+template <bool ACC>
+__device__ __forceinline__ void mma_ts_bf16(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc)
 {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(acc)
+        "r"(a_tmem), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
         : "memory");
 }
 
@@ -106,18 +107,18 @@ struct FusedMaps {
     CUtensorMap v;       // V, box [128 x BR] (H side, no swizzle) or [32 x 128] (W side, 128B swizzle)
     CUtensorMap y;       // TF32 hi part of the other factor (rows x KP), box rows = BR
     CUtensorMap yt;      // its transposed split: per 32 rows, [hi^T (KP x 32) ; lo^T (KP x 32)]
-    CUtensorMap ylb;     // BF16 copy of its lo part (rows x KP), box [KP x BR]
+    CUtensorMap ylb;     // BF16 copy of its lo part (KP = 16: the FP32 lo part; rows x KP), box [KP x BR]
     CUtensorMap yb;      // BF16 copy (rows x KP), box [KP x BR]
     CUtensorMap ybt;     // BF16 transposed tiles: per BR rows, KP rows of BR values; box [BR x KP]
 };
 
 struct FusedArgs {
     uint32_t O, R;        // output rows, reduction length
-    uint32_t tiles_per_split, nsplit;
-    float *part;          // [split][O][KP]
+    TileSplit ts;
+    float *part;          // [slot][O][KP]
     uint32_t *err;        // device error word
     const ConvState *st;
-    const float *X;       // factor being updated (O x KP), read once per CTA into TMEM
+    const float *X;       // factor being updated (O x KP), read once per row block into TMEM
     unsigned long long wait_ns;  // limit of every bounded wait (%globaltimer ns)
 #ifdef NMFB_FUSED_DEBUG
     float *dbg;           // block 0, tile 0: D | V | Rh | Acc (debug builds only; 128 x 64 each)
@@ -142,6 +143,11 @@ struct Geo {
     static constexpr int YBB = BR * KP * 2;                // one BF16 tile of BR rows of 2 KP bytes
     static constexpr int YBTB = KP * BR * 2;               // bf16(Y)^T tile, KP rows of 2 BR bytes
     static constexpr int YBSTAGE = 2 * YBB + YBTB;         // bf16(Yl) | bf16(Y) | bf16(Y)^T
+    // MMA1's small terms Xh Yl + Xl Y: TF32 at KP = 16 (Xh Yl + Xl Yh, from an FP32 copy of
+    // Yl that takes the place of the two BF16 tiles; 2 of 18 MMAs more, and MMAs do not bound
+    // the small problems of these ranks), BF16 above (4 of 20 MMAs fewer at KP = 32).
+    static constexpr bool LO32 = KP == 16;
+    static_assert(!LO32 || YBYTES == 2 * YBB, "the FP32 tile of Yl takes the BF16 tiles' place");
     static constexpr uint32_t BLAYOUT = umma_layout(2 * KP);
     static constexpr uint32_t BTLAYOUT = umma_layout(2 * BR);
     static constexpr int YST = 3;
@@ -157,25 +163,28 @@ struct Geo {
     static constexpr uint32_t ACC = 2 * KP;                // TMEM columns of one per-tile accumulator
     static constexpr uint32_t NDB = (KP == 16) ? 4 : (KP == 32) ? 3 : 2;   // D buffers (MMA1 runs NDB tiles ahead)
     static constexpr uint32_t DA0 = 2 * ACC;               // D[b] (then Rh[b]) at DA0 + b BR
+    static constexpr uint32_t NRL = (KP == 32) ? 2 : NDB;  // bf16(Rl) buffers (2: one per R team)
     static constexpr uint32_t RL0 = DA0 + NDB * BR;        // bf16(Rl)[b] at RL0 + b BR/2
-    static constexpr uint32_t XC0 = RL0 + NDB * BR / 2;    // X hi (TF32), KP columns
-    static constexpr uint32_t XB0 = XC0 + KP;              // bf16(X hi) | bf16(X lo), KP/2 columns each
-    static_assert(XB0 + KP <= 512, "TMEM columns exceeded");
+    static constexpr uint32_t NXB = (KP == 64) ? 1 : 2;    // X buffers (2: the next row block's X while this one is read)
+    static constexpr uint32_t XC0 = RL0 + NRL * BR / 2;    // X hi (TF32, KP columns) | bf16(X hi) | bf16(X lo)
+                                                           // (KP/2 each) or X lo (TF32, KP); buffer b at XC0 + 2 KP b
+    static_assert(XC0 + NXB * 2 * KP <= 512, "TMEM columns exceeded");
 };
 
 // TMEM columns: per-tile accumulators Acc[b] at b*2KP (2KP columns: the Rh Yh +
 // bf16(Rl) bf16(Y) sum and the Rh Yl part side by side); D[b] (BR columns, then
-// Rh[b]) at DA0 + b*BR and bf16(Rl)[b] (BR/2 columns, column group g of 16 in
-// its 8 columns RL0 + b*BR/2 + 8g), b < NDB; then the CTA's 128 rows of X as
-// TF32 hi (KP columns) and bf16(X hi) | bf16(X lo) (KP/2 columns each), the A
-// operands of MMA1 for every tile (so MMA1 reads only Y from shared memory).
+// Rh[b]) at DA0 + b*BR, b < NDB; bf16(Rl)[b] (BR/2 columns, column group g of
+// 16 in its 8 columns RL0 + b*BR/2 + 8g), b < NRL; then, per X buffer, a row
+// block's 128 rows of X as TF32 hi (KP columns) and bf16(X hi) | bf16(X lo)
+// (KP/2 columns each), the A operands of MMA1 for every tile of that row block
+// (so MMA1 reads only Y from shared memory).
 
 // Split a factor Y (rows x kp, FP32, padding columns zero) for the fused
 // kernel's TMA loads, one CTA per block of `br` rows (br = the kernel's tile):
 //   hi = TF32(y) (round to nearest), rows x kp;
 //   T: per 32 rows, the transposed hi block (kp rows of 32 floats) followed by
 //      the transposed lo block (lo = y - hi, exact), rows past the end zero;
-//   Bl = bf16(lo), B = bf16(y): rows x kp each;
+//   Bl = bf16(lo), B = bf16(y): rows x kp each (kp = 16: lo, FP32, in their place);
 //   BT: per br rows, the transposed bf16(y) block (kp rows of br values), rows
 //      past the end zero.
 // The transposes go through shared memory.
@@ -196,8 +205,12 @@ __global__ void __launch_bounds__(256) k_split_factor(const float *__restrict__ 
         __nv_bfloat16 const yb = __float2bfloat16_rn(y);
         if (in) {
             hi[(size_t)(r0 + r) * kp + c] = h;
-            Bl[(size_t)(r0 + r) * kp + c] = __float2bfloat16_rn(l);
-            B[(size_t)(r0 + r) * kp + c] = yb;
+            if (kp == 16) {
+                reinterpret_cast<float *>(Bl)[(size_t)(r0 + r) * kp + c] = l;
+            } else {
+                Bl[(size_t)(r0 + r) * kp + c] = __float2bfloat16_rn(l);
+                B[(size_t)(r0 + r) * kp + c] = yb;
+            }
         }
         th[r][c] = h;
         tl[r][c] = l;
@@ -218,10 +231,14 @@ __global__ void __launch_bounds__(256) k_split_factor(const float *__restrict__ 
     for (uint32_t e = threadIdx.x; e < kp * br; e += blockDim.x) bt[e] = tb[e % br][e / br];
 }
 
-// Warp roles: 0 = V producer (TMA), 1 = MMA issuer + TMEM owner, 2 = X and Y
-// producer (TMA), 3 = idle, 4..11 = R warps (V / D, feed MMA2), 12..15 =
-// accumulator warps (sum the per-tile MMA2 results in FP32 registers; split X
-// and, YST tiles ahead, each Y tile into TF32 hi/lo and its transpose).
+// Warp roles: 0 = V producer (TMA), 1 = MMA issuer + TMEM owner, 2 = Y
+// producer (TMA), 3 = idle, 4 .. 3 + NR = R warps (V / D, feed MMA2), last four =
+// accumulator warps (sum the per-tile MMA2 results in FP32 registers; split X).
+//
+// Persistent, one CTA per SM: the tiles of all row blocks form one list and
+// every CTA takes an equal run of it (TileSplit), so the launch is one wave
+// whatever the shape and pays the pipeline's fill (about six tile times) once
+// per CTA instead of once per (row block, split) pair.
 template <bool HSIDE, int KP, int NTERMS>
 __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     k_fused_half(const __grid_constant__ FusedMaps maps, const FusedArgs args)
@@ -248,19 +265,19 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     uint64_t *const rfull = dfull + G::NDB;         // [NDB]  R warps -> MMA2
     uint64_t *const accrdy = rfull + G::NDB;        // [2]    MMA2 commit -> accumulator warps
     uint64_t *const accfree = accrdy + 2;           // [2]    accumulator warps -> MMA2
-    uint64_t *const xready = accfree + 2;           // [1]    X split into TMEM -> MMA1
-    uint64_t *const mdrain = xready + 1;            // [1]    issuer's final commit (drain)
+    uint64_t *const xready = accfree + 2;           // [NXB]  X split into TMEM -> MMA1
+    uint64_t *const xfree = xready + G::NXB;        // [NXB]  last MMA1 of a row block -> accumulator warps
+    uint64_t *const mdrain = xfree + G::NXB;        // [1]    issuer's final commit (drain)
     uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(mdrain + 1);
     volatile uint32_t *const abort_flag = tmem_slot + 1;
 
-    uint32_t const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    uint32_t const oblk = blockIdx.x / args.nsplit;
-    uint32_t const split = blockIdx.x % args.nsplit;
-    uint32_t const o0 = oblk * BO;
-    uint32_t const T_all = (args.R + BR - 1) / BR;
-    uint32_t const t_begin = split * args.tiles_per_split;
-    uint32_t const t_end = min(T_all, t_begin + args.tiles_per_split);
-    uint32_t const T = t_end > t_begin ? t_end - t_begin : 0;
+    uint32_t const warp = uniform(threadIdx.x / 32), lane = threadIdx.x % 32;
+    // This CTA's run of tiles [g0, g0 + T) of the whole (row block, reduction tile)
+    // list, row-block-major: tile g is reduction tile g % TB of row block g / TB.
+    uint32_t const TB = args.ts.tb;
+    uint32_t const g0 = blockIdx.x * args.ts.tpc;
+    uint32_t const T = min(args.ts.total - g0, args.ts.tpc);
+    uint32_t const ob0 = g0 / TB, c00 = g0 - ob0 * TB;
 #ifdef NMFB_FUSED_DEBUG
     // Per-tile event times of block 0 (ns since kernel start), 8 events x 64 tiles.
     unsigned long long const ts0 = globaltimer();
@@ -296,7 +313,10 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             mbar_init(&accrdy[b], 1);
             mbar_init(&accfree[b], 4);
         }
-        mbar_init(xready, 4);
+        for (uint32_t b = 0; b < G::NXB; b++) {
+            mbar_init(&xready[b], 4);
+            mbar_init(&xfree[b], 1);
+        }
         mbar_init(mdrain, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -312,29 +332,27 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     tc_fence_after();
     uint32_t const tmem = *tmem_slot;
 
-    if (T == 0 && warp < 4 + NR) {
-        // idle (the accumulator warps write a zero partial)
-    } else if (warp == 0) {
+    if (warp == 0) {
         // ------------------------------------------------------------ V producer
         if (lane == 0) {
             uint64_t const pol = policy_evict_first();
-            uint32_t issued = 0;
-            for (uint32_t t = 0; t < T; t++) {
+            uint32_t issued = 0, ob = ob0, c = c00;
+            for (uint32_t t = 0; t < T; t++, ob += (c + 1 == TB), c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::VST;
                 if (t >= (uint32_t)G::VST &&
                     !mbar_wait(&vempty[s], ((t / G::VST) - 1) & 1, abort_flag, args.err, 1u, args.wait_ns))
                     break;
                 issued = t + 1;
                 unsigned char *sv = sV + s * G::VBYTES;
-                int const r0 = (int)((t_begin + t) * BR);
+                int const r0 = (int)(c * BR), o0 = (int)(ob * BO);
                 DBG_TS(0, t);
                 mbar_expect_tx(&vfull[s], G::VBYTES);
                 if (HSIDE) {
-                    tma_load_2d(sv, &maps.v, &vfull[s], (int)o0, r0, pol);     // V[r0:r0+BR][o0:o0+128]
+                    tma_load_2d(sv, &maps.v, &vfull[s], o0, r0, pol);          // V[r0:r0+BR][o0:o0+128]
                 } else {
 #pragma unroll
                     for (int b = 0; b < BR / 32; b++)                          // V[o0:o0+128][r0+32b : +32]
-                        tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, (int)o0, pol);
+                        tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, o0, pol);
                 }
             }
             // drain: the last load into every stage has landed (each earlier one
@@ -346,23 +364,23 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         // ------------------------------------------------------------ Y producer
         if (lane == 0) {
             uint64_t const pol = policy_evict_last();
-            uint32_t issued = 0;
-            for (uint32_t t = 0; t < T; t++) {
+            uint32_t issued = 0, c = c00;
+            for (uint32_t t = 0; t < T; t++, c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::YST;
                 if (t >= (uint32_t)G::YST &&
                     !mbar_wait(&yempty[s], ((t / G::YST) - 1) & 1, abort_flag, args.err, 2u, args.wait_ns))
                     break;
                 issued = t + 1;
                 unsigned char *syh = sY + s * G::YSTAGE;
-                int const r0 = (int)((t_begin + t) * BR);
+                int const r0 = (int)(c * BR);
                 DBG_TS(1, t);
                 mbar_expect_tx(&yfull[s], G::YBYTES + G::YTSTAGE + (NTERMS == 3 ? G::YBSTAGE : 0));
                 for (int b = 0; b < G::NB; b++) tma_load_2d(syh + b * G::YBLK, &maps.y, &yfull[s], b * G::CB, r0, pol);
                 if (NTERMS == 3) {
                     unsigned char *syb = sYB + s * G::YBSTAGE;
                     tma_load_2d(syb, &maps.ylb, &yfull[s], 0, r0, pol);
-                    tma_load_2d(syb + G::YBB, &maps.yb, &yfull[s], 0, r0, pol);
-                    tma_load_2d(syb + 2 * G::YBB, &maps.ybt, &yfull[s], 0, (int)((t_begin + t) * KP), pol);
+                    if (!G::LO32) tma_load_2d(syb + G::YBB, &maps.yb, &yfull[s], 0, r0, pol);
+                    tma_load_2d(syb + 2 * G::YBB, &maps.ybt, &yfull[s], 0, (int)(c * KP), pol);
                 }
                 // Y^T: the BR / 32 row blocks of this tile, 2 KP rows of 128 B each
                 tma_load_2d(sYT + s * G::YTSTAGE, &maps.yt, &yfull[s], 0, (r0 / 32) * 2 * KP, pol);
@@ -372,105 +390,126 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        // Two issue queues, polled without blocking (shortest nanosleep between polls):
+        // Two issue queues, polled without blocking:
         //   MMA2(n2): needs the R warps' R(n2) and, for n2 >= 2, the accumulator
         //             warps to have read Acc[n2 % 2] of tile n2-2;
         //   MMA1(n1): needs Y(n1) loaded and a free D buffer (MMA2(n1-NDB)
-        //             issued, i.e. n1 < n2 + NDB); A = X from TMEM.
+        //             issued, i.e. n1 < n2 + NDB); A = X from TMEM, which for the
+        //             first tile of a row block has to be ready, and whose buffer the
+        //             last one's MMA1 releases.
         // The Y stage of tile t is released when MMA2(t), the last reader, completes.
-        if (lane == 0) {
-            constexpr uint32_t IDESC1 = idesc_tf32(BO, BR, 0);
-            constexpr uint32_t IDESC1B = idesc_bf16xf32(BO, BR);
-            constexpr uint32_t IDESC2 = idesc_tf32(BO, KP, 0);
-            constexpr uint32_t IDESC2W = idesc_tf32(BO, 2 * KP, 0);
-            constexpr uint32_t IDESC2B = idesc_bf16xf32(BO, KP);
-            // Shared-memory descriptors are built once; a k-step or stage offset is
-            // added to the start-address field (16-byte units, no carry out of it:
-            // every operand lies below 256 KB).
-            uint64_t const dY0 = smem_desc(smem_u32(sY), 16, 8 * G::ROWB, G::LAYOUT);
-            uint64_t const dYT0 = smem_desc(smem_u32(sYT), 16, 1024, 2u);
-            uint64_t const dYB0 = smem_desc(smem_u32(sYB), 16, 8 * 2 * KP, G::BLAYOUT);
-            uint64_t const dYBT0 = smem_desc(smem_u32(sYB + 2 * G::YBB), 16, 8 * 2 * BR, G::BTLAYOUT);
-            bool ok = mbar_wait(xready, 0, abort_flag, args.err, 3u, args.wait_ns);
-            tc_fence_after();
-            uint32_t n1 = 0, n2 = 0;
-            unsigned long long last = globaltimer();
-            while (ok && n2 < T) {
-                bool progressed = false;
-                if (n2 < n1 && mbar_test(&rfull[n2 % G::NDB], (n2 / G::NDB) & 1) &&
-                    (n2 < 2 || mbar_test(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
-                    tc_fence_after();
-                    uint32_t const sp = n2 % G::YST, bp = n2 & 1, db = n2 % G::NDB;
-                    uint64_t const dYT = dYT0 + ((sp * G::YTSTAGE) >> 4);
-                    uint32_t const rh = tmem + G::DA0 + db * BR;
-                    uint32_t const rl = tmem + G::RL0 + db * (BR / 2);
-                    uint32_t const dacc = tmem + bp * ACC_COLS;
+        constexpr uint32_t IDESC1 = idesc_tf32(BO, BR, 0);
+        constexpr uint32_t IDESC1B = idesc_bf16xf32(BO, BR);
+        constexpr uint32_t IDESC2 = NTERMS == 3 ? idesc_tf32(BO, 2 * KP, 0) : idesc_tf32(BO, KP, 0);
+        constexpr uint32_t IDESC2B = idesc_bf16xf32(BO, KP);
+        uint64_t const dY0 = smem_desc(base_u32, 16, 8 * G::ROWB, G::LAYOUT);
+        uint64_t const dYT0 = smem_desc(base_u32 + G::YST * G::YSTAGE, 16, 1024, 2u);
+        uint32_t const yb_u32 = base_u32 + G::YST * (G::YSTAGE + G::YTSTAGE);
+        uint64_t const dYB0 = G::LO32 ? smem_desc(yb_u32, 16, 8 * G::ROWB, G::LAYOUT)
+                                      : smem_desc(yb_u32, 16, 8 * 2 * KP, G::BLAYOUT);
+        uint64_t const dYBT0 = smem_desc(yb_u32 + 2 * G::YBB, 16, 8 * 2 * BR, G::BTLAYOUT);
+        uint32_t const tm = uniform(tmem);
+        bool ok = true, x_ok = false;
+        uint32_t n1 = 0, n2 = 0, c1 = c00, xs = 0;   // c1: reduction tile of n1; xs: its row block, counted from the CTA's first
+        PollLimit limit(args.wait_ns);
+        while (ok && n2 < T) {
+            bool progressed = false;
+            if (n2 < n1 && mbar_test_warp(&rfull[n2 % G::NDB], (n2 / G::NDB) & 1) &&
+                (n2 < 2 || mbar_test_warp(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
+                tc_fence_after();
+                uint32_t const sp = n2 % G::YST, bp = n2 & 1, db = n2 % G::NDB;
+                uint32_t const rh = tm + G::DA0 + db * BR;
+                uint32_t const rl = tm + G::RL0 + (n2 % G::NRL) * (BR / 2);
+                uint32_t const dacc = tm + bp * ACC_COLS;
+                uint32_t const oyt = sp * (G::YTSTAGE >> 4), oybt = sp * (G::YBSTAGE >> 4);
+                if (elect_one()) {
                     // MMA2 for this tile only, K = BR reduction rows:
                     //   Acc[bp][0:2KP] (+)= Rh [Y^T_hi; Y^T_lo]     (kind::tf32, N = 2 KP, k-steps of 8)
                     //   Acc[bp][0:KP]   += bf16(Rl) bf16(Y)^T      (kind::f16, N = KP, k-steps of 16;
                     //                      column group g of the R warps = k-step g, A at rl + 8 g)
                     // so Acc[0:KP] + Acc[KP:2KP] = Rh Yh + Rh Yl + Rl Y (summed by the
                     // accumulator warps in FP32 registers).
-#pragma unroll
-                    for (int ks = 0; ks < BR / 8; ks++) {
-                        uint32_t const ob = ((ks / 4) * G::YTPAIR + (ks % 4) * 32) >> 4;
-                        mma_ts(dacc, rh + ks * 8, dYT + ob, NTERMS == 3 ? IDESC2W : IDESC2, ks > 0 ? 1u : 0u);
-                    }
+                    // Each MMA truncates its FP32 sums, so the small terms come while the sums are
+                    // still small (after the first k-step, whose MMA also clears Acc[KP:2KP]).
+                    mma_ts<false>(dacc, rh, desc_at(dYT0, oyt), IDESC2);
                     if (NTERMS == 3) {
-                        uint64_t const dYBT = dYBT0 + ((sp * G::YBSTAGE) >> 4);
 #pragma unroll
-                        for (int g = 0; g < BR / 16; g++) mma_ts_bf16(dacc, rl + g * 8, dYBT + g * 2, IDESC2B, 1u);
+                        for (int g = 0; g < BR / 16; g++)
+                            mma_ts_bf16<true>(dacc, rl + g * 8, desc_at(dYBT0, oybt + g * 2), IDESC2B);
                     }
+#pragma unroll
+                    for (int ks = 1; ks < BR / 8; ks++)
+                        mma_ts<true>(dacc, rh + ks * 8, desc_at(dYT0, oyt + (((ks / 4) * G::YTPAIR + (ks % 4) * 32) >> 4)),
+                                     IDESC2);
                     tc_commit(&accrdy[bp]);
                     tc_commit(&yempty[sp]);
                     DBG_TS(3, n2);
-                    n2++;
-                    progressed = true;
                 }
-                if (n1 < T && n1 < n2 + G::NDB && mbar_test(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
-                    tc_fence_after();
-                    uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
-                    uint64_t const dYh = dY0 + ((s * G::YSTAGE) >> 4);
-                    uint32_t const dcol = tmem + G::DA0 + db * BR;
-                    uint32_t const xh = tmem + G::XC0;
-                    // MMA1, K = KP:  D = Xh Yh^T (TF32, k-steps of 8 per column block), then
-                    // D += [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T (K = 2 KP, k-steps of 16:
-                    // the first KP / 16 read bf16(Yl), the rest bf16(Y)).
+                n2++;
+                progressed = true;
+            }
+            if (n1 < T && !x_ok) x_ok = mbar_test_warp(&xready[xs % G::NXB], (xs / G::NXB) & 1);
+            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
+                tc_fence_after();
+                uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
+                uint32_t const dcol = tm + G::DA0 + db * BR;
+                uint32_t const xh = tm + G::XC0 + (xs % G::NXB) * 2 * KP;
+                uint32_t const oy = s * (G::YSTAGE >> 4), oyb = s * (G::YBSTAGE >> 4);
+                bool const last = c1 + 1 == TB;   // the row block's last tile
+                if (elect_one()) {
+                    // MMA1, K = KP: D = the small terms, then += Xh Yh^T (TF32, k-steps of 8 per
+                    // column block).  Small terms: [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T
+                    // (K = 2 KP, k-steps of 16: the first KP / 16 read bf16(Yl), the rest bf16(Y)),
+                    // or Xh Yl^T + Xl Yh^T in TF32.
+                    constexpr int KPB = G::CB / 8;     // k-steps per swizzle column block
+                    if (NTERMS == 3 && G::LO32) {
+                        mma_ts<false>(dcol, xh, desc_at(dYB0, oyb), IDESC1);
+                        mma_ts<true>(dcol, xh + KP, desc_at(dY0, oy), IDESC1);
 #pragma unroll
-                    for (int ks = 0; ks < KP / 8; ks++) {
-                        constexpr int KPB = G::CB / 8;     // k-steps per swizzle column block
-                        uint32_t const ob = ((ks / KPB) * G::YBLK + (ks % KPB) * 32) >> 4;
-                        mma_ts(dcol, xh + ks * 8, dYh + ob, IDESC1, ks > 0 ? 1u : 0u);
-                    }
-                    if (NTERMS == 3) {
-                        uint64_t const dYB = dYB0 + ((s * G::YBSTAGE) >> 4);
-#pragma unroll
-                        for (int j = 0; j < KP / 8; j++) {
-                            uint32_t const ob = ((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4;
-                            mma_ts_bf16(dcol, tmem + G::XB0 + j * 8, dYB + ob, IDESC1B, 1u);
+                        for (int ks = 1; ks < KP / 8; ks++) {
+                            mma_ts<true>(dcol, xh + ks * 8, desc_at(dYB0, oyb + ks * 2), IDESC1);
+                            mma_ts<true>(dcol, xh + KP + ks * 8, desc_at(dY0, oy + ks * 2), IDESC1);
                         }
+                    } else if (NTERMS == 3) {
+                        mma_ts_bf16<false>(dcol, xh + KP, desc_at(dYB0, oyb), IDESC1B);
+#pragma unroll
+                        for (int j = 1; j < KP / 8; j++)
+                            mma_ts_bf16<true>(dcol, xh + KP + j * 8,
+                                              desc_at(dYB0, oyb + (((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4)),
+                                              IDESC1B);
                     }
+                    mma_ts<NTERMS == 3>(dcol, xh, desc_at(dY0, oy), IDESC1);
+#pragma unroll
+                    for (int ks = 1; ks < KP / 8; ks++)
+                        mma_ts<true>(dcol, xh + ks * 8, desc_at(dY0, oy + (((ks / KPB) * G::YBLK + (ks % KPB) * 32) >> 4)),
+                                     IDESC1);
                     tc_commit(&dfull[db]);
+                    if (last) tc_commit(&xfree[xs % G::NXB]);
                     DBG_TS(2, n1);
-                    n1++;
-                    progressed = true;
                 }
-                if (progressed) {
-                    last = globaltimer();
-                } else if (*abort_flag) {
+                n1++;
+                c1 = last ? 0 : c1 + 1;
+                xs += last;
+                x_ok = !last;
+                progressed = true;
+            }
+            if (progressed) {
+                limit.reset();
+            } else {
+                bool const stop = *abort_flag != 0, late = limit.expired();
+                if (__any_sync(0xffffffffu, stop || late)) {
+                    if (!stop && lane == 0) {
+                        *abort_flag = 1;
+                        atomicExch(args.err, 4u);
+                    }
                     ok = false;
-                } else if (globaltimer() - last > args.wait_ns) {
-                    *abort_flag = 1;
-                    atomicExch(args.err, 4u);
-                    ok = false;
-                } else {
-                    __nanosleep(0);
                 }
             }
-            // drain: every MMA issued above has completed (and with it its reads of
-            // shared memory and writes of tensor memory) before the CTA frees them
-            mma_drain(mdrain);
         }
+        // drain: every MMA issued above has completed (and with it its reads of
+        // shared memory and writes of tensor memory) before the CTA frees them
+        if (elect_one()) mma_drain(mdrain);
+        __syncwarp();
     } else if (warp >= 4 && warp < 4 + NR) {
         // ------------------------------------------------------------ R warps
         // Two teams of NR/2 warps take alternate tiles (team 0 even, team 1 odd), so
@@ -488,22 +527,24 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
         for (uint32_t t = team; t < T; t += 2) {
             uint32_t const s = t % G::VST, b = t % G::NDB;
+            uint32_t const c = (c00 + t) % TB;            // reduction tile
             if (warp == 4 && lane == 0) DBG_TS(4, t);
             DBG_PH(0, t);
-            if (!mbar_wait(&dfull[b], (t / G::NDB) & 1, abort_flag, args.err, 6u, args.wait_ns)) break;
+            if (!mbar_wait_warp(&dfull[b], (t / G::NDB) & 1, abort_flag, args.err, 6u, args.wait_ns)) break;
             DBG_PH(1, t);
-            if (!mbar_wait(&vfull[s], (t / G::VST) & 1, abort_flag, args.err, 7u, args.wait_ns)) break;
+            if (!mbar_wait_warp(&vfull[s], (t / G::VST) & 1, abort_flag, args.err, 7u, args.wait_ns)) break;
             tc_fence_after();
             DBG_PH(2, t);
             if (warp == 4 && lane == 0) DBG_TS(5, t);
             const unsigned char *sv = sV + s * G::VBYTES;
-            bool const edge = (t_begin + t + 1) * BR > args.R;   // the partial last reduction tile
-            int const valid = (int)(args.R - (t_begin + t) * BR);          // its columns before R
+            bool const edge = (c + 1) * BR > args.R;      // the partial last reduction tile
+            int const valid = (int)(args.R - c * BR);     // its columns before R
+            bool aborted = false;
 #pragma unroll 1
             for (int ch = 0; ch < CW / 16; ch++) {
                 int const col0 = grp * CW + ch * 16;                          // first tile column of the chunk
                 uint32_t const dcol = G::DA0 + b * BR + col0;                 // its columns of D
-                uint32_t const rlcol = G::RL0 + b * (BR / 2) + (col0 / 16) * 8;  // and of bf16(Rl)
+                uint32_t const rlcol = G::RL0 + (t % G::NRL) * (BR / 2) + (col0 / 16) * 8;  // and of bf16(Rl)
                 uint32_t d[32];   // D, then the TF32 hi part of R
                 uint32_t v[32];   // V, then the lo part of R
                 tmem_ld16(lane_addr + dcol, d);
@@ -525,20 +566,6 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                         v[4 * c + 2] = x.z;
                         v[4 * c + 3] = x.w;
                     }
-                }
-                if (ch == CW / 16 - 1) {
-#ifdef NMFB_FUSED_DEBUG
-                    {   // debug timing only: consume the loaded V values before the next phase mark
-                        uint32_t x = 0;
-#pragma unroll
-                        for (int c = 0; c < 16; c++) x ^= v[c];
-                        asm volatile("" ::"r"(x));
-                        if (x == 0x7fffffffu && dts) dts[0] = x;
-                    }
-#endif
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&vempty[s]);      // V stage consumed (values are in registers)
-                    DBG_PH(3, t);
                 }
                 tmem_wait_ld_dep(d);
                 if (ch == CW / 16 - 1) DBG_PH(4, t);
@@ -577,9 +604,25 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                     for (int j = 0; j < 8; j++) pl[j] = bf16x2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
                 }
                 if (ch == CW / 16 - 1) DBG_PH(5, t);
+                // this team's bf16(Rl) buffer: MMA2 of the team's previous tile has read it
+                // (its commit to accrdy; the next one on that barrier waits for this tile)
+                if (NTERMS == 3 && G::NRL < G::NDB && ch == 0 && t >= 2) {
+                    if (!mbar_wait_warp(&accrdy[t & 1], ((t >> 1) - 1) & 1, abort_flag, args.err, 5u, args.wait_ns)) {
+                        aborted = true;
+                        break;
+                    }
+                    tc_fence_after();
+                }
                 tmem_st16(lane_addr + dcol, d);
                 if (NTERMS == 3) tmem_st8(lane_addr + rlcol, pl);
             }
+            if (aborted) break;
+            // The V stage is released once its values have been used, not when their loads
+            // have been issued: an arrive does not wait for the warp's loads in flight, and
+            // the next TMA load could overwrite the stage under them.
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&vempty[s]);
+            DBG_PH(3, t);
             tmem_wait_st();
             DBG_PH(6, t);
             tc_fence_before();
@@ -594,65 +637,104 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     } else if (warp >= 4 + NR) {
         // ------------------------------------------------------------ accumulator warps
         // Warp 4+NR+q owns TMEM lanes 32q..32q+31: sums the per-tile Acc into FP32
-        // registers, and (all four together) splits X once.
+        // registers, writes the sum at the end of each row block (of this CTA's run
+        // of tiles), and (all four together) splits the X of every row block into
+        // tensor memory, ahead of its tiles as soon as an X buffer is free.
         uint32_t const quad = warp & 3;
         uint32_t const row = quad * 32 + lane;
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
+        uint32_t const nseg = (g0 + T - 1) / TB - ob0 + 1;   // row blocks of the run
         float sum[KP];
 #pragma unroll
         for (int c = 0; c < KP; c++) sum[c] = 0.0f;
-        bool ok = true;
-        if (T > 0) {   // this thread's row of X as TF32 hi and bf16(hi) | bf16(lo), into TMEM lanes = rows
-            uint32_t const o = o0 + row;
+        // this thread's row of X in row block ob0 + xs as TF32 hi and bf16(hi) | bf16(lo), into TMEM lanes = rows
+        auto write_X = [&](uint32_t xs) {
+            uint32_t const o = (ob0 + xs) * BO + row;
             const float *xr = args.X + (size_t)o * KP;
-#pragma unroll
+            uint32_t const xc = lane_addr + G::XC0 + (xs % G::NXB) * 2 * KP;
+#pragma unroll 1   // the sums leave registers for 16 columns at a time
             for (int c0 = 0; c0 < KP; c0 += 16) {
-                uint32_t h[32], hb[8], lb[8];
+                float x[16];
 #pragma unroll
                 for (int c = 0; c < 16; c += 4) {
-                    float4 const x = (o < args.O) ? *reinterpret_cast<const float4 *>(xr + c0 + c)
+                    float4 const v = (o < args.O) ? *reinterpret_cast<const float4 *>(xr + c0 + c)
                                                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                    float const xs[4] = {x.x, x.y, x.z, x.w};
-                    float hv[4], lo[4];
-#pragma unroll
-                    for (int i = 0; i < 4; i++) {
-                        hv[i] = tf32_rna(xs[i]);
-                        h[c + i] = __float_as_uint(hv[i]);
-                        lo[i] = xs[i] - hv[i];
-                    }
-                    hb[c / 2] = bf16x2_rn(hv[0], hv[1]);
-                    hb[c / 2 + 1] = bf16x2_rn(hv[2], hv[3]);
-                    lb[c / 2] = bf16x2_rn(lo[0], lo[1]);
-                    lb[c / 2 + 1] = bf16x2_rn(lo[2], lo[3]);
+                    x[c] = v.x;
+                    x[c + 1] = v.y;
+                    x[c + 2] = v.z;
+                    x[c + 3] = v.w;
                 }
-                tmem_st16(lane_addr + G::XC0 + c0, h);
-                if (NTERMS == 3) {
-                    tmem_st8(lane_addr + G::XB0 + c0 / 2, hb);
-                    tmem_st8(lane_addr + G::XB0 + KP / 2 + c0 / 2, lb);
+                uint32_t h[8], b8[8];
+#pragma unroll
+                for (int half = 0; half < 2; half++) {
+#pragma unroll
+                    for (int c = 0; c < 8; c++) h[c] = __float_as_uint(tf32_rna(x[8 * half + c]));
+                    tmem_st8(xc + c0 + 8 * half, h);
+                }
+                if (NTERMS == 3 && G::LO32) {
+#pragma unroll
+                    for (int half = 0; half < 2; half++) {
+#pragma unroll
+                        for (int c = 0; c < 8; c++) h[c] = __float_as_uint(x[8 * half + c] - tf32_rna(x[8 * half + c]));
+                        tmem_st8(xc + KP + c0 + 8 * half, h);
+                    }
+                } else if (NTERMS == 3) {
+#pragma unroll
+                    for (int c = 0; c < 8; c++) b8[c] = bf16x2_rn(tf32_rna(x[2 * c]), tf32_rna(x[2 * c + 1]));
+                    tmem_st8(xc + KP + c0 / 2, b8);
+#pragma unroll
+                    for (int c = 0; c < 8; c++)
+                        b8[c] = bf16x2_rn(x[2 * c] - tf32_rna(x[2 * c]), x[2 * c + 1] - tf32_rna(x[2 * c + 1]));
+                    tmem_st8(xc + KP + KP / 2 + c0 / 2, b8);
                 }
             }
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(xready);
-        }
+            if (lane == 0) mbar_arrive(&xready[xs % G::NXB]);
+        };
+        bool ok = true;
+        uint32_t xw = 0, ob = ob0, c1 = c00;   // X blocks written; row block and reduction tile of t
+        bool gap_done = c00 == 0 || c00 % args.ts.run != 0;
         for (uint32_t t = 0; ok && t < T; t++) {
             uint32_t const bp = t & 1;
-            if (!mbar_wait(&accrdy[bp], (t >> 1) & 1, abort_flag, args.err, 8u, args.wait_ns)) { ok = false; break; }
-            tc_fence_after();
-            // Acc columns [0, KP) and, for the 3-term arm, [KP, 2 KP) both add to sum.
-#pragma unroll
-            for (int part = 0; part < (NTERMS == 3 ? 2 : 1); part++) {
-#pragma unroll
-                for (int c0 = 0; c0 < KP; c0 += 32) {
-                    uint32_t a[32];
-                    if (KP - c0 >= 32) tmem_ld32(lane_addr + bp * ACC_COLS + part * KP + c0, a);
-                    else tmem_ld16(lane_addr + bp * ACC_COLS + part * KP + c0, a);
-                    tmem_wait_ld_dep(a);
-#pragma unroll
-                    for (int c = 0; c < 32; c++)
-                        if (c0 + c < KP) sum[c0 + c] += __uint_as_float(a[c]);
+            PollLimit limit(args.wait_ns);
+            for (;;) {
+                // the next row block's X first: MMA1 of its first tile waits for it
+                if (xw < nseg &&
+                    (xw < G::NXB || __all_sync(0xffffffffu, mbar_test(&xfree[xw % G::NXB], ((xw / G::NXB) - 1) & 1)))) {
+                    tc_fence_after();
+                    write_X(xw);
+                    xw++;
+                    limit.reset();
+                    continue;
                 }
+                if (__all_sync(0xffffffffu, mbar_try_wait(&accrdy[bp], (t >> 1) & 1))) break;
+                bool const stop = *abort_flag != 0;
+                bool const late = limit.expired();
+                if (__any_sync(0xffffffffu, stop || late)) {
+                    if (!stop && lane == 0) {
+                        *abort_flag = 1;
+                        atomicExch(args.err, 8u);
+                    }
+                    ok = false;
+                    break;
+                }
+            }
+            if (!ok) break;
+            tc_fence_after();
+            // Acc columns [0, KP) plus, for the 3-term arm, [KP, 2 KP): the tile's sum, added
+            // to the running one in one rounding.
+#pragma unroll
+            for (int c0 = 0; c0 < KP; c0 += 16) {
+                uint32_t a[32], a2[32];
+                tmem_ld16(lane_addr + bp * ACC_COLS + c0, a);
+                if (NTERMS == 3) tmem_ld16(lane_addr + bp * ACC_COLS + KP + c0, a2);
+                tmem_wait_ld_dep16(a);
+                if (NTERMS == 3) tmem_wait_ld_dep16(a2);
+#pragma unroll
+                for (int c = 0; c < 16; c++)
+                    sum[c0 + c] += NTERMS == 3 ? __uint_as_float(a[c]) + __uint_as_float(a2[c]) : __uint_as_float(a[c]);
             }
             tc_fence_before();
             __syncwarp();
@@ -660,21 +742,29 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             if (warp == 4 + NR && lane == 0) DBG_TS(7, t);
 #ifdef NMFB_FUSED_DEBUG
             if (lane == 0 && dts && blockIdx.x == 0 && t < 64) dts[1024 + (warp - 4 - NR) * 64 + t] = globaltimer() - ts0;
+            if (args.dbg && blockIdx.x == 0 && t + 1 == T)
+                for (int c = 0; c < KP; c++) args.dbg[3 * BO * 64 + row * KP + c] = sum[c];
 #endif
-        }
-#ifdef NMFB_FUSED_DEBUG
-        if (ok && args.dbg && blockIdx.x == 0)
-            for (int c = 0; c < KP; c++) args.dbg[3 * BO * 64 + row * KP + c] = sum[c];
-#endif
-        // this split's partial (zero for an idle split); k_finish sums the splits
-        if (ok) {
-            uint32_t const o = o0 + row;
-            if (o < args.O) {
-                float *dst = args.part + ((size_t)split * args.O + o) * KP;
+            bool const done = c1 + 1 == TB;   // the row block's last tile
+            if (done || t + 1 == T || (c1 + 1) % args.ts.run == 0) {   // a partial of the row block
+                uint32_t const o = ob * BO + row;
+                if (o < args.O) {
+                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP;
 #pragma unroll
-                for (int c = 0; c < KP; c += 4)
-                    *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                    for (int c = 0; c < KP; c += 4)
+                        *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                    if (!gap_done) {   // the unused slot (TileSplit::slot)
+                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP;
+#pragma unroll
+                        for (int c = 0; c < KP; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    }
+                }
+                gap_done = true;
+#pragma unroll
+                for (int c = 0; c < KP; c++) sum[c] = 0.0f;
             }
+            c1 = done ? 0 : c1 + 1;
+            ob += done;
         }
     }
     tc_fence_before();
@@ -719,7 +809,8 @@ int encode_2d(nmfb_ctx *ctx, CUtensorMap *map, const void *base, uint64_t inner,
 
 // Layout of one factor's split copies (k_split_factor's outputs), in one buffer:
 // hi (rows x kp FP32) | transposed hi/lo per 32 rows | bf16(lo) (rows x kp) |
-// bf16(y) (rows x kp) | bf16(y) transposed per br rows.
+// bf16(y) (rows x kp) | bf16(y) transposed per br rows; at kp = 16 lo itself (FP32)
+// in place of bf16(lo) | bf16(y).
 struct SplitLayout {
     size_t t, bl, b, bt, floats;   // offsets in floats (bl, b, bt: start of the BF16 parts)
     uint32_t br, nblk32, nblkbr;
@@ -758,33 +849,13 @@ int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     FusedPlan *plan = (FusedPlan *)ctx->tmaps;
     uint32_t const O = HSIDE ? ctx->m : ctx->n;
     uint32_t const R = HSIDE ? ctx->n : ctx->m;
-    uint32_t const oblocks = (O + BO - 1) / BO;
-    uint32_t const T = (R + BR - 1) / BR;
-    // Splits of the reduction: one CTA per SM at a time, so the launch takes
-    // ceil(CTAs / SMs) waves of (tiles per split + pipeline fill) tile times;
-    // pick the split count that minimises that (fill ~ 6 tiles: TMEM
-    // allocation, X load and split, pipeline ramp, partial write; measured
-    // best among 1, 3 and 6).
-    uint32_t tps = T, best = 0xffffffffu;
-    for (uint32_t want = 1; want <= NMFB_MAX_SPLIT && want <= T; want++) {
-        uint32_t const t_ps = (T + want - 1) / want;
-        uint32_t const ns = (T + t_ps - 1) / t_ps;
-        if ((size_t)ns * O * KP > ctx->part_items) break;
-        uint32_t const waves = (oblocks * ns + (uint32_t)ctx->sm_count - 1) / (uint32_t)ctx->sm_count;
-        uint32_t const cost = waves * (t_ps + 6);
-        if (cost < best) {
-            best = cost;
-            tps = t_ps;
-        }
-    }
-    uint32_t const nsplit = (T + tps - 1) / tps;
-    if ((size_t)nsplit * O * KP > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "fused: partial buffer too small (%u splits)", nsplit);
+    TileSplit const ts = plan_tiles(O, R, BR, (uint32_t)ctx->sm_count, ctx->part_items / KP);
+    if ((size_t)ts.slots * O * KP > ctx->part_items)
+        return nmfb_fail(ctx, NMFB_EINVAL, "fused: partial buffer too small (%u slots)", ts.slots);
     FusedArgs args;
     args.O = O;
     args.R = R;
-    args.tiles_per_split = tps;
-    args.nsplit = nsplit;
+    args.ts = ts;
     args.part = ctx->dPart;
     args.err = plan->dErr;
     args.st = ctx->dState;
@@ -796,7 +867,7 @@ int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     int const main = HSIDE ? 0 : 1;
     int rc = nmfb_prof_begin(ctx, main);
     if (rc) return rc;
-    kern<<<oblocks * nsplit, G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
+    kern<<<ts.ctas(), G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
     NMFB_LAUNCH_CHECK(ctx);
     if ((rc = nmfb_prof_end(ctx, main))) return rc;
 
@@ -804,7 +875,7 @@ int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     float *xsp = HSIDE ? plan->dSplitH : plan->dSplitW;
     SplitLayout const L(O, KP);
     fa.O = O;
-    fa.nsplit = nsplit;
+    fa.ts = ts;
     fa.k = ctx->k;
     fa.adjust = adjust;
     fa.part = ctx->dPart;
@@ -822,12 +893,12 @@ int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     fa.accX = HSIDE ? ctx->dAccH : ctx->dAccW;
     fa.tick = plan->dTick;
     fa.st = ctx->dState;
-    uint32_t const fblocks = fin_blocks(O, fin_rpt(nsplit));
+    uint32_t const fblocks = fin_blocks(O, fin_rpt(ts.slots));
     if (fblocks > plan->csoff || (fblocks + FIN_ECH - 1) / FIN_ECH + 1 > plan->nticks)
         return nmfb_fail(ctx, NMFB_EINVAL, "fused: column-sum buffers too small");
     fin_launch<KP, BR, 0>(fa, ctx->stream);
     NMFB_LAUNCH_CHECK(ctx);
-    return (int)nsplit;
+    return NMFB_OK;
 }
 
 template <bool HSIDE>
@@ -873,8 +944,8 @@ int fused_half(nmfb_ctx *ctx, bool is_H, int adjust)
     if (rc) return rc;
     bool const yw = is_H;   // Y = W for update_H
     if (!ctx->fz_ok[yw ? 0 : 1] && (rc = prepare_factor(ctx, yw))) return rc;
-    int const nsplit = is_H ? dispatch<true>(ctx, plan->mapsH, adjust) : dispatch<false>(ctx, plan->mapsW, adjust);
-    if (nsplit < 0) return nsplit;
+    rc = is_H ? dispatch<true>(ctx, plan->mapsH, adjust) : dispatch<false>(ctx, plan->mapsW, adjust);
+    if (rc) return rc;
     ctx->fz_ok[is_H ? 1 : 0] = 1;
     return nmfb_prof_end(ctx, whole);
 }
@@ -933,8 +1004,11 @@ int nmfb_fused_prepare(nmfb_ctx *ctx)
     auto const y_maps = [&](FusedMaps &mp, const float *sp, const SplitLayout &L, uint32_t rows) -> int {
         int r;
         if ((r = encode_2d(ctx, &mp.y, sp, kp, rows, frow, cb, br, fsw))) return r;
-        if ((r = encode_2d(ctx, &mp.ylb, sp + L.bl, kp, rows, (uint64_t)kp * 2, kp, br, sw_for(2 * kp), BF16)))
-            return r;
+        if (kp == 16)
+            r = encode_2d(ctx, &mp.ylb, sp + L.bl, kp, rows, frow, cb, br, fsw);
+        else
+            r = encode_2d(ctx, &mp.ylb, sp + L.bl, kp, rows, (uint64_t)kp * 2, kp, br, sw_for(2 * kp), BF16);
+        if (r) return r;
         if ((r = encode_2d(ctx, &mp.yt, sp + L.t, 32, (uint64_t)L.nblk32 * 2 * kp, 128, 32, 2 * kp * (br / 32),
                            CU_TENSOR_MAP_SWIZZLE_128B)))
             return r;
