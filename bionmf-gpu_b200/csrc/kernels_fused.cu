@@ -6,7 +6,7 @@
 // without ever materialising the n x m quotient:
 //
 //   TMA      : V tile (128 x BR, FP32) into a VST-deep ring; the Y tile
-//              operands into a YST-deep ring.
+//              operands of MMA1 and of MMA2 into a ring each.
 //   split    : k_split_factor, once per half-iteration, writes the other
 //              factor Y as TF32 hi (round to nearest) and the transposed hi/lo
 //              blocks that MMA2 reads K-major (lo = y - hi, exact; an MN-major
@@ -43,11 +43,11 @@
 // 1014-1164): two cuBLAS SGEMMs around matrix_div_sub with WH in HBM.
 //
 // Warp roles: warp 0 = V producer (TMA), warp 1 = MMA issuer and TMEM owner,
-// warp 2 = Y producer (TMA), warps 4-11 (or 4-19) = R warps in two teams that
-// take alternate tiles (warp w reads TMEM lanes 32*(w%4)..+31), last 4 warps =
-// accumulator and split warps.
-// V stages are released as soon as the epilogue has read them, Y stages when
-// MMA2 (the last reader) has completed.
+// warps 2 and 3 = Y producers (TMA), warps 4-11 (or 4-19) = R warps in two teams that
+// take alternate tiles (warp w reads TMEM lanes 32*(w%4)..+31), last 4 (or 8) warps
+// = accumulator and split warps.
+// V stages are released once the epilogue has used them, Y stages when the MMA
+// that reads them has completed.
 // Every mbarrier wait is bounded (1 s of %globaltimer); on expiry the kernel
 // records an error word that the host turns into NMFB_ETIMEOUT.
 // No TMA multicast is used anywhere.
@@ -128,7 +128,7 @@ struct FusedArgs {
 // ---------------------------------------------------------------------------
 template <int KP>
 struct Geo {
-    static constexpr int BR = (KP >= 64) ? 32 : 64;       // reduction rows per tile
+    static constexpr int BR = 64;                         // reduction rows per tile
     static constexpr int CB = (KP == 16) ? 16 : 32;       // floats per swizzle column block
     static constexpr int NB = KP / CB;                     // column blocks
     static constexpr int ROWB = CB * 4;                    // bytes per row of a block
@@ -138,11 +138,13 @@ struct Geo {
     static constexpr int YTPAIR = 2 * YTBLK;               // Y^T hi part followed by its lo part
     static constexpr int YBYTES = BR * KP * 4;
     static constexpr int VBYTES = BO * BR * 4;
-    static constexpr int YSTAGE = YBYTES;                  // Yh (TF32), NB column blocks
-    static constexpr int YTSTAGE = 2 * YBYTES;             // YTh | YTl (per 32 rows)
+    // Two rings for Y: MMA1's operands (released by MMA1, up to NDB tiles before the
+    // tile's MMA2) and MMA2's.  With one ring for both a stage was held through the
+    // whole distance between the two, and MMA1 could not run ahead of MMA2.
     static constexpr int YBB = BR * KP * 2;                // one BF16 tile of BR rows of 2 KP bytes
     static constexpr int YBTB = KP * BR * 2;               // bf16(Y)^T tile, KP rows of 2 BR bytes
-    static constexpr int YBSTAGE = 2 * YBB + YBTB;         // bf16(Yl) | bf16(Y) | bf16(Y)^T
+    static constexpr int Y1STAGE = YBYTES + 2 * YBB;       // Yh (TF32, NB column blocks) | bf16(Yl) | bf16(Y)
+    static constexpr int Y2STAGE = 2 * YBYTES + YBTB;      // YTh | YTl (per 32 rows) | bf16(Y)^T
     // MMA1's small terms Xh Yl + Xl Y: TF32 at KP = 16 (Xh Yl + Xl Yh, from an FP32 copy of
     // Yl that takes the place of the two BF16 tiles; 2 of 18 MMAs more, and MMAs do not bound
     // the small problems of these ranks), BF16 above (4 of 20 MMAs fewer at KP = 32).
@@ -150,20 +152,25 @@ struct Geo {
     static_assert(!LO32 || YBYTES == 2 * YBB, "the FP32 tile of Yl takes the BF16 tiles' place");
     static constexpr uint32_t BLAYOUT = umma_layout(2 * KP);
     static constexpr uint32_t BTLAYOUT = umma_layout(2 * BR);
-    static constexpr int YST = 3;
+    static constexpr int Y1ST = (KP == 64) ? 2 : 3, Y2ST = 2;   // what is left goes to V
     static constexpr int FIXED = 1024 + 512;
-    static constexpr int YALL = YST * (YSTAGE + YTSTAGE + YBSTAGE);
+    static constexpr int YALL = Y1ST * Y1STAGE + Y2ST * Y2STAGE;
     static constexpr int VAVAIL = (SMEM_LIMIT - FIXED - YALL) / VBYTES;
     static constexpr int VST = VAVAIL > 6 ? 6 : VAVAIL;    // V ring depth (HBM stream)
     static constexpr int SMEM = FIXED + YALL + VST * VBYTES;
-    static_assert(VST >= 3, "shared-memory ring too small");
-    static_assert(YBB % 1024 == 0 && YBSTAGE % 1024 == 0 && YSTAGE % 1024 == 0, "1024-byte stage alignment");
+    static_assert(VST >= 2, "shared-memory ring too small");
+    static_assert(YBB % 1024 == 0 && Y1STAGE % 1024 == 0 && Y2STAGE % 1024 == 0, "1024-byte stage alignment");
     static constexpr int NR = (KP >= 64) ? 8 : 16;        // R warps
-    static constexpr int NTHR = (4 + NR + 4) * 32;
+    // Accumulator warps: sets of four, KP / NA columns each.  At KP = 64 tensor memory
+    // holds one accumulator besides three D buffers, so it has to be read fast.
+    static constexpr int NA = (KP == 64) ? 2 : 1;
+    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;
     static constexpr uint32_t ACC = 2 * KP;                // TMEM columns of one per-tile accumulator
-    static constexpr uint32_t NDB = (KP == 16) ? 4 : (KP == 32) ? 3 : 2;   // D buffers (MMA1 runs NDB tiles ahead)
-    static constexpr uint32_t DA0 = 2 * ACC;               // D[b] (then Rh[b]) at DA0 + b BR
-    static constexpr uint32_t NRL = (KP == 32) ? 2 : NDB;  // bf16(Rl) buffers (2: one per R team)
+    static constexpr uint32_t NACC = (KP == 64) ? 1 : 2;   // accumulators
+    static constexpr uint32_t NDB = (KP == 16) ? 4 : 3;    // D buffers (MMA1 runs NDB tiles ahead)
+    static constexpr uint32_t DA0 = NACC * ACC;            // D[b] (then Rh[b]) at DA0 + b BR
+    static constexpr uint32_t NRL = (KP == 16) ? NDB : 2;  // bf16(Rl) buffers (2: one per R team)
+    static_assert(NRL == NDB || (NRL == 2 && Y2ST == 2), "the R teams wait on y2empty for their Rl buffer");
     static constexpr uint32_t RL0 = DA0 + NDB * BR;        // bf16(Rl)[b] at RL0 + b BR/2
     static constexpr uint32_t NXB = (KP == 64) ? 1 : 2;    // X buffers (2: the next row block's X while this one is read)
     static constexpr uint32_t XC0 = RL0 + NRL * BR / 2;    // X hi (TF32, KP columns) | bf16(X hi) | bf16(X lo)
@@ -171,7 +178,7 @@ struct Geo {
     static_assert(XC0 + NXB * 2 * KP <= 512, "TMEM columns exceeded");
 };
 
-// TMEM columns: per-tile accumulators Acc[b] at b*2KP (2KP columns: the Rh Yh +
+// TMEM columns: per-tile accumulators Acc[b] at b*2KP, b < NACC (2KP columns: the Rh Yh +
 // bf16(Rl) bf16(Y) sum and the Rh Yl part side by side); D[b] (BR columns, then
 // Rh[b]) at DA0 + b*BR, b < NDB; bf16(Rl)[b] (BR/2 columns, column group g of
 // 16 in its 8 columns RL0 + b*BR/2 + 8g), b < NRL; then, per X buffer, a row
@@ -231,8 +238,8 @@ __global__ void __launch_bounds__(256) k_split_factor(const float *__restrict__ 
     for (uint32_t e = threadIdx.x; e < kp * br; e += blockDim.x) bt[e] = tb[e % br][e / br];
 }
 
-// Warp roles: 0 = V producer (TMA), 1 = MMA issuer + TMEM owner, 2 = Y
-// producer (TMA), 3 = idle, 4 .. 3 + NR = R warps (V / D, feed MMA2), last four =
+// Warp roles: 0 = V producer (TMA), 1 = MMA issuer + TMEM owner, 2, 3 = Y
+// producers (TMA), 4 .. 3 + NR = R warps (V / D, feed MMA2), the others =
 // accumulator warps (sum the per-tile MMA2 results in FP32 registers; split X).
 //
 // Persistent, one CTA per SM: the tiles of all row blocks form one list and
@@ -252,20 +259,21 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     extern __shared__ unsigned char smem_raw[];
     uint32_t const base_u32 = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *const base = smem_raw + (base_u32 - smem_u32(smem_raw));
-    unsigned char *const sY = base;                                 // [YST][Yh | Yl]
-    unsigned char *const sYT = sY + G::YST * G::YSTAGE;             // [YST][YTh | YTl]
-    unsigned char *const sYB = sYT + G::YST * G::YTSTAGE;           // [YST][bf16 Y | bf16 Y^T]
-    unsigned char *const sV = sYB + G::YST * G::YBSTAGE;            // [VST][VBYTES]
+    unsigned char *const sY1 = base;                                // [Y1ST][Yh | bf16 Yl | bf16 Y]
+    unsigned char *const sY2 = sY1 + G::Y1ST * G::Y1STAGE;          // [Y2ST][YTh | YTl | bf16 Y^T]
+    unsigned char *const sV = sY2 + G::Y2ST * G::Y2STAGE;           // [VST][VBYTES]
     uint64_t *const bars = reinterpret_cast<uint64_t *>(sV + G::VST * G::VBYTES);
     uint64_t *const vfull = bars;                   // [VST]  TMA -> epilogue
     uint64_t *const vempty = vfull + G::VST;        // [VST]  epilogue -> V producer
-    uint64_t *const yfull = vempty + G::VST;        // [YST]  TMA (Yh, Yl, Y^T) -> MMA1 / MMA2
-    uint64_t *const yempty = yfull + G::YST;        // [YST]  MMA2 commit -> Y producer
-    uint64_t *const dfull = yempty + G::YST;        // [NDB]  MMA1 commit -> R warps
+    uint64_t *const y1full = vempty + G::VST;       // [Y1ST] TMA -> MMA1
+    uint64_t *const y1empty = y1full + G::Y1ST;     // [Y1ST] MMA1 commit -> Y1 producer
+    uint64_t *const y2full = y1empty + G::Y1ST;     // [Y2ST] TMA -> MMA2
+    uint64_t *const y2empty = y2full + G::Y2ST;     // [Y2ST] MMA2 commit -> Y2 producer
+    uint64_t *const dfull = y2empty + G::Y2ST;      // [NDB]  MMA1 commit -> R warps
     uint64_t *const rfull = dfull + G::NDB;         // [NDB]  R warps -> MMA2
-    uint64_t *const accrdy = rfull + G::NDB;        // [2]    MMA2 commit -> accumulator warps
-    uint64_t *const accfree = accrdy + 2;           // [2]    accumulator warps -> MMA2
-    uint64_t *const xready = accfree + 2;           // [NXB]  X split into TMEM -> MMA1
+    uint64_t *const accrdy = rfull + G::NDB;        // [NACC] MMA2 commit -> accumulator warps
+    uint64_t *const accfree = accrdy + G::NACC;     // [NACC] accumulator warps -> MMA2
+    uint64_t *const xready = accfree + G::NACC;     // [NXB]  X split into TMEM -> MMA1
     uint64_t *const xfree = xready + G::NXB;        // [NXB]  last MMA1 of a row block -> accumulator warps
     uint64_t *const mdrain = xfree + G::NXB;        // [1]    issuer's final commit (drain)
     uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(mdrain + 1);
@@ -301,20 +309,24 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             mbar_init(&vfull[s], 1);
             mbar_init(&vempty[s], NR / 2);   // one team reads each V tile
         }
-        for (int s = 0; s < G::YST; s++) {
-            mbar_init(&yfull[s], 1);
-            mbar_init(&yempty[s], 1);
+        for (int s = 0; s < G::Y1ST; s++) {
+            mbar_init(&y1full[s], 1);
+            mbar_init(&y1empty[s], 1);
+        }
+        for (int s = 0; s < G::Y2ST; s++) {
+            mbar_init(&y2full[s], 1);
+            mbar_init(&y2empty[s], 1);
         }
         for (uint32_t b = 0; b < G::NDB; b++) {
             mbar_init(&dfull[b], 1);
             mbar_init(&rfull[b], NR / 2);
         }
-        for (int b = 0; b < 2; b++) {
+        for (uint32_t b = 0; b < G::NACC; b++) {
             mbar_init(&accrdy[b], 1);
-            mbar_init(&accfree[b], 4);
+            mbar_init(&accfree[b], 4 * G::NA);
         }
         for (uint32_t b = 0; b < G::NXB; b++) {
-            mbar_init(&xready[b], 4);
+            mbar_init(&xready[b], 4 * G::NA);
             mbar_init(&xfree[b], 1);
         }
         mbar_init(mdrain, 1);
@@ -360,54 +372,61 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             for (uint32_t t = issued > (uint32_t)G::VST ? issued - G::VST : 0; t < issued; t++)
                 mbar_drain(&vfull[t % G::VST], (t / G::VST) & 1);
         }
-    } else if (warp == 2) {
-        // ------------------------------------------------------------ Y producer
+    } else if (warp == 2 || warp == 3) {
+        // ------------------------------------------------------------ Y producers
+        // warp 2: MMA1's operands, warp 3: MMA2's
         if (lane == 0) {
+            bool const one = warp == 2;
             uint64_t const pol = policy_evict_last();
-            uint32_t issued = 0, c = c00;
+            uint64_t *const full = one ? y1full : y2full, *const empty = one ? y1empty : y2empty;
+            uint32_t const nst = one ? G::Y1ST : G::Y2ST;
+            uint32_t issued = 0, c = c00, s = 0, ph = 0;   // stage and its phase
             for (uint32_t t = 0; t < T; t++, c = (c + 1 == TB) ? 0 : c + 1) {
-                uint32_t const s = t % G::YST;
-                if (t >= (uint32_t)G::YST &&
-                    !mbar_wait(&yempty[s], ((t / G::YST) - 1) & 1, abort_flag, args.err, 2u, args.wait_ns))
-                    break;
+                if (t >= nst && !mbar_wait(&empty[s], ph ^ 1, abort_flag, args.err, 2u, args.wait_ns)) break;
                 issued = t + 1;
-                unsigned char *syh = sY + s * G::YSTAGE;
                 int const r0 = (int)(c * BR);
-                DBG_TS(1, t);
-                mbar_expect_tx(&yfull[s], G::YBYTES + G::YTSTAGE + (NTERMS == 3 ? G::YBSTAGE : 0));
-                for (int b = 0; b < G::NB; b++) tma_load_2d(syh + b * G::YBLK, &maps.y, &yfull[s], b * G::CB, r0, pol);
-                if (NTERMS == 3) {
-                    unsigned char *syb = sYB + s * G::YBSTAGE;
-                    tma_load_2d(syb, &maps.ylb, &yfull[s], 0, r0, pol);
-                    if (!G::LO32) tma_load_2d(syb + G::YBB, &maps.yb, &yfull[s], 0, r0, pol);
-                    tma_load_2d(syb + 2 * G::YBB, &maps.ybt, &yfull[s], 0, (int)(c * KP), pol);
+                if (one) {
+                    unsigned char *sy = sY1 + s * G::Y1STAGE;
+                    DBG_TS(1, t);
+                    mbar_expect_tx(&full[s], G::YBYTES + (NTERMS == 3 ? 2 * G::YBB : 0));
+                    for (int b = 0; b < G::NB; b++) tma_load_2d(sy + b * G::YBLK, &maps.y, &full[s], b * G::CB, r0, pol);
+                    if (NTERMS == 3) {
+                        tma_load_2d(sy + G::YBYTES, &maps.ylb, &full[s], 0, r0, pol);
+                        if (!G::LO32) tma_load_2d(sy + G::YBYTES + G::YBB, &maps.yb, &full[s], 0, r0, pol);
+                    }
+                } else {
+                    unsigned char *sy = sY2 + s * G::Y2STAGE;
+                    mbar_expect_tx(&full[s], 2 * G::YBYTES + (NTERMS == 3 ? G::YBTB : 0));
+                    // Y^T: the BR / 32 row blocks of this tile, 2 KP rows of 128 B each
+                    tma_load_2d(sy, &maps.yt, &full[s], 0, (r0 / 32) * 2 * KP, pol);
+                    if (NTERMS == 3) tma_load_2d(sy + 2 * G::YBYTES, &maps.ybt, &full[s], 0, (int)(c * KP), pol);
                 }
-                // Y^T: the BR / 32 row blocks of this tile, 2 KP rows of 128 B each
-                tma_load_2d(sYT + s * G::YTSTAGE, &maps.yt, &yfull[s], 0, (r0 / 32) * 2 * KP, pol);
+                if (++s == nst) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
-            for (uint32_t t = issued > (uint32_t)G::YST ? issued - G::YST : 0; t < issued; t++)
-                mbar_drain(&yfull[t % G::YST], (t / G::YST) & 1);
+            for (uint32_t t = issued > nst ? issued - nst : 0; t < issued; t++) mbar_drain(&full[t % nst], (t / nst) & 1);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         // Two issue queues, polled without blocking:
-        //   MMA2(n2): needs the R warps' R(n2) and, for n2 >= 2, the accumulator
-        //             warps to have read Acc[n2 % 2] of tile n2-2;
-        //   MMA1(n1): needs Y(n1) loaded and a free D buffer (MMA2(n1-NDB)
+        //   MMA2(n2): needs the R warps' R(n2), its Y operands and, for n2 >= NACC, the
+        //             accumulator warps to have read Acc[n2 % NACC] of tile n2-NACC;
+        //   MMA1(n1): needs its Y operands and a free D buffer (MMA2(n1-NDB)
         //             issued, i.e. n1 < n2 + NDB); A = X from TMEM, which for the
         //             first tile of a row block has to be ready, and whose buffer the
         //             last one's MMA1 releases.
-        // The Y stage of tile t is released when MMA2(t), the last reader, completes.
         constexpr uint32_t IDESC1 = idesc_tf32(BO, BR, 0);
         constexpr uint32_t IDESC1B = idesc_bf16xf32(BO, BR);
         constexpr uint32_t IDESC2 = NTERMS == 3 ? idesc_tf32(BO, 2 * KP, 0) : idesc_tf32(BO, KP, 0);
         constexpr uint32_t IDESC2B = idesc_bf16xf32(BO, KP);
         uint64_t const dY0 = smem_desc(base_u32, 16, 8 * G::ROWB, G::LAYOUT);
-        uint64_t const dYT0 = smem_desc(base_u32 + G::YST * G::YSTAGE, 16, 1024, 2u);
-        uint32_t const yb_u32 = base_u32 + G::YST * (G::YSTAGE + G::YTSTAGE);
-        uint64_t const dYB0 = G::LO32 ? smem_desc(yb_u32, 16, 8 * G::ROWB, G::LAYOUT)
-                                      : smem_desc(yb_u32, 16, 8 * 2 * KP, G::BLAYOUT);
-        uint64_t const dYBT0 = smem_desc(yb_u32 + 2 * G::YBB, 16, 8 * 2 * BR, G::BTLAYOUT);
+        uint64_t const dYB0 = G::LO32 ? smem_desc(base_u32 + G::YBYTES, 16, 8 * G::ROWB, G::LAYOUT)
+                                      : smem_desc(base_u32 + G::YBYTES, 16, 8 * 2 * KP, G::BLAYOUT);
+        uint32_t const y2_u32 = base_u32 + G::Y1ST * G::Y1STAGE;
+        uint64_t const dYT0 = smem_desc(y2_u32, 16, 1024, 2u);
+        uint64_t const dYBT0 = smem_desc(y2_u32 + 2 * G::YBYTES, 16, 8 * 2 * BR, G::BTLAYOUT);
         uint32_t const tm = uniform(tmem);
         bool ok = true, x_ok = false;
         uint32_t n1 = 0, n2 = 0, c1 = c00, xs = 0;   // c1: reduction tile of n1; xs: its row block, counted from the CTA's first
@@ -415,13 +434,14 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         while (ok && n2 < T) {
             bool progressed = false;
             if (n2 < n1 && mbar_test_warp(&rfull[n2 % G::NDB], (n2 / G::NDB) & 1) &&
-                (n2 < 2 || mbar_test_warp(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
+                mbar_test_warp(&y2full[n2 % G::Y2ST], (n2 / G::Y2ST) & 1) &&
+                (n2 < G::NACC || mbar_test_warp(&accfree[n2 % G::NACC], ((n2 / G::NACC) - 1) & 1))) {
                 tc_fence_after();
-                uint32_t const sp = n2 % G::YST, bp = n2 & 1, db = n2 % G::NDB;
+                uint32_t const sp = n2 % G::Y2ST, bp = n2 % G::NACC, db = n2 % G::NDB;
                 uint32_t const rh = tm + G::DA0 + db * BR;
                 uint32_t const rl = tm + G::RL0 + (n2 % G::NRL) * (BR / 2);
                 uint32_t const dacc = tm + bp * ACC_COLS;
-                uint32_t const oyt = sp * (G::YTSTAGE >> 4), oybt = sp * (G::YBSTAGE >> 4);
+                uint32_t const oy = sp * (G::Y2STAGE >> 4);
                 if (elect_one()) {
                     // MMA2 for this tile only, K = BR reduction rows:
                     //   Acc[bp][0:2KP] (+)= Rh [Y^T_hi; Y^T_lo]     (kind::tf32, N = 2 KP, k-steps of 8)
@@ -431,30 +451,30 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                     // accumulator warps in FP32 registers).
                     // Each MMA truncates its FP32 sums, so the small terms come while the sums are
                     // still small (after the first k-step, whose MMA also clears Acc[KP:2KP]).
-                    mma_ts<false>(dacc, rh, desc_at(dYT0, oyt), IDESC2);
+                    mma_ts<false>(dacc, rh, desc_at(dYT0, oy), IDESC2);
                     if (NTERMS == 3) {
 #pragma unroll
                         for (int g = 0; g < BR / 16; g++)
-                            mma_ts_bf16<true>(dacc, rl + g * 8, desc_at(dYBT0, oybt + g * 2), IDESC2B);
+                            mma_ts_bf16<true>(dacc, rl + g * 8, desc_at(dYBT0, oy + g * 2), IDESC2B);
                     }
 #pragma unroll
                     for (int ks = 1; ks < BR / 8; ks++)
-                        mma_ts<true>(dacc, rh + ks * 8, desc_at(dYT0, oyt + (((ks / 4) * G::YTPAIR + (ks % 4) * 32) >> 4)),
+                        mma_ts<true>(dacc, rh + ks * 8, desc_at(dYT0, oy + (((ks / 4) * G::YTPAIR + (ks % 4) * 32) >> 4)),
                                      IDESC2);
                     tc_commit(&accrdy[bp]);
-                    tc_commit(&yempty[sp]);
+                    tc_commit(&y2empty[sp]);
                     DBG_TS(3, n2);
                 }
                 n2++;
                 progressed = true;
             }
             if (n1 < T && !x_ok) x_ok = mbar_test_warp(&xready[xs % G::NXB], (xs / G::NXB) & 1);
-            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
+            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&y1full[n1 % G::Y1ST], (n1 / G::Y1ST) & 1)) {
                 tc_fence_after();
-                uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
+                uint32_t const s = n1 % G::Y1ST, db = n1 % G::NDB;
                 uint32_t const dcol = tm + G::DA0 + db * BR;
                 uint32_t const xh = tm + G::XC0 + (xs % G::NXB) * 2 * KP;
-                uint32_t const oy = s * (G::YSTAGE >> 4), oyb = s * (G::YBSTAGE >> 4);
+                uint32_t const oy = s * (G::Y1STAGE >> 4);
                 bool const last = c1 + 1 == TB;   // the row block's last tile
                 if (elect_one()) {
                     // MMA1, K = KP: D = the small terms, then += Xh Yh^T (TF32, k-steps of 8 per
@@ -463,19 +483,19 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                     // or Xh Yl^T + Xl Yh^T in TF32.
                     constexpr int KPB = G::CB / 8;     // k-steps per swizzle column block
                     if (NTERMS == 3 && G::LO32) {
-                        mma_ts<false>(dcol, xh, desc_at(dYB0, oyb), IDESC1);
+                        mma_ts<false>(dcol, xh, desc_at(dYB0, oy), IDESC1);
                         mma_ts<true>(dcol, xh + KP, desc_at(dY0, oy), IDESC1);
 #pragma unroll
                         for (int ks = 1; ks < KP / 8; ks++) {
-                            mma_ts<true>(dcol, xh + ks * 8, desc_at(dYB0, oyb + ks * 2), IDESC1);
+                            mma_ts<true>(dcol, xh + ks * 8, desc_at(dYB0, oy + ks * 2), IDESC1);
                             mma_ts<true>(dcol, xh + KP + ks * 8, desc_at(dY0, oy + ks * 2), IDESC1);
                         }
                     } else if (NTERMS == 3) {
-                        mma_ts_bf16<false>(dcol, xh + KP, desc_at(dYB0, oyb), IDESC1B);
+                        mma_ts_bf16<false>(dcol, xh + KP, desc_at(dYB0, oy), IDESC1B);
 #pragma unroll
                         for (int j = 1; j < KP / 8; j++)
                             mma_ts_bf16<true>(dcol, xh + KP + j * 8,
-                                              desc_at(dYB0, oyb + (((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4)),
+                                              desc_at(dYB0, oy + (((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4)),
                                               IDESC1B);
                     }
                     mma_ts<NTERMS == 3>(dcol, xh, desc_at(dY0, oy), IDESC1);
@@ -484,6 +504,7 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                         mma_ts<true>(dcol, xh + ks * 8, desc_at(dY0, oy + (((ks / KPB) * G::YBLK + (ks % KPB) * 32) >> 4)),
                                      IDESC1);
                     tc_commit(&dfull[db]);
+                    tc_commit(&y1empty[s]);
                     if (last) tc_commit(&xfree[xs % G::NXB]);
                     DBG_TS(2, n1);
                 }
@@ -605,9 +626,9 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                 }
                 if (ch == CW / 16 - 1) DBG_PH(5, t);
                 // this team's bf16(Rl) buffer: MMA2 of the team's previous tile has read it
-                // (its commit to accrdy; the next one on that barrier waits for this tile)
+                // (its commit to y2empty; the next one on that barrier waits for this tile)
                 if (NTERMS == 3 && G::NRL < G::NDB && ch == 0 && t >= 2) {
-                    if (!mbar_wait_warp(&accrdy[t & 1], ((t >> 1) - 1) & 1, abort_flag, args.err, 5u, args.wait_ns)) {
+                    if (!mbar_wait_warp(&y2empty[t & 1], ((t >> 1) - 1) & 1, abort_flag, args.err, 5u, args.wait_ns)) {
                         aborted = true;
                         break;
                     }
@@ -636,24 +657,26 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         }
     } else if (warp >= 4 + NR) {
         // ------------------------------------------------------------ accumulator warps
-        // Warp 4+NR+q owns TMEM lanes 32q..32q+31: sums the per-tile Acc into FP32
-        // registers, writes the sum at the end of each row block (of this CTA's run
-        // of tiles), and (all four together) splits the X of every row block into
-        // tensor memory, ahead of its tiles as soon as an X buffer is free.
+        // Warp 4+NR+4a+q owns TMEM lanes 32q..32q+31 and columns KC a..KC a + KC - 1: sums
+        // the per-tile Acc into FP32 registers, writes the sum at the end of each row
+        // block (of this CTA's run of tiles), and (all together) splits the X of every
+        // row block into tensor memory, ahead of its tiles as soon as an X buffer is free.
+        constexpr int KC = KP / G::NA;
         uint32_t const quad = warp & 3;
+        uint32_t const k0 = ((warp - 4 - NR) >> 2) * KC;   // first column
         uint32_t const row = quad * 32 + lane;
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
         uint32_t const nseg = (g0 + T - 1) / TB - ob0 + 1;   // row blocks of the run
-        float sum[KP];
+        float sum[KC];
 #pragma unroll
-        for (int c = 0; c < KP; c++) sum[c] = 0.0f;
-        // this thread's row of X in row block ob0 + xs as TF32 hi and bf16(hi) | bf16(lo), into TMEM lanes = rows
+        for (int c = 0; c < KC; c++) sum[c] = 0.0f;
+        // this thread's part of its row of X in row block ob0 + xs as TF32 hi and bf16(hi) | bf16(lo), into TMEM lanes = rows
         auto write_X = [&](uint32_t xs) {
             uint32_t const o = (ob0 + xs) * BO + row;
             const float *xr = args.X + (size_t)o * KP;
             uint32_t const xc = lane_addr + G::XC0 + (xs % G::NXB) * 2 * KP;
 #pragma unroll 1   // the sums leave registers for 16 columns at a time
-            for (int c0 = 0; c0 < KP; c0 += 16) {
+            for (uint32_t c0 = k0; c0 < k0 + KC; c0 += 16) {
                 float x[16];
 #pragma unroll
                 for (int c = 0; c < 16; c += 4) {
@@ -697,7 +720,7 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
         uint32_t xw = 0, ob = ob0, c1 = c00;   // X blocks written; row block and reduction tile of t
         bool gap_done = c00 == 0 || c00 % args.ts.run != 0;
         for (uint32_t t = 0; ok && t < T; t++) {
-            uint32_t const bp = t & 1;
+            uint32_t const bp = t % G::NACC;
             PollLimit limit(args.wait_ns);
             for (;;) {
                 // the next row block's X first: MMA1 of its first tile waits for it
@@ -709,7 +732,7 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                     limit.reset();
                     continue;
                 }
-                if (__all_sync(0xffffffffu, mbar_try_wait(&accrdy[bp], (t >> 1) & 1))) break;
+                if (__all_sync(0xffffffffu, mbar_try_wait(&accrdy[bp], (t / G::NACC) & 1))) break;
                 bool const stop = *abort_flag != 0;
                 bool const late = limit.expired();
                 if (__any_sync(0xffffffffu, stop || late)) {
@@ -726,10 +749,10 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             // Acc columns [0, KP) plus, for the 3-term arm, [KP, 2 KP): the tile's sum, added
             // to the running one in one rounding.
 #pragma unroll
-            for (int c0 = 0; c0 < KP; c0 += 16) {
+            for (int c0 = 0; c0 < KC; c0 += 16) {
                 uint32_t a[32], a2[32];
-                tmem_ld16(lane_addr + bp * ACC_COLS + c0, a);
-                if (NTERMS == 3) tmem_ld16(lane_addr + bp * ACC_COLS + KP + c0, a2);
+                tmem_ld16(lane_addr + bp * ACC_COLS + k0 + c0, a);
+                if (NTERMS == 3) tmem_ld16(lane_addr + bp * ACC_COLS + KP + k0 + c0, a2);
                 tmem_wait_ld_dep16(a);
                 if (NTERMS == 3) tmem_wait_ld_dep16(a2);
 #pragma unroll
@@ -743,25 +766,25 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
 #ifdef NMFB_FUSED_DEBUG
             if (lane == 0 && dts && blockIdx.x == 0 && t < 64) dts[1024 + (warp - 4 - NR) * 64 + t] = globaltimer() - ts0;
             if (args.dbg && blockIdx.x == 0 && t + 1 == T)
-                for (int c = 0; c < KP; c++) args.dbg[3 * BO * 64 + row * KP + c] = sum[c];
+                for (int c = 0; c < KC; c++) args.dbg[3 * BO * 64 + row * KP + k0 + c] = sum[c];
 #endif
             bool const done = c1 + 1 == TB;   // the row block's last tile
             if (done || t + 1 == T || (c1 + 1) % args.ts.run == 0) {   // a partial of the row block
                 uint32_t const o = ob * BO + row;
                 if (o < args.O) {
-                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP;
+                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP + k0;
 #pragma unroll
-                    for (int c = 0; c < KP; c += 4)
+                    for (int c = 0; c < KC; c += 4)
                         *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
                     if (!gap_done) {   // the unused slot (TileSplit::slot)
-                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP;
+                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP + k0;
 #pragma unroll
-                        for (int c = 0; c < KP; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                 }
                 gap_done = true;
 #pragma unroll
-                for (int c = 0; c < KP; c++) sum[c] = 0.0f;
+                for (int c = 0; c < KC; c++) sum[c] = 0.0f;
             }
             c1 = done ? 0 : c1 + 1;
             ob += done;
@@ -816,7 +839,7 @@ struct SplitLayout {
     uint32_t br, nblk32, nblkbr;
     SplitLayout(uint32_t rows, uint32_t kp)
     {
-        br = (kp >= 64) ? 32 : 64;
+        br = 64;
         nblk32 = (rows + 31) / 32;
         nblkbr = (rows + br - 1) / br;
         size_t const f = (size_t)rows * kp;
