@@ -31,11 +31,12 @@
 // of 64 values) that MMA2 reads K-major -- written by k_finish when the factor
 // is updated, or by k_split_bf16 when it is not current (start of a run, after
 // the test's EPS adjust of H).  The R warps work in two teams on alternate tiles.
-// R goes to shared memory (128B-swizzled, K-major), so both MMAs take A and B
-// from shared memory.
+// R replaces D in tensor memory, 16 columns of D becoming 8 of packed Rh and 8 of
+// Rl, and is MMA2's A operand there.
 //
-// Warp roles (768 threads): 0 = V producer, 1 = MMA issuer / TMEM owner,
-// 2 = X and Y producer, 3 = idle, 4..19 = R warps, 20..23 = accumulator warps.
+// Warp roles: 0 = V producer, 1 = MMA issuer / TMEM owner,
+// 2 = X and MMA1's Y producer, 3 = MMA2's Y producer, 4..19 (4..11 at
+// rank 64) = R warps, the last four (eight) = accumulator warps.
 // Persistent like the FP32 arm: every CTA takes an equal run of the list of all
 // row blocks' tiles (TileSplit), loading X anew where the run enters a row block.
 // Every wait is bounded (1 s); on expiry the kernel records an error word that
@@ -54,12 +55,7 @@ using namespace nmfb_tc;
 
 namespace {
 
-// kind::f16 instruction descriptor: BF16 A and B, both K-major, FP32 D.
-__host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-
+// D = or += A B, kind::f16, both operands from shared memory.
 template <bool ACC>
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc)
 {
@@ -90,24 +86,26 @@ struct GeoB {
     static constexpr int XBYTES = BO * KP * 2;
     static constexpr int YBYTES = BR * KP * 2;              // = KP rows of 128 B: one Y^T part
     static constexpr int YTROWS = (MODE == 2 ? 2 : 1) * KP; // Y^T hi (and lo) rows per tile
-    static constexpr int YSTAGE = 2 * YBYTES + YTROWS * 128;   // Yh | Yl | Y^T
-    static constexpr int RBYTES = BO * BR * 2;              // one R part
-    static constexpr int RSTAGE = (MODE == 2 ? 2 : 1) * RBYTES;  // Rh (| Rl)
+    // A ring each for MMA1's and MMA2's Y operands, as in the FP32 kernel.
+    static constexpr int Y1STAGE = (MODE >= 1 ? 2 : 1) * YBYTES;   // Yh (| Yl)
+    static constexpr int Y2STAGE = YTROWS * 128;            // Y^T
     static constexpr int VBYTES = BO * BR * 4;
-    static constexpr int YST = (KP == 64 && MODE == 2) ? 2 : 3;
-    static constexpr int NRB = 2;                           // R stages
-    static constexpr uint32_t NDB = 4;                      // D buffers in TMEM
+    static constexpr int Y1ST = 3, Y2ST = 2;
+    static constexpr uint32_t NDB = 4;                      // D buffers in TMEM; R takes D's place
     static constexpr int FIXED = 1024 + 512;
-    static constexpr int VAVAIL = (SMEM_LIMIT - FIXED - 2 * XBYTES - YST * YSTAGE - NRB * RSTAGE) / VBYTES;
+    static constexpr int XALL = (MODE >= 1 ? 2 : 1) * XBYTES, YALL = Y1ST * Y1STAGE + Y2ST * Y2STAGE;
+    static constexpr int VAVAIL = (SMEM_LIMIT - FIXED - XALL - YALL) / VBYTES;
     static constexpr int VST = VAVAIL > 6 ? 6 : VAVAIL;
-    static_assert(VST >= 2, "shared-memory ring too small");
-    static constexpr int SMEM = FIXED + 2 * XBYTES + YST * YSTAGE + NRB * RSTAGE + VST * VBYTES;
-    static constexpr int NR = 16;                           // R warps
-    static constexpr int NTHR = (4 + NR + 4) * 32;
+    static_assert(VST >= 3, "shared-memory ring too small");
+    static constexpr int SMEM = FIXED + XALL + YALL + VST * VBYTES;
+    static constexpr int NR = (KP == 64) ? 8 : 16;          // R warps
+    static constexpr int NA = (KP == 64) ? 2 : 1;           // accumulator warps: sets of four, KP / NA columns each
+    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;
     static constexpr uint32_t ACCW = (MODE == 2 ? 2 : 1) * KP;   // TMEM columns of one accumulator
     static constexpr uint32_t DB0 = 2 * ACCW;               // Acc[0..1] at 0 and ACCW; D[b] at DB0 + b*BR
     static_assert(DB0 + NDB * BR <= TMEM_COLS, "TMEM columns exceeded");
-    static_assert(YBYTES % 1024 == 0 && YSTAGE % 1024 == 0 && XBYTES % 1024 == 0, "1024-byte stage alignment");
+    static_assert(YBYTES % 1024 == 0 && Y1STAGE % 1024 == 0 && Y2STAGE % 1024 == 0 && XBYTES % 1024 == 0,
+                  "1024-byte stage alignment");
 };
 
 struct MapsB {
@@ -174,19 +172,20 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     extern __shared__ unsigned char smem_raw[];
     uint32_t const base_u32 = (smem_u32(smem_raw) + 1023u) & ~1023u;
     unsigned char *const base = smem_raw + (base_u32 - smem_u32(smem_raw));
-    unsigned char *const sX = base;                                  // Xh | Xl
-    unsigned char *const sY = sX + 2 * G::XBYTES;                    // [YST][Yh | Yl | Y^T]
-    unsigned char *const sR = sY + G::YST * G::YSTAGE;               // [NRB][Rh | Rl]
-    unsigned char *const sV = sR + G::NRB * G::RSTAGE;               // [VST][V]
+    unsigned char *const sX = base;                                  // Xh (| Xl)
+    unsigned char *const sY1 = sX + G::XALL;                         // [Y1ST][Yh (| Yl)]
+    unsigned char *const sY2 = sY1 + G::Y1ST * G::Y1STAGE;           // [Y2ST][Y^T]
+    unsigned char *const sV = sY2 + G::Y2ST * G::Y2STAGE;            // [VST][V]
     uint64_t *const bars = reinterpret_cast<uint64_t *>(sV + G::VST * G::VBYTES);
     uint64_t *const vfull = bars;                    // [VST]  TMA -> R warps
     uint64_t *const vempty = vfull + G::VST;         // [VST]  R warps -> V producer
-    uint64_t *const yfull = vempty + G::VST;         // [YST]  TMA -> MMA1 / MMA2
-    uint64_t *const yempty = yfull + G::YST;         // [YST]  MMA2 commit -> Y producer
-    uint64_t *const dfull = yempty + G::YST;         // [NDB]  MMA1 commit -> R warps
-    uint64_t *const rfull = dfull + G::NDB;          // [NRB]  R warps -> MMA2
-    uint64_t *const rempty = rfull + G::NRB;         // [NRB]  MMA2 commit -> R warps
-    uint64_t *const accrdy = rempty + G::NRB;        // [2]    MMA2 commit -> accumulator warps
+    uint64_t *const y1full = vempty + G::VST;        // [Y1ST] TMA -> MMA1
+    uint64_t *const y1empty = y1full + G::Y1ST;      // [Y1ST] MMA1 commit -> Y1 producer
+    uint64_t *const y2full = y1empty + G::Y1ST;      // [Y2ST] TMA -> MMA2
+    uint64_t *const y2empty = y2full + G::Y2ST;      // [Y2ST] MMA2 commit -> Y2 producer
+    uint64_t *const dfull = y2empty + G::Y2ST;       // [NDB]  MMA1 commit -> R warps
+    uint64_t *const rfull = dfull + G::NDB;          // [NDB]  R warps -> MMA2
+    uint64_t *const accrdy = rfull + G::NDB;         // [2]    MMA2 commit -> accumulator warps
     uint64_t *const accfree = accrdy + 2;            // [2]    accumulator warps -> MMA2
     uint64_t *const xfull = accfree + 2;             // [1]    TMA -> MMA1
     uint64_t *const xfree = xfull + 1;               // [1]    last MMA1 of a row block -> X producer
@@ -206,18 +205,21 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             mbar_init(&vfull[s], 1);
             mbar_init(&vempty[s], NR / 2);   // one team reads each V tile
         }
-        for (int s = 0; s < G::YST; s++) {
-            mbar_init(&yfull[s], 1);
-            mbar_init(&yempty[s], 1);
+        for (int s = 0; s < G::Y1ST; s++) {
+            mbar_init(&y1full[s], 1);
+            mbar_init(&y1empty[s], 1);
         }
-        for (uint32_t b = 0; b < G::NDB; b++) mbar_init(&dfull[b], 1);
-        for (int b = 0; b < G::NRB; b++) {
+        for (int s = 0; s < G::Y2ST; s++) {
+            mbar_init(&y2full[s], 1);
+            mbar_init(&y2empty[s], 1);
+        }
+        for (uint32_t b = 0; b < G::NDB; b++) {
+            mbar_init(&dfull[b], 1);
             mbar_init(&rfull[b], NR / 2);
-            mbar_init(&rempty[b], 1);
         }
         for (int b = 0; b < 2; b++) {
             mbar_init(&accrdy[b], 1);
-            mbar_init(&accfree[b], 4);
+            mbar_init(&accfree[b], 4 * G::NA);
         }
         mbar_init(xfull, 1);
         mbar_init(xfree, 1);
@@ -263,26 +265,25 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                 mbar_drain(&vfull[t % G::VST], (t / G::VST) & 1);
         }
     } else if (warp == 2) {
-        // ------------------------------------------------------------ X and Y producer
+        // ------------------------------------------------------------ X and MMA1's Y producer
         if (lane == 0) {
             uint64_t const pol = policy_evict_last();
             uint32_t issued = 0, xs = 0, c = c00;   // xs: row blocks whose X has been requested
             for (uint32_t t = 0; t < T; t++, c = (c + 1 == TB) ? 0 : c + 1) {
-                uint32_t const s = t % G::YST;
-                if (t >= (uint32_t)G::YST &&
-                    !mbar_wait(&yempty[s], ((t / G::YST) - 1) & 1, abort_flag, args.err, 22u, args.wait_ns))
+                uint32_t const s = t % G::Y1ST;
+                if (t >= (uint32_t)G::Y1ST &&
+                    !mbar_wait(&y1empty[s], ((t / G::Y1ST) - 1) & 1, abort_flag, args.err, 22u, args.wait_ns))
                     break;
                 issued = t + 1;
-                unsigned char *sy = sY + s * G::YSTAGE;
+                unsigned char *sy = sY1 + s * G::Y1STAGE;
                 int const r0 = (int)(c * BR);
-                mbar_expect_tx(&yfull[s], (SPLIT ? 2 : 1) * G::YBYTES + G::YTROWS * 128);
-                tma_load_2d(sy, &maps.yh, &yfull[s], 0, r0, pol);
-                if (SPLIT) tma_load_2d(sy + G::YBYTES, &maps.yl, &yfull[s], 0, r0, pol);
-                tma_load_2d(sy + 2 * G::YBYTES, &maps.yt, &yfull[s], 0, (int)(c * 2 * KP), pol);
+                mbar_expect_tx(&y1full[s], G::Y1STAGE);
+                tma_load_2d(sy, &maps.yh, &y1full[s], 0, r0, pol);
+                if (SPLIT) tma_load_2d(sy + G::YBYTES, &maps.yl, &y1full[s], 0, r0, pol);
                 if (t == 0 || c == 0) {   // X of the row block, once MMA1 has read the previous one's
                     if (xs > 0 && !mbar_wait(xfree, (xs - 1) & 1, abort_flag, args.err, 29u, args.wait_ns)) break;
                     int const o0 = (int)((ob0 + xs) * BO);
-                    mbar_expect_tx(xfull, (SPLIT ? 2 : 1) * G::XBYTES);
+                    mbar_expect_tx(xfull, G::XALL);
                     tma_load_2d(sX, &maps.xh, xfull, 0, o0, pol);
                     if (SPLIT) tma_load_2d(sX + G::XBYTES, &maps.xl, xfull, 0, o0, pol);
                     xs++;
@@ -290,61 +291,74 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             }
             // drain: the last X and the last load into every Y stage have landed
             if (xs > 0) mbar_drain(xfull, (xs - 1) & 1);
-            for (uint32_t t = issued > (uint32_t)G::YST ? issued - G::YST : 0; t < issued; t++)
-                mbar_drain(&yfull[t % G::YST], (t / G::YST) & 1);
+            for (uint32_t t = issued > (uint32_t)G::Y1ST ? issued - G::Y1ST : 0; t < issued; t++)
+                mbar_drain(&y1full[t % G::Y1ST], (t / G::Y1ST) & 1);
+        }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------ MMA2's Y producer
+        if (lane == 0) {
+            uint64_t const pol = policy_evict_last();
+            uint32_t issued = 0, c = c00;
+            for (uint32_t t = 0; t < T; t++, c = (c + 1 == TB) ? 0 : c + 1) {
+                uint32_t const s = t % G::Y2ST;
+                if (t >= (uint32_t)G::Y2ST &&
+                    !mbar_wait(&y2empty[s], ((t / G::Y2ST) - 1) & 1, abort_flag, args.err, 30u, args.wait_ns))
+                    break;
+                issued = t + 1;
+                mbar_expect_tx(&y2full[s], G::Y2STAGE);
+                tma_load_2d(sY2 + s * G::Y2STAGE, &maps.yt, &y2full[s], 0, (int)(c * 2 * KP), pol);
+            }
+            for (uint32_t t = issued > (uint32_t)G::Y2ST ? issued - G::Y2ST : 0; t < issued; t++)
+                mbar_drain(&y2full[t % G::Y2ST], (t / G::Y2ST) & 1);
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        //   MMA2(n2): needs R(n2) in shared memory and, for n2 >= 2, Acc[n2 % 2]
-        //             read by the accumulator warps (tile n2-2);
-        //   MMA1(n1): needs Y(n1), a free D buffer (n1 < n2 + NDB) and, for the
+        //   MMA2(n2): needs R(n2) in tensor memory, its Y operands and, for n2 >= 2,
+        //             Acc[n2 % 2] read by the accumulator warps (tile n2-2);
+        //   MMA1(n1): needs its Y operands, a free D buffer (n1 < n2 + NDB) and, for the
         //             first tile of a row block, its X; the last one's releases X.
-        // MMA2(t) is the last reader of Y stage t % YST and R stage t % NRB.
-        constexpr uint32_t IDESC1 = idesc_bf16(BO, BR);
-        constexpr uint32_t IDESC2 = idesc_bf16(BO, KP);
-        constexpr uint32_t IDESC2W = idesc_bf16(BO, 2 * KP);
-        uint32_t const sy_u32 = base_u32 + 2 * G::XBYTES, sr_u32 = sy_u32 + G::YST * G::YSTAGE;
+        constexpr uint32_t IDESC1 = idesc_bf16xf32(BO, BR);
+        constexpr uint32_t IDESC2 = idesc_bf16xf32(BO, KP);
+        constexpr uint32_t IDESC2W = idesc_bf16xf32(BO, 2 * KP);
+        uint32_t const y1_u32 = base_u32 + G::XALL, y2_u32 = y1_u32 + G::Y1ST * G::Y1STAGE;
         uint64_t const dX = smem_desc(base_u32, 16, 8 * G::ROWB, G::LAYOUT);   // Xh, then Xl
-        uint64_t const dY0 = smem_desc(sy_u32, 16, 8 * G::ROWB, G::LAYOUT);
-        uint64_t const dYT0 = smem_desc(sy_u32 + 2 * G::YBYTES, 16, 1024, 2u);
-        uint64_t const dR0 = smem_desc(sr_u32, 16, 1024, 2u);
+        uint64_t const dY0 = smem_desc(y1_u32, 16, 8 * G::ROWB, G::LAYOUT);
+        uint64_t const dYT0 = smem_desc(y2_u32, 16, 1024, 2u);
         uint32_t const tm = uniform(tmem);
         bool ok = true, x_ok = false;
         uint32_t n1 = 0, n2 = 0, c1 = c00, xs = 0;   // c1: reduction tile of n1; xs: its row block, from the CTA's first
         PollLimit limit(args.wait_ns);
         while (ok && n2 < T) {
             bool progressed = false;
-            if (n2 < n1 && mbar_test_warp(&rfull[n2 % G::NRB], (n2 / G::NRB) & 1) &&
+            if (n2 < n1 && mbar_test_warp(&rfull[n2 % G::NDB], (n2 / G::NDB) & 1) &&
+                mbar_test_warp(&y2full[n2 % G::Y2ST], (n2 / G::Y2ST) & 1) &&
                 (n2 < 2 || mbar_test_warp(&accfree[n2 & 1], ((n2 >> 1) - 1) & 1))) {
                 tc_fence_after();
-                uint32_t const ys = n2 % G::YST, rs = n2 % G::NRB, bp = n2 & 1;
-                uint32_t const oyt = ys * (G::YSTAGE >> 4), orr = rs * (G::RSTAGE >> 4);
+                uint32_t const ys = n2 % G::Y2ST, bp = n2 & 1;
+                uint32_t const oyt = ys * (G::Y2STAGE >> 4);
+                uint32_t const r = tm + G::DB0 + (n2 % G::NDB) * BR;   // k-step g: Rh at r + 16 g, Rl at r + 16 g + 8
                 uint32_t const dacc = tm + bp * G::ACCW;
                 if (elect_one()) {
                     // Acc[0:2KP] (+)= Rh [Y^T_hi; Y^T_lo];  Acc[0:KP] += Rl Y^T_hi  (MODE 2), or
                     // Acc (+)= Rh Y^T_hi
-                    mma_bf16<false>(dacc, desc_at(dR0, orr), desc_at(dYT0, oyt), SPLIT2 ? IDESC2W : IDESC2);
-                    if (SPLIT2) mma_bf16<true>(dacc, desc_at(dR0, orr + (G::RBYTES >> 4)), desc_at(dYT0, oyt), IDESC2);
+                    mma_ts_bf16<false>(dacc, r, desc_at(dYT0, oyt), SPLIT2 ? IDESC2W : IDESC2);
+                    if (SPLIT2) mma_ts_bf16<true>(dacc, r + 8, desc_at(dYT0, oyt), IDESC2);
 #pragma unroll
                     for (int ks = 1; ks < BR / 16; ks++) {
-                        mma_bf16<true>(dacc, desc_at(dR0, orr + ks * 2), desc_at(dYT0, oyt + ks * 2),
-                                       SPLIT2 ? IDESC2W : IDESC2);
-                        if (SPLIT2)
-                            mma_bf16<true>(dacc, desc_at(dR0, orr + (G::RBYTES >> 4) + ks * 2),
-                                           desc_at(dYT0, oyt + ks * 2), IDESC2);
+                        mma_ts_bf16<true>(dacc, r + ks * 16, desc_at(dYT0, oyt + ks * 2), SPLIT2 ? IDESC2W : IDESC2);
+                        if (SPLIT2) mma_ts_bf16<true>(dacc, r + ks * 16 + 8, desc_at(dYT0, oyt + ks * 2), IDESC2);
                     }
                     tc_commit(&accrdy[bp]);
-                    tc_commit(&yempty[ys]);
-                    tc_commit(&rempty[rs]);
+                    tc_commit(&y2empty[ys]);
                 }
                 n2++;
                 progressed = true;
             }
             if (n1 < T && !x_ok) x_ok = mbar_test_warp(xfull, xs & 1);
-            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&yfull[n1 % G::YST], (n1 / G::YST) & 1)) {
+            if (n1 < T && x_ok && n1 < n2 + G::NDB && mbar_test_warp(&y1full[n1 % G::Y1ST], (n1 / G::Y1ST) & 1)) {
                 tc_fence_after();
-                uint32_t const s = n1 % G::YST, db = n1 % G::NDB;
-                uint32_t const oy = s * (G::YSTAGE >> 4);
+                uint32_t const s = n1 % G::Y1ST, db = n1 % G::NDB;
+                uint32_t const oy = s * (G::Y1STAGE >> 4);
                 uint32_t const dcol = tm + G::DB0 + db * BR;
                 bool const last = c1 + 1 == TB;   // the row block's last tile
                 if (elect_one()) {
@@ -363,6 +377,7 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                             mma_bf16<true>(dcol, desc_at(dX, xo + ks * 2), desc_at(dY0, yo + ks * 2), IDESC1);
                     }
                     tc_commit(&dfull[db]);
+                    tc_commit(&y1empty[s]);
                     if (last) tc_commit(xfree);
                 }
                 n1++;
@@ -402,13 +417,10 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         uint32_t const row = quad * 32 + lane;          // TMEM lane = output row within the block
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
         for (uint32_t t = team; t < T; t += 2) {
-            uint32_t const s = t % G::VST, b = t % G::NDB, rs = t % G::NRB;
+            uint32_t const s = t % G::VST, b = t % G::NDB;
             uint32_t const c = (c00 + t) % TB;              // reduction tile
             if (!mbar_wait_warp(&dfull[b], (t / G::NDB) & 1, abort_flag, args.err, 25u, args.wait_ns)) break;
             if (!mbar_wait_warp(&vfull[s], (t / G::VST) & 1, abort_flag, args.err, 26u, args.wait_ns)) break;
-            if (t >= (uint32_t)G::NRB &&
-                !mbar_wait_warp(&rempty[rs], ((t / G::NRB) - 1) & 1, abort_flag, args.err, 27u, args.wait_ns))
-                break;
             tc_fence_after();
             const unsigned char *sv = sV + s * G::VBYTES;
             bool const edge = (c + 1) * BR > args.R;        // the partial last reduction tile
@@ -461,23 +473,16 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                         pl[c / 2] = pack_bf16x2(r0 - h0, r1 - h1);
                     }
                 }
-                // R row `row`, columns col0 .. +16: 16-byte chunks of a 128-byte K-major row, 128B swizzle.
-                unsigned char *rrow = sR + rs * G::RSTAGE + row * 128;
-#pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    uint32_t const off = ((col0 / 8 + q) ^ (row & 7)) << 4;
-                    *reinterpret_cast<uint4 *>(rrow + off) = make_uint4(pk[4 * q + 0], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-                    if (SPLIT2)
-                        *reinterpret_cast<uint4 *>(rrow + G::RBYTES + off) =
-                            make_uint4(pl[4 * q + 0], pl[4 * q + 1], pl[4 * q + 2], pl[4 * q + 3]);
-                }
+                // R over the 16 columns of D it came from: Rh packed in the first 8, Rl in the others.
+                tmem_st8(lane_addr + G::DB0 + b * BR + col0, pk);
+                if (SPLIT2) tmem_st8(lane_addr + G::DB0 + b * BR + col0 + 8, pl);
             }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&vempty[s]);   // the values of V have been used (see the FP32 kernel)
-                mbar_arrive(&rfull[rs]);
+                mbar_arrive(&rfull[b]);
             }
         }
     } else if (warp >= 4 + NR) {
@@ -485,9 +490,11 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
         uint32_t const quad = warp & 3;
         uint32_t const row = quad * 32 + lane;
         uint32_t const lane_addr = tmem + ((quad * 32) << 16);
-        float sum[KP];
+        constexpr int KC = KP / G::NA;
+        uint32_t const k0 = ((warp - 4 - NR) >> 2) * KC;   // first column
+        float sum[KC];
 #pragma unroll
-        for (int c = 0; c < KP; c++) sum[c] = 0.0f;
+        for (int c = 0; c < KC; c++) sum[c] = 0.0f;
         uint32_t ob = ob0, c1 = c00;   // row block and reduction tile of t
         bool gap_done = c00 == 0 || c00 % args.ts.run != 0;
         for (uint32_t t = 0; t < T; t++) {
@@ -495,10 +502,10 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             if (!mbar_wait_warp(&accrdy[bp], (t >> 1) & 1, abort_flag, args.err, 28u, args.wait_ns)) break;
             tc_fence_after();
 #pragma unroll
-            for (int c0 = 0; c0 < KP; c0 += 16) {
+            for (int c0 = 0; c0 < KC; c0 += 16) {
                 uint32_t a[32], a2[32];
-                tmem_ld16(lane_addr + bp * G::ACCW + c0, a);
-                if (SPLIT2) tmem_ld16(lane_addr + bp * G::ACCW + KP + c0, a2);
+                tmem_ld16(lane_addr + bp * G::ACCW + k0 + c0, a);
+                if (SPLIT2) tmem_ld16(lane_addr + bp * G::ACCW + KP + k0 + c0, a2);
                 tmem_wait_ld_dep16(a);
                 if (SPLIT2) tmem_wait_ld_dep16(a2);
 #pragma unroll
@@ -512,19 +519,19 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             if (done || t + 1 == T || (c1 + 1) % args.ts.run == 0) {   // a partial of the row block
                 uint32_t const o = ob * BO + row;
                 if (o < args.O) {
-                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP;
+                    float *dst = args.part + ((size_t)args.ts.slot(ob, blockIdx.x, c1) * args.O + o) * KP + k0;
 #pragma unroll
-                    for (int c = 0; c < KP; c += 4)
+                    for (int c = 0; c < KC; c += 4)
                         *reinterpret_cast<float4 *>(dst + c) = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
                     if (!gap_done) {   // the unused slot (TileSplit::slot)
-                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP;
+                        dst = args.part + ((size_t)(args.ts.slot(ob0, blockIdx.x, c00) - 1) * args.O + o) * KP + k0;
 #pragma unroll
-                        for (int c = 0; c < KP; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                        for (int c = 0; c < KC; c += 4) *reinterpret_cast<float4 *>(dst + c) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
                 }
                 gap_done = true;
 #pragma unroll
-                for (int c = 0; c < KP; c++) sum[c] = 0.0f;
+                for (int c = 0; c < KC; c++) sum[c] = 0.0f;
             }
             c1 = done ? 0 : c1 + 1;
             ob += done;

@@ -65,38 +65,12 @@ using namespace nmfb_tc;
 
 namespace {
 
-// kind::f16 instruction descriptor with BF16 A and B (K-major) and FP32 D.
-__host__ __device__ constexpr uint32_t idesc_bf16xf32(uint32_t M, uint32_t N)
-{
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
-}
-
-// D = or += A B, kind::f16, with A from tensor memory (two BF16 per 32-bit column, the
-// lower K index in the low half) and B from shared memory.
-template <bool ACC>
-__device__ __forceinline__ void mma_ts_bf16(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "r"(a_tmem), "l"(bdesc), "r"(idesc), "n"(ACC ? 1 : 0)
-        : "memory");
-}
-
 // Two floats to a BF16 pair (round to nearest even), `first` in the low half.
 __device__ __forceinline__ uint32_t bf16x2_rn(float first, float second)
 {
     uint32_t r;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(second), "f"(first));
     return r;
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *r)
-{
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-                 "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
 }
 
 // Swizzle of a K-major operand whose rows are `bytes` long: the UMMA layout code
