@@ -16,7 +16,6 @@ using nmfb::ConvState;
 using nmfb_tc::BO;
 using nmfb_tc::tf32_rna;
 
-constexpr uint32_t FIN_ECH = 32;   // row blocks per chunk of k_finish's column sums
 constexpr uint32_t FIN_RB = 32;    // rows of X per k_finish CTA
 
 // k_finish's launch shape for a factor of `rows` rows: KP / 4 threads per row
@@ -48,15 +47,18 @@ __device__ __forceinline__ uint32_t fin_bf16x2(float first, float second)
 //   (matrix_mul_div, src/GPU_kernels.cu:1885-2058: product first, then the
 //   division, correctly rounded) with the EPS adjust when asked (kernel_adjust,
 //   :2338-2345); then X's split copies in the arm's layout (LAYOUT 0:
-//   k_split_factor's, LAYOUT 1: k_split_bf16's) and its column
-//   sums (matrix_to_row, src/GPU_kernels.cu:871-1066) in FP64: a shuffle tree over
-//   each warp's rows, the warps in order, row blocks in chunks of FIN_ECH in block
-//   order, the chunks in order -- fixed orders throughout, so the result does not
-//   depend on scheduling.  It replaces the reference's mul_div + adjust and, for the
-//   next half-iteration, its column sums, in one launch.  Small blocks and the
-//   partials of up to eight splits in flight per thread keep each CTA's chain of
-//   dependent memory round trips short: the kernel is latency-bound, its traffic
-//   (the partials, X and its copies) small.
+//   the FP32 arm's SplitLayout, LAYOUT 1: BF16 hi, lo and transposed blocks) and a
+//   partial of its column sums (matrix_to_row, src/GPU_kernels.cu:871-1066) in FP64,
+//   one per CTA: a shuffle tree over each warp's rows, the warps in order; the next
+//   main kernel adds the partials (column_sums).  Fixed orders throughout, so the
+//   result does not depend on scheduling.  With nothing to update (a.part null) it
+//   writes the copies and partials of X as it is: the factor read first in a run.
+//   It replaces the reference's mul_div + adjust and, for the next half-iteration,
+//   its column sums, in one launch.  Small blocks and the partials of up to eight
+//   slots in flight per thread keep each CTA's chain of dependent memory round trips
+//   short: the kernel is latency-bound, its traffic (the partials, X and its copies)
+//   small.  (Adding the column sums here, by retirement counters over chunks of CTAs,
+//   made the chain twice as long: 8.5 us a launch at 5000 x 16.)
 struct FinishArgs {
     uint32_t O, k;
     nmfb_tc::TileSplit ts;
@@ -69,10 +71,7 @@ struct FinishArgs {
     uint32_t xnblk32, xnblkbr;
     __nv_bfloat16 *bhi, *blo, *bT;   // LAYOUT 1: bf16 hi, lo (rows x KP) and per 64 rows [hi^T ; lo^T]
     uint32_t bnblk64;
-    double *cs;           // [row block][KP] FP64 column-sum partials, then from row csoff [chunk][KP]
-    uint32_t csoff;
-    float *accX;          // column sums of the new X (KP)
-    uint32_t *tick;       // [chunks + 1] retirement counters (left at 0)
+    double *cs;           // [CTA][KP] FP64 column-sum partials
     const ConvState *st;
 };
 
@@ -84,13 +83,14 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
     constexpr int NW = NT / 32;                  // warps
     constexpr int QB = 8 / RPT;                  // splits per row in flight (8 loads per thread)
     static_assert(32 % TPR == 0 && NT % KP == 0 && QB >= 1, "k_finish shape");
+    nmfb_tc::chain_next();
+    nmfb_tc::chain_wait();
     if (a.st && *(volatile const uint32_t *)&a.st->converged) return;
-    __shared__ double ws[NW * KP + NT];
+    __shared__ double ws[NW * KP];
     __shared__ float sx[KP * 33];                // x of one 32-row set, column-major (padded)
-    __shared__ uint32_t eflag;
     uint32_t const tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     uint32_t const row = tid / TPR, c0 = (tid % TPR) * 4;
-    uint32_t const blk = blockIdx.x, nob = gridDim.x;
+    uint32_t const blk = blockIdx.x;
     size_t const qs = (size_t)a.O * KP;
     // this thread's rows: one in each 32-row set of the CTA's block
     uint32_t o[RPT];
@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
     // row sets of a CTA lie in one row block: BO is a multiple of FIN_RB RPT)
     static_assert(BO % ((int)FIN_RB * RPT) == 0, "row sets of a CTA in one row block");
     uint32_t const ob = blk * (FIN_RB * RPT) / BO;
-    uint32_t const nslot = a.ts.nslot(ob);
+    bool const update = a.part != nullptr;
+    uint32_t const nslot = update ? a.ts.nslot(ob) : 0;
     for (uint32_t q = 0; q < nslot; q += QB) {
         float4 v[RPT][QB];
 #pragma unroll
@@ -141,12 +142,13 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
                 uint32_t const cc = c0 + i;
                 float v = 0.0f;
                 if (cc < a.k) {
-                    v = __fdiv_rn(xs[i] * x[r][i], __ldg(a.accY + cc));
+                    v = update ? __fdiv_rn(xs[i] * x[r][i], __ldcg(a.accY + cc)) : xs[i];
                     if (a.adjust) v = fmaxf(v, FLT_MIN);
                 }
                 x[r][i] = v;
             }
-            *reinterpret_cast<float4 *>(a.X + (size_t)o[r] * KP + c0) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
+            if (update)
+                *reinterpret_cast<float4 *>(a.X + (size_t)o[r] * KP + c0) = make_float4(x[r][0], x[r][1], x[r][2], x[r][3]);
         }
 #pragma unroll
         for (int i = 0; i < 4; i++) csum[i] += (double)x[r][i];
@@ -173,7 +175,7 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
                 }
             }
         } else if (in[r]) {
-            // hi = bf16(x), lo = bf16(x - hi), both rounded to nearest (k_split_bf16)
+            // hi = bf16(x), lo = bf16(x - hi), both rounded to nearest
             size_t const e = (size_t)o[r] * KP + c0;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
@@ -231,59 +233,16 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
         for (int w = 0; w < NW; w++) t += ws[w * KP + tid];
         a.cs[(size_t)blk * KP + tid] = t;
     }
-    __threadfence();
-    __syncthreads();
-    uint32_t const nch = (nob + FIN_ECH - 1) / FIN_ECH, ch = blk / FIN_ECH;
-    uint32_t const b0 = ch * FIN_ECH, bn = min(nob - b0, FIN_ECH);
-    if (tid == 0) eflag = (atomicAdd(&a.tick[ch], 1u) == bn - 1) ? 1u : 0u;
-    __syncthreads();
-    if (!eflag) return;
-    // last row block of its chunk: the chunk's partials in block order
-    __threadfence();
-    constexpr int GRP = NT / KP;
-    uint32_t const g = tid / KP, c = tid % KP;
-    double t = 0.0;
-    for (uint32_t b = g; b < bn; b += GRP) t += __ldcg(a.cs + (size_t)(b0 + b) * KP + c);
-    ws[NW * KP + tid] = t;
-    __syncthreads();
-    if (tid < (uint32_t)KP) {
-        double u = 0.0;
-        for (int gg = 0; gg < GRP; gg++) u += ws[NW * KP + gg * KP + tid];
-        a.cs[((size_t)a.csoff + ch) * KP + tid] = u;
-    }
-    if (tid == 0) a.tick[ch] = 0u;
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) eflag = (atomicAdd(&a.tick[nch], 1u) == nch - 1) ? 1u : 0u;
-    __syncthreads();
-    if (!eflag) return;
-    // last chunk: the chunk sums in order
-    __threadfence();
-    double v = 0.0;
-    for (uint32_t q = g; q < nch; q += GRP) v += __ldcg(a.cs + ((size_t)a.csoff + q) * KP + c);
-    __syncthreads();
-    ws[NW * KP + tid] = v;
-    __syncthreads();
-    if (tid < (uint32_t)KP) {
-        double u = 0.0;
-        for (int gg = 0; gg < GRP; gg++) u += ws[NW * KP + gg * KP + tid];
-        a.accX[tid] = (float)u;
-    }
-    if (tid == 0) a.tick[nch] = 0u;
 }
 
 // k_finish for the factor of a.O rows, with the row sets per thread that its
 // partial count calls for (the block count is fin_blocks(a.O, fin_rpt(a.ts.slots))).
 template <int KP, int BR, int LAYOUT>
-void fin_launch(const FinishArgs &a, cudaStream_t s)
+cudaError_t fin_launch(const FinishArgs &a, cudaStream_t s)
 {
     uint32_t const rpt = fin_rpt(a.ts.slots), nb = fin_blocks(a.O, rpt);
-    if (rpt == 4)
-        k_finish<KP, BR, LAYOUT, 4><<<nb, fin_threads<KP>(), 0, s>>>(a);
-    else if (rpt == 2)
-        k_finish<KP, BR, LAYOUT, 2><<<nb, fin_threads<KP>(), 0, s>>>(a);
-    else
-        k_finish<KP, BR, LAYOUT, 1><<<nb, fin_threads<KP>(), 0, s>>>(a);
+    auto const kern = rpt == 4 ? k_finish<KP, BR, LAYOUT, 4> : rpt == 2 ? k_finish<KP, BR, LAYOUT, 2> : k_finish<KP, BR, LAYOUT, 1>;
+    return nmfb_tc::launch_chained(kern, nb, fin_threads<KP>(), 0, s, a);
 }
 
 }  // namespace

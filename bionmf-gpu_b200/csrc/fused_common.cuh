@@ -65,6 +65,63 @@ inline TileSplit plan_tiles(uint32_t O, uint32_t R, uint32_t br, uint32_t sms, s
     return s;
 }
 
+// Programmatic dependent launch: a kernel launched by launch_chained starts as
+// soon as every CTA of the kernel before it has called chain_next (or left),
+// and runs up to its own chain_wait, which returns when that kernel -- and so,
+// each kernel of the chain waiting for the one before, all earlier work -- has
+// completed and its writes are visible.  Every thread that reads or writes
+// global memory calls chain_wait first, and what the kernel just before wrote is
+// read through L2.  It hides a launch and the prologue
+// (barriers, tensor-memory allocation), about 2 us of each of an iteration's
+// four launches.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kern)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream, A &&...args)
+{
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
+// Column sums of a factor.  k_finish leaves one FP64 partial per CTA and column
+// (cs[block][KP]); the next half-iteration's main kernel, which runs long before
+// anything divides by the sums, adds them with its V producer's warp: CTA b takes
+// columns b, b + gridDim.x, ... once its V loads are issued; lane l adds blocks l, l + 32, ... in order, then
+// a shuffle tree.
+struct ColSum {
+    const double *cs;
+    uint32_t nblk;
+    float *acc;   // [KP]
+};
+template <int KP>
+__device__ __forceinline__ void column_sums(const ColSum &a)
+{
+    uint32_t const lane = threadIdx.x % 32;
+    for (uint32_t c = blockIdx.x; c < (uint32_t)KP; c += gridDim.x) {
+        double t = 0.0;
+        for (uint32_t b = lane; b < a.nblk; b += 32 * 8) {   // eight loads in flight
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = b + 32 * i < a.nblk ? __ldcg(a.cs + (size_t)(b + 32 * i) * KP + c) : 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) t += v[i];
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) t += __shfl_xor_sync(0xffffffffu, t, off);
+        if (lane == 0) a.acc[c] = (float)t;
+    }
+}
+
 // PTX helpers
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

@@ -29,8 +29,8 @@
 // hi / lo copies of X and Y (rows x KP, K-major) and, per 64-row block, the
 // transposed hi block followed by the transposed lo block (64 rows -> 2 KP rows
 // of 64 values) that MMA2 reads K-major -- written by k_finish when the factor
-// is updated, or by k_split_bf16 when it is not current (start of a run, after
-// the test's EPS adjust of H).  The R warps work in two teams on alternate tiles.
+// is updated, or on its own when it is not current (start of a run, after the
+// test's EPS adjust of H).  The R warps work in two teams on alternate tiles.
 // R replaces D in tensor memory, 16 columns of D becoming 8 of packed Rh and 8 of
 // Rl, and is MMA2's A operand there.
 //
@@ -100,7 +100,7 @@ struct GeoB {
     static constexpr int SMEM = FIXED + XALL + YALL + VST * VBYTES;
     static constexpr int NR = (KP == 64) ? 8 : 16;          // R warps
     static constexpr int NA = (KP == 64) ? 2 : 1;           // accumulator warps: sets of four, KP / NA columns each
-    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;
+    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;   // (a multiple of four warps: one more would cost 8 registers a thread)
     static constexpr uint32_t ACCW = (MODE == 2 ? 2 : 1) * KP;   // TMEM columns of one accumulator
     static constexpr uint32_t DB0 = 2 * ACCW;               // Acc[0..1] at 0 and ACCW; D[b] at DB0 + b*BR
     static_assert(DB0 + NDB * BR <= TMEM_COLS, "TMEM columns exceeded");
@@ -118,44 +118,12 @@ struct MapsB {
 struct ArgsB {
     uint32_t O, R;
     TileSplit ts;
+    ColSum csy;           // column sums of the other factor
     float *part;                 // [slot][O][KP]
     uint32_t *err;
     const ConvState *st;
     unsigned long long wait_ns;  // limit of every bounded wait (%globaltimer ns)
 };
-
-// BF16 hi / lo copies of a factor (rows x kp FP32, padding columns zero) and,
-// when T is given, per 64-row block the transposed hi block (kp rows of 64)
-// followed by the transposed lo block, rows past the end zero.  One CTA per
-// 64-row block.
-__global__ void __launch_bounds__(256) k_split_bf16(const float *__restrict__ Y, uint32_t rows, uint32_t kp,
-                                                    __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                                    __nv_bfloat16 *__restrict__ T, const ConvState *st)
-{
-    if (st && *(volatile const uint32_t *)&st->converged) return;
-    __shared__ __nv_bfloat16 th[64][66], tl[64][66];
-    uint32_t const r0 = blockIdx.x * 64;
-    for (uint32_t e = threadIdx.x; e < 64 * kp; e += blockDim.x) {
-        uint32_t const r = e / kp, c = e % kp;
-        bool const in = r0 + r < rows;
-        float const y = in ? Y[(size_t)(r0 + r) * kp + c] : 0.0f;
-        __nv_bfloat16 const h = __float2bfloat16_rn(y);
-        __nv_bfloat16 const l = __float2bfloat16_rn(y - __bfloat162float(h));
-        if (in) {
-            hi[(size_t)(r0 + r) * kp + c] = h;
-            lo[(size_t)(r0 + r) * kp + c] = l;
-        }
-        th[r][c] = h;
-        tl[r][c] = l;
-    }
-    if (!T) return;
-    __syncthreads();
-    __nv_bfloat16 *dst = T + (size_t)blockIdx.x * 2 * kp * 64;
-    for (uint32_t e = threadIdx.x; e < 2 * kp * 64; e += blockDim.x) {
-        uint32_t const row = e / 64, rr = e % 64;
-        dst[e] = row < kp ? th[rr][row] : tl[rr][row - kp];
-    }
-}
 
 template <bool HSIDE, int KP, int MODE>
 __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
@@ -167,7 +135,6 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     constexpr bool SPLIT = MODE >= 1;                // MMA1 split
     constexpr bool SPLIT2 = MODE == 2;               // MMA2 split
     constexpr int NTERMS = SPLIT ? 3 : 1;
-    if (args.st && *(volatile const uint32_t *)&args.st->converged) return;
 
     extern __shared__ unsigned char smem_raw[];
     uint32_t const base_u32 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -193,11 +160,12 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(mdrain + 1);
     volatile uint32_t *const abort_flag = tmem_slot + 1;
 
+    chain_next();
     uint32_t const warp = uniform(threadIdx.x / 32), lane = threadIdx.x % 32;
     // This CTA's run of tiles [g0, g0 + T) of the (row block, reduction tile) list.
     uint32_t const TB = args.ts.tb;
     uint32_t const g0 = blockIdx.x * args.ts.tpc;
-    uint32_t const T = min(args.ts.total - g0, args.ts.tpc);
+    uint32_t T = min(args.ts.total - g0, args.ts.tpc);
     uint32_t const ob0 = g0 / TB, c00 = g0 - ob0 * TB;
 
     if (threadIdx.x == 0) {
@@ -237,12 +205,15 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
     __syncthreads();
     tc_fence_after();
     uint32_t const tmem = *tmem_slot;
+    chain_wait();   // nothing above reads or writes global memory
+    if (args.st && *(volatile const uint32_t *)&args.st->converged) T = 0;   // every role's loop is empty
 
     if (warp == 0) {
-        // ------------------------------------------------------------ V producer
+        // ------------------------------------------------------------ V producer, then the column sums of Y
+        uint32_t issued = 0;
         if (lane == 0) {
             uint64_t const pol = policy_evict_first();
-            uint32_t issued = 0, ob = ob0, c = c00;
+            uint32_t ob = ob0, c = c00;
             for (uint32_t t = 0; t < T; t++, ob += (c + 1 == TB), c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::VST;
                 if (t >= (uint32_t)G::VST &&
@@ -260,10 +231,13 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                         tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, o0, pol);
                 }
             }
+        }
+        __syncwarp();
+        if (T > 0) column_sums<KP>(args.csy);   // (while the last tiles are worked on; k_finish divides by them)
+        if (lane == 0)
             // drain: the last load into every stage has landed
             for (uint32_t t = issued > (uint32_t)G::VST ? issued - G::VST : 0; t < issued; t++)
                 mbar_drain(&vfull[t % G::VST], (t / G::VST) & 1);
-        }
     } else if (warp == 2) {
         // ------------------------------------------------------------ X and MMA1's Y producer
         if (lane == 0) {
@@ -580,9 +554,7 @@ struct PlanB {
     __nv_bfloat16 *wsplit, *hsplit;   // hi | lo | transposed hi/lo blocks, for W and for H
     uint32_t *dErr;                   // shared with the FP32 arm's error word
     int arm;                          // arm the Y^T maps were encoded for
-    double *dCs;                      // k_finish's column-sum partials (row blocks, then chunks)
-    uint32_t *dTick;                  // k_finish's retirement counters
-    uint32_t nticks, csoff;
+    double *dCsW, *dCsH;              // k_finish's column-sum partials of W and of H
 };
 
 template <int KP, int MODE>
@@ -603,60 +575,58 @@ int set_attrs_b(nmfb_ctx *ctx)
     return rc;
 }
 
+// How the half-iteration that updates W (or H) is dealt out.
+TileSplit plan_of_b(const nmfb_ctx *ctx, bool w)
+{
+    return plan_tiles(w ? ctx->n : ctx->m, w ? ctx->m : ctx->n, 64, (uint32_t)ctx->sm_count, ctx->part_items / ctx->kp);
+}
+
 template <bool HSIDE, int KP, int MODE>
-int launch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
+int launch_b(nmfb_ctx *ctx, const MapsB &maps, PlanB *plan)
 {
     using G = GeoB<KP, MODE>;
-    constexpr int BR = G::BR;
-    uint32_t const O = HSIDE ? ctx->m : ctx->n;
-    uint32_t const R = HSIDE ? ctx->n : ctx->m;
-    ts = plan_tiles(O, R, BR, (uint32_t)ctx->sm_count, ctx->part_items / KP);
-    if ((size_t)ts.slots * O * KP > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arm: partial buffer too small (%u slots)", ts.slots);
+    static_assert(G::BR == 64, "plan_of_b");
     ArgsB args;
-    args.O = O;
-    args.R = R;
-    args.ts = ts;
+    args.O = HSIDE ? ctx->m : ctx->n;
+    args.R = HSIDE ? ctx->n : ctx->m;
+    args.ts = plan_of_b(ctx, !HSIDE);
+    if ((size_t)args.ts.slots * args.O * KP > ctx->part_items)
+        return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arm: partial buffer too small (%u slots)", args.ts.slots);
+    args.csy.cs = HSIDE ? plan->dCsW : plan->dCsH;
+    args.csy.nblk = fin_blocks(args.R, fin_rpt(plan_of_b(ctx, HSIDE).slots));
+    args.csy.acc = HSIDE ? ctx->dAccW : ctx->dAccH;
     args.part = ctx->dPart;
-    args.err = err;
+    args.err = plan->dErr;
     args.st = ctx->dState;
     args.wait_ns = ctx->wait_ns ? ctx->wait_ns : WAIT_LIMIT_NS;
     int const main = HSIDE ? 0 : 1;
     int rc = nmfb_prof_begin(ctx, main);
     if (rc) return rc;
-    k_fused_bf16<HSIDE, KP, MODE><<<ts.ctas(), G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
+    NMFB_CUDA_TRY(ctx, launch_chained(k_fused_bf16<HSIDE, KP, MODE>, args.ts.ctas(), G::NTHR, G::SMEM, ctx->stream, maps,
+                                      args));
     NMFB_LAUNCH_CHECK(ctx);
     return nmfb_prof_end(ctx, main);
 }
 
 template <bool HSIDE, int KP>
-int dispatch_kp(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
+int dispatch_kp(nmfb_ctx *ctx, const MapsB &maps, PlanB *plan)
 {
     switch (ctx->arm) {
-    case NMFB_ARM_BF16: return launch_b<HSIDE, KP, 0>(ctx, maps, err, ts);
-    case NMFB_ARM_SPLIT_BF16: return launch_b<HSIDE, KP, 1>(ctx, maps, err, ts);
-    default: return launch_b<HSIDE, KP, 2>(ctx, maps, err, ts);
+    case NMFB_ARM_BF16: return launch_b<HSIDE, KP, 0>(ctx, maps, plan);
+    case NMFB_ARM_SPLIT_BF16: return launch_b<HSIDE, KP, 1>(ctx, maps, plan);
+    default: return launch_b<HSIDE, KP, 2>(ctx, maps, plan);
     }
 }
 
 template <bool HSIDE>
-int dispatch_b(nmfb_ctx *ctx, const MapsB &maps, uint32_t *err, TileSplit &ts)
+int dispatch_b(nmfb_ctx *ctx, const MapsB &maps, PlanB *plan)
 {
     switch (ctx->kp) {
-    case 16: return dispatch_kp<HSIDE, 16>(ctx, maps, err, ts);
-    case 32: return dispatch_kp<HSIDE, 32>(ctx, maps, err, ts);
-    case 64: return dispatch_kp<HSIDE, 64>(ctx, maps, err, ts);
+    case 16: return dispatch_kp<HSIDE, 16>(ctx, maps, plan);
+    case 32: return dispatch_kp<HSIDE, 32>(ctx, maps, plan);
+    case 64: return dispatch_kp<HSIDE, 64>(ctx, maps, plan);
     default: return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arms: unsupported padded rank %u", ctx->kp);
     }
-}
-
-int split_factor(nmfb_ctx *ctx, const float *F, uint32_t rows, __nv_bfloat16 *dst, bool with_t)
-{
-    size_t const part = (size_t)rows * ctx->kp;
-    k_split_bf16<<<(rows + 63) / 64, 256, 0, ctx->stream>>>(F, rows, ctx->kp, dst, dst + part,
-                                                            with_t ? dst + 2 * part : nullptr, ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    return NMFB_OK;
 }
 
 int encode_maps_b(nmfb_ctx *ctx, PlanB *plan)
@@ -694,49 +664,41 @@ int encode_maps_b(nmfb_ctx *ctx, PlanB *plan)
     return NMFB_OK;
 }
 
-// A factor's BF16 copies (hi, lo, transposed blocks) and column sums, when the
-// previous half-iteration's k_finish did not produce them.
-int prepare_b(nmfb_ctx *ctx, bool w)
-{
-    PlanB *plan = (PlanB *)ctx->bplan;
-    const float *F = w ? ctx->dW : ctx->dH;
-    uint32_t const rows = w ? ctx->n : ctx->m;
-    int rc = nmfb_colsum(ctx, F, rows, w ? ctx->dAccW : ctx->dAccH, w ? 0 : 1);
-    if (!rc) rc = split_factor(ctx, F, rows, w ? plan->wsplit : plan->hsplit, true);
-    if (!rc) ctx->fz_ok[w ? 0 : 1] = 1;
-    return rc;
-}
-
+// k_finish on W (or H): its update from the partials, or, with update = false,
+// only its BF16 copies and column-sum partials.
 template <int KP>
-int launch_finish_b(nmfb_ctx *ctx, bool is_H, const TileSplit &ts, int adjust)
+int launch_finish_b(nmfb_ctx *ctx, bool w, bool update, int adjust)
 {
     PlanB *plan = (PlanB *)ctx->bplan;
-    uint32_t const O = is_H ? ctx->m : ctx->n;
-    uint32_t const fblocks = fin_blocks(O, fin_rpt(ts.slots));
-    if (fblocks > plan->csoff || (fblocks + FIN_ECH - 1) / FIN_ECH + 1 > plan->nticks)
-        return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arms: column-sum buffers too small");
-    __nv_bfloat16 *xs = is_H ? plan->hsplit : plan->wsplit;
-    size_t const sz = (size_t)O * KP;
     FinishArgs fa = {};
-    fa.O = O;
-    fa.ts = ts;
+    fa.O = w ? ctx->n : ctx->m;
+    __nv_bfloat16 *xs = w ? plan->wsplit : plan->hsplit;
+    size_t const sz = (size_t)fa.O * KP;
+    fa.ts = plan_of_b(ctx, w);
     fa.k = ctx->k;
     fa.adjust = adjust;
-    fa.part = ctx->dPart;
-    fa.X = is_H ? ctx->dH : ctx->dW;
-    fa.accY = is_H ? ctx->dAccW : ctx->dAccH;
+    fa.part = update ? ctx->dPart : nullptr;
+    fa.X = w ? ctx->dW : ctx->dH;
+    fa.accY = w ? ctx->dAccH : ctx->dAccW;
     fa.bhi = xs;
     fa.blo = xs + sz;
     fa.bT = xs + 2 * sz;
-    fa.bnblk64 = (O + 63) / 64;
-    fa.cs = plan->dCs;
-    fa.csoff = plan->csoff;
-    fa.accX = is_H ? ctx->dAccH : ctx->dAccW;
-    fa.tick = plan->dTick;
+    fa.bnblk64 = (fa.O + 63) / 64;
+    fa.cs = w ? plan->dCsW : plan->dCsH;
     fa.st = ctx->dState;
-    fin_launch<KP, 64, 1>(fa, ctx->stream);
+    NMFB_CUDA_TRY(ctx, (fin_launch<KP, 64, 1>(fa, ctx->stream)));
     NMFB_LAUNCH_CHECK(ctx);
+    ctx->fz_ok[w ? 0 : 1] = 1;
     return NMFB_OK;
+}
+
+int finish_b(nmfb_ctx *ctx, bool w, bool update, int adjust)
+{
+    switch (ctx->kp) {
+    case 16: return launch_finish_b<16>(ctx, w, update, adjust);
+    case 32: return launch_finish_b<32>(ctx, w, update, adjust);
+    default: return launch_finish_b<64>(ctx, w, update, adjust);
+    }
 }
 
 // One half-iteration: the fused BF16 kernel and k_finish (which writes X's BF16
@@ -750,18 +712,11 @@ int bf16_half(nmfb_ctx *ctx, bool is_H, int adjust)
     if (plan->arm != ctx->arm && (rc = encode_maps_b(ctx, plan))) return rc;
     int const whole = is_H ? 2 : 3;
     if ((rc = nmfb_prof_begin(ctx, whole))) return rc;
-    if (!ctx->fz_ok[is_H ? 0 : 1] && (rc = prepare_b(ctx, is_H))) return rc;    // Y
-    if (!ctx->fz_ok[is_H ? 1 : 0] && (rc = prepare_b(ctx, !is_H))) return rc;   // X
-    TileSplit ts;
-    if ((rc = is_H ? dispatch_b<true>(ctx, plan->mapsH, plan->dErr, ts) : dispatch_b<false>(ctx, plan->mapsW, plan->dErr, ts)))
-        return rc;
-    switch (ctx->kp) {
-    case 16: rc = launch_finish_b<16>(ctx, is_H, ts, adjust); break;
-    case 32: rc = launch_finish_b<32>(ctx, is_H, ts, adjust); break;
-    default: rc = launch_finish_b<64>(ctx, is_H, ts, adjust); break;
-    }
+    if (!ctx->fz_ok[is_H ? 0 : 1] && (rc = finish_b(ctx, is_H, false, 0))) return rc;    // Y
+    if (!ctx->fz_ok[is_H ? 1 : 0] && (rc = finish_b(ctx, !is_H, false, 0))) return rc;   // X
+    rc = is_H ? dispatch_b<true>(ctx, plan->mapsH, plan) : dispatch_b<false>(ctx, plan->mapsW, plan);
+    if (!rc) rc = finish_b(ctx, !is_H, true, adjust);
     if (rc) return rc;
-    ctx->fz_ok[is_H ? 1 : 0] = 1;
     return nmfb_prof_end(ctx, whole);
 }
 
@@ -786,14 +741,9 @@ int nmfb_bf16_prepare(nmfb_ctx *ctx)
     size_t const wt = (size_t)((ctx->n + 63) / 64) * 128 * kp, ht = (size_t)((ctx->m + 63) / 64) * 128 * kp;
     cudaError_t e = nmfb_malloc(ctx, (void **)&plan->wsplit, (2 * wsz + wt) * sizeof(__nv_bfloat16));
     if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->hsplit, (2 * hsz + ht) * sizeof(__nv_bfloat16));
-    uint32_t const maxblk = fin_blocks(ctx->n > ctx->m ? ctx->n : ctx->m, 1);   // k_finish's most row blocks
-    plan->csoff = maxblk;
-    plan->nticks = (maxblk + FIN_ECH - 1) / FIN_ECH + 1;
-    if (e == cudaSuccess)
-        e = nmfb_malloc(ctx, (void **)&plan->dCs, (size_t)(maxblk + (maxblk + FIN_ECH - 1) / FIN_ECH) * kp * sizeof(double));
-    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dTick, plan->nticks * sizeof(uint32_t));
+    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dCsW, (size_t)fin_blocks(ctx->n, 1) * kp * sizeof(double));
+    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dCsH, (size_t)fin_blocks(ctx->m, 1) * kp * sizeof(double));
     if (e != cudaSuccess) return nmfb_fail(ctx, NMFB_ENOMEM, "bf16 split buffers: %s", cudaGetErrorString(e));
-    NMFB_CUDA_TRY(ctx, cudaMemsetAsync(plan->dTick, 0, plan->nticks * sizeof(uint32_t), ctx->own_stream));
     return NMFB_OK;
 }
 
@@ -803,8 +753,8 @@ int nmfb_bf16_release(nmfb_ctx *ctx)
     if (!plan) return NMFB_OK;
     if (plan->wsplit) nmfb_free(ctx, plan->wsplit);
     if (plan->hsplit) nmfb_free(ctx, plan->hsplit);
-    if (plan->dCs) nmfb_free(ctx, plan->dCs);
-    if (plan->dTick) nmfb_free(ctx, plan->dTick);
+    if (plan->dCsW) nmfb_free(ctx, plan->dCsW);
+    if (plan->dCsH) nmfb_free(ctx, plan->dCsH);
     free(plan);
     ctx->bplan = nullptr;
     return NMFB_OK;
@@ -818,5 +768,5 @@ int nmfb_bf16_update_W(nmfb_ctx *ctx, int adjust) { return bf16_half(ctx, false,
 int nmfb_bf16_ready_W(nmfb_ctx *ctx)
 {
     if (!ctx->bplan || ctx->fz_ok[0]) return NMFB_OK;
-    return prepare_b(ctx, true);
+    return finish_b(ctx, true, false, 0);
 }

@@ -7,12 +7,11 @@
 //
 //   TMA      : V tile (128 x BR, FP32) into a VST-deep ring; the Y tile
 //              operands of MMA1 and of MMA2 into a ring each.
-//   split    : k_split_factor, once per half-iteration, writes the other
-//              factor Y as TF32 hi (round to nearest) and the transposed hi/lo
-//              blocks that MMA2 reads K-major (lo = y - hi, exact; an MN-major
-//              read of a TF32 operand returns zeros on sm_100a), plus BF16
-//              copies bf16(lo), bf16(y) and bf16(y) transposed per tile; the Y
-//              producer TMA-loads them per tile.  X (128 rows per CTA) is split
+//   split    : k_finish, when it updates a factor, writes it as TF32 hi (round
+//              to nearest) and the transposed hi/lo blocks that MMA2 reads K-major
+//              (lo = y - hi, exact; an MN-major read of a TF32 operand returns
+//              zeros on sm_100a), plus BF16 copies bf16(lo), bf16(y) and bf16(y)
+//              transposed per tile; the Y producers TMA-load them per tile.  X (128 rows per CTA) is split
 //              once per CTA by the accumulator warps.
 //   MMA1     : D (TMEM, 128 x BR) = Xh Yh^T                    (kind::tf32, k-steps of 8)
 //              + [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T (kind::f16, K = 2 KP, k-steps of 16),
@@ -89,6 +88,7 @@ struct FusedMaps {
 struct FusedArgs {
     uint32_t O, R;        // output rows, reduction length
     TileSplit ts;
+    ColSum csy;           // column sums of the other factor
     float *part;          // [slot][O][KP]
     uint32_t *err;        // device error word
     const ConvState *st;
@@ -138,7 +138,7 @@ struct Geo {
     // Accumulator warps: sets of four, KP / NA columns each.  At KP = 64 tensor memory
     // holds one accumulator besides three D buffers, so it has to be read fast.
     static constexpr int NA = (KP == 64) ? 2 : 1;
-    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;
+    static constexpr int NTHR = (4 + NR + 4 * NA) * 32;   // (a multiple of four warps: one more would cost 8 registers a thread)
     static constexpr uint32_t ACC = 2 * KP;                // TMEM columns of one per-tile accumulator
     static constexpr uint32_t NACC = (KP == 64) ? 1 : 2;   // accumulators
     static constexpr uint32_t NDB = (KP == 16) ? 4 : 3;    // D buffers (MMA1 runs NDB tiles ahead)
@@ -160,58 +160,6 @@ struct Geo {
 // (KP/2 columns each), the A operands of MMA1 for every tile of that row block
 // (so MMA1 reads only Y from shared memory).
 
-// Split a factor Y (rows x kp, FP32, padding columns zero) for the fused
-// kernel's TMA loads, one CTA per block of `br` rows (br = the kernel's tile):
-//   hi = TF32(y) (round to nearest), rows x kp;
-//   T: per 32 rows, the transposed hi block (kp rows of 32 floats) followed by
-//      the transposed lo block (lo = y - hi, exact), rows past the end zero;
-//   Bl = bf16(lo), B = bf16(y): rows x kp each (kp = 16: lo, FP32, in their place);
-//   BT: per br rows, the transposed bf16(y) block (kp rows of br values), rows
-//      past the end zero.
-// The transposes go through shared memory.
-__global__ void __launch_bounds__(256) k_split_factor(const float *__restrict__ Y, uint32_t rows, uint32_t kp,
-                                                      uint32_t br, float *__restrict__ hi, float *__restrict__ T,
-                                                      __nv_bfloat16 *__restrict__ Bl, __nv_bfloat16 *__restrict__ B,
-                                                      __nv_bfloat16 *__restrict__ BT, const ConvState *st)
-{
-    if (st && *(volatile const uint32_t *)&st->converged) return;
-    __shared__ float th[64][65], tl[64][65];
-    __shared__ __nv_bfloat16 tb[64][66];
-    uint32_t const r0 = blockIdx.x * br;
-    for (uint32_t e = threadIdx.x; e < br * kp; e += blockDim.x) {
-        uint32_t const r = e / kp, c = e % kp;
-        bool const in = r0 + r < rows;
-        float const y = in ? Y[(size_t)(r0 + r) * kp + c] : 0.0f;
-        float const h = tf32_rna(y), l = y - h;
-        __nv_bfloat16 const yb = __float2bfloat16_rn(y);
-        if (in) {
-            hi[(size_t)(r0 + r) * kp + c] = h;
-            if (kp == 16) {
-                reinterpret_cast<float *>(Bl)[(size_t)(r0 + r) * kp + c] = l;
-            } else {
-                Bl[(size_t)(r0 + r) * kp + c] = __float2bfloat16_rn(l);
-                B[(size_t)(r0 + r) * kp + c] = yb;
-            }
-        }
-        th[r][c] = h;
-        tl[r][c] = l;
-        tb[r][c] = yb;
-    }
-    __syncthreads();
-    uint32_t const nblk32 = (rows + 31) / 32;
-    for (uint32_t sub = 0; sub < br / 32; sub++) {
-        uint32_t const blk = r0 / 32 + sub;
-        if (blk >= nblk32) break;
-        float *dst = T + (size_t)blk * 2 * kp * 32;
-        for (uint32_t e = threadIdx.x; e < 2 * kp * 32; e += blockDim.x) {
-            uint32_t const row = e / 32, rr = sub * 32 + e % 32;
-            dst[e] = row < kp ? th[rr][row] : tl[rr][row - kp];
-        }
-    }
-    __nv_bfloat16 *bt = BT + (size_t)blockIdx.x * kp * br;
-    for (uint32_t e = threadIdx.x; e < kp * br; e += blockDim.x) bt[e] = tb[e % br][e / br];
-}
-
 // Warp roles: 0 = V producer (TMA), 1 = MMA issuer + TMEM owner, 2, 3 = Y
 // producers (TMA), 4 .. 3 + NR = R warps (V / D, feed MMA2), the others =
 // accumulator warps (sum the per-tile MMA2 results in FP32 registers; split X).
@@ -228,7 +176,6 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     constexpr int BR = G::BR;
     constexpr int NR = G::NR;
     constexpr uint32_t ACC_COLS = G::ACC;
-    if (args.st && *(volatile const uint32_t *)&args.st->converged) return;
 
     extern __shared__ unsigned char smem_raw[];
     uint32_t const base_u32 = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -253,12 +200,13 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     uint32_t *const tmem_slot = reinterpret_cast<uint32_t *>(mdrain + 1);
     volatile uint32_t *const abort_flag = tmem_slot + 1;
 
+    chain_next();
     uint32_t const warp = uniform(threadIdx.x / 32), lane = threadIdx.x % 32;
     // This CTA's run of tiles [g0, g0 + T) of the whole (row block, reduction tile)
     // list, row-block-major: tile g is reduction tile g % TB of row block g / TB.
     uint32_t const TB = args.ts.tb;
     uint32_t const g0 = blockIdx.x * args.ts.tpc;
-    uint32_t const T = min(args.ts.total - g0, args.ts.tpc);
+    uint32_t T = min(args.ts.total - g0, args.ts.tpc);
     uint32_t const ob0 = g0 / TB, c00 = g0 - ob0 * TB;
 #ifdef NMFB_FUSED_DEBUG
     // Per-tile event times of block 0 (ns since kernel start), 8 events x 64 tiles.
@@ -317,12 +265,15 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
     __syncthreads();
     tc_fence_after();
     uint32_t const tmem = *tmem_slot;
+    chain_wait();   // nothing above reads or writes global memory
+    if (args.st && *(volatile const uint32_t *)&args.st->converged) T = 0;   // every role's loop is empty
 
     if (warp == 0) {
-        // ------------------------------------------------------------ V producer
+        // ------------------------------------------------------------ V producer, then the column sums of Y
+        uint32_t issued = 0;
         if (lane == 0) {
             uint64_t const pol = policy_evict_first();
-            uint32_t issued = 0, ob = ob0, c = c00;
+            uint32_t ob = ob0, c = c00;
             for (uint32_t t = 0; t < T; t++, ob += (c + 1 == TB), c = (c + 1 == TB) ? 0 : c + 1) {
                 uint32_t const s = t % G::VST;
                 if (t >= (uint32_t)G::VST &&
@@ -341,11 +292,14 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                         tma_load_2d(sv + b * (BO * 128), &maps.v, &vfull[s], r0 + 32 * b, o0, pol);
                 }
             }
+        }
+        __syncwarp();
+        if (T > 0) column_sums<KP>(args.csy);   // (while the last tiles are worked on; k_finish divides by them)
+        if (lane == 0)
             // drain: the last load into every stage has landed (each earlier one
             // had to, before its stage was released for reuse)
             for (uint32_t t = issued > (uint32_t)G::VST ? issued - G::VST : 0; t < issued; t++)
                 mbar_drain(&vfull[t % G::VST], (t / G::VST) & 1);
-        }
     } else if (warp == 2 || warp == 3) {
         // ------------------------------------------------------------ Y producers
         // warp 2: MMA1's operands, warp 3: MMA2's
@@ -804,7 +758,7 @@ int encode_2d(nmfb_ctx *ctx, CUtensorMap *map, const void *base, uint64_t inner,
     return NMFB_OK;
 }
 
-// Layout of one factor's split copies (k_split_factor's outputs), in one buffer:
+// Layout of one factor's split copies (k_finish's outputs), in one buffer:
 // hi (rows x kp FP32) | transposed hi/lo per 32 rows | bf16(lo) (rows x kp) |
 // bf16(y) (rows x kp) | bf16(y) transposed per br rows; at kp = 16 lo itself (FP32)
 // in place of bf16(lo) | bf16(y).
@@ -828,31 +782,64 @@ struct SplitLayout {
 struct FusedPlan {
     FusedMaps mapsH, mapsW;  // update_H (HSIDE) and update_W
     uint32_t *dErr;
-    float *dSplitW, *dSplitH;  // split copies of W and of H (k_split_factor, SplitLayout)
-    double *dCs;               // [row blocks + chunks][kp] column-sum partials of k_finish
-    uint32_t *dTick;           // [chunks + 1] retirement counters of k_finish
-    uint32_t nticks, csoff;
+    float *dSplitW, *dSplitH;  // split copies of W and of H (SplitLayout)
+    double *dCsW, *dCsH;       // [CTAs of k_finish][kp] column-sum partials of W and of H
 #ifdef NMFB_FUSED_DEBUG
     float *dDbg;
 #endif
 };
 
+// How the half-iteration that updates W (or H) is dealt out.
+TileSplit plan_of(const nmfb_ctx *ctx, bool w)
+{
+    return plan_tiles(w ? ctx->n : ctx->m, w ? ctx->m : ctx->n, 64, (uint32_t)ctx->sm_count, ctx->part_items / ctx->kp);
+}
+
+// k_finish on W (or H): its update from the partials, or, with update = false,
+// only its split copies and column-sum partials.
+template <int KP>
+int launch_finish(nmfb_ctx *ctx, bool w, bool update, int adjust)
+{
+    FusedPlan *plan = (FusedPlan *)ctx->tmaps;
+    FinishArgs fa = {};
+    float *xsp = w ? plan->dSplitW : plan->dSplitH;
+    fa.O = w ? ctx->n : ctx->m;
+    SplitLayout const L(fa.O, KP);
+    fa.ts = plan_of(ctx, w);
+    fa.k = ctx->k;
+    fa.adjust = adjust;
+    fa.part = update ? ctx->dPart : nullptr;
+    fa.X = w ? ctx->dW : ctx->dH;
+    fa.accY = w ? ctx->dAccH : ctx->dAccW;
+    fa.xhi = xsp;
+    fa.xT = xsp + L.t;
+    fa.xBl = reinterpret_cast<__nv_bfloat16 *>(xsp + L.bl);
+    fa.xB = reinterpret_cast<__nv_bfloat16 *>(xsp + L.b);
+    fa.xBT = reinterpret_cast<__nv_bfloat16 *>(xsp + L.bt);
+    fa.xnblk32 = L.nblk32;
+    fa.xnblkbr = L.nblkbr;
+    fa.cs = w ? plan->dCsW : plan->dCsH;
+    fa.st = ctx->dState;
+    NMFB_CUDA_TRY(ctx, (fin_launch<KP, 64, 0>(fa, ctx->stream)));
+    NMFB_LAUNCH_CHECK(ctx);
+    return NMFB_OK;
+}
+
 template <bool HSIDE, int KP, int NTERMS>
 int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
 {
     using G = Geo<KP>;
-    constexpr int BR = G::BR;
-    auto kern = k_fused_half<HSIDE, KP, NTERMS>;
+    static_assert(G::BR == 64, "plan_of");
     FusedPlan *plan = (FusedPlan *)ctx->tmaps;
-    uint32_t const O = HSIDE ? ctx->m : ctx->n;
-    uint32_t const R = HSIDE ? ctx->n : ctx->m;
-    TileSplit const ts = plan_tiles(O, R, BR, (uint32_t)ctx->sm_count, ctx->part_items / KP);
-    if ((size_t)ts.slots * O * KP > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "fused: partial buffer too small (%u slots)", ts.slots);
     FusedArgs args;
-    args.O = O;
-    args.R = R;
-    args.ts = ts;
+    args.O = HSIDE ? ctx->m : ctx->n;
+    args.R = HSIDE ? ctx->n : ctx->m;
+    args.ts = plan_of(ctx, !HSIDE);
+    if ((size_t)args.ts.slots * args.O * KP > ctx->part_items)
+        return nmfb_fail(ctx, NMFB_EINVAL, "fused: partial buffer too small (%u slots)", args.ts.slots);
+    args.csy.cs = HSIDE ? plan->dCsW : plan->dCsH;
+    args.csy.nblk = fin_blocks(args.R, fin_rpt(plan_of(ctx, HSIDE).slots));
+    args.csy.acc = HSIDE ? ctx->dAccW : ctx->dAccH;
     args.part = ctx->dPart;
     args.err = plan->dErr;
     args.st = ctx->dState;
@@ -864,38 +851,11 @@ int launch_fused(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     int const main = HSIDE ? 0 : 1;
     int rc = nmfb_prof_begin(ctx, main);
     if (rc) return rc;
-    kern<<<ts.ctas(), G::NTHR, G::SMEM, ctx->stream>>>(maps, args);
+    NMFB_CUDA_TRY(ctx, launch_chained(k_fused_half<HSIDE, KP, NTERMS>, args.ts.ctas(), G::NTHR, G::SMEM, ctx->stream, maps,
+                                      args));
     NMFB_LAUNCH_CHECK(ctx);
     if ((rc = nmfb_prof_end(ctx, main))) return rc;
-
-    FinishArgs fa;
-    float *xsp = HSIDE ? plan->dSplitH : plan->dSplitW;
-    SplitLayout const L(O, KP);
-    fa.O = O;
-    fa.ts = ts;
-    fa.k = ctx->k;
-    fa.adjust = adjust;
-    fa.part = ctx->dPart;
-    fa.X = HSIDE ? ctx->dH : ctx->dW;
-    fa.accY = HSIDE ? ctx->dAccW : ctx->dAccH;
-    fa.xhi = xsp;
-    fa.xT = xsp + L.t;
-    fa.xBl = reinterpret_cast<__nv_bfloat16 *>(xsp + L.bl);
-    fa.xB = reinterpret_cast<__nv_bfloat16 *>(xsp + L.b);
-    fa.xBT = reinterpret_cast<__nv_bfloat16 *>(xsp + L.bt);
-    fa.xnblk32 = L.nblk32;
-    fa.xnblkbr = L.nblkbr;
-    fa.cs = plan->dCs;
-    fa.csoff = plan->csoff;
-    fa.accX = HSIDE ? ctx->dAccH : ctx->dAccW;
-    fa.tick = plan->dTick;
-    fa.st = ctx->dState;
-    uint32_t const fblocks = fin_blocks(O, fin_rpt(ts.slots));
-    if (fblocks > plan->csoff || (fblocks + FIN_ECH - 1) / FIN_ECH + 1 > plan->nticks)
-        return nmfb_fail(ctx, NMFB_EINVAL, "fused: column-sum buffers too small");
-    fin_launch<KP, BR, 0>(fa, ctx->stream);
-    NMFB_LAUNCH_CHECK(ctx);
-    return NMFB_OK;
+    return launch_finish<KP>(ctx, !HSIDE, true, adjust);
 }
 
 template <bool HSIDE>
@@ -910,28 +870,19 @@ int dispatch(nmfb_ctx *ctx, const FusedMaps &maps, int adjust)
     }
 }
 
-// Split copies and column sums of a factor, for a half-iteration that reads
-// it as Y when the previous half-iteration's epilogue did not produce them.
+// Split copies and column-sum partials of a factor, for a half-iteration that
+// reads it as Y when the previous one's k_finish did not leave them.
 int prepare_factor(nmfb_ctx *ctx, bool w)
 {
-    FusedPlan *plan = (FusedPlan *)ctx->tmaps;
-    const float *F = w ? ctx->dW : ctx->dH;
-    uint32_t const rows = w ? ctx->n : ctx->m;
-    int rc = nmfb_colsum(ctx, F, rows, w ? ctx->dAccW : ctx->dAccH, w ? 0 : 1);
-    if (rc) return rc;
-    float *sp = w ? plan->dSplitW : plan->dSplitH;
-    SplitLayout const L(rows, ctx->kp);
-    k_split_factor<<<L.nblkbr, 256, 0, ctx->stream>>>(F, rows, ctx->kp, L.br, sp, sp + L.t,
-                                                     reinterpret_cast<__nv_bfloat16 *>(sp + L.bl),
-                                                     reinterpret_cast<__nv_bfloat16 *>(sp + L.b),
-                                                     reinterpret_cast<__nv_bfloat16 *>(sp + L.bt), ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    ctx->fz_ok[w ? 0 : 1] = 1;
-    return NMFB_OK;
+    int const rc = ctx->kp == 16   ? launch_finish<16>(ctx, w, false, 0)
+                   : ctx->kp == 32 ? launch_finish<32>(ctx, w, false, 0)
+                                   : launch_finish<64>(ctx, w, false, 0);
+    if (!rc) ctx->fz_ok[w ? 0 : 1] = 1;
+    return rc;
 }
 
-// One half-iteration: a single launch when the other factor's split copies and
-// column sums are current (the previous half-iteration's epilogue wrote them).
+// One half-iteration: two launches when the other factor's split copies and
+// column-sum partials are current (the previous half-iteration's k_finish left them).
 int fused_half(nmfb_ctx *ctx, bool is_H, int adjust)
 {
     FusedPlan *plan = (FusedPlan *)ctx->tmaps;
@@ -989,14 +940,9 @@ int nmfb_fused_prepare(nmfb_ctx *ctx)
     uint32_t const br = LW.br;
     e = nmfb_malloc(ctx, (void **)&plan->dSplitW, LW.floats * sizeof(float));
     if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dSplitH, LH.floats * sizeof(float));
-    uint32_t const maxblk = fin_blocks(ctx->n > ctx->m ? ctx->n : ctx->m, 1);   // k_finish's most row blocks
-    plan->csoff = maxblk;
-    plan->nticks = (maxblk + FIN_ECH - 1) / FIN_ECH + 1;
-    if (e == cudaSuccess)
-        e = nmfb_malloc(ctx, (void **)&plan->dCs, (size_t)(maxblk + (maxblk + FIN_ECH - 1) / FIN_ECH) * kp * sizeof(double));
-    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dTick, plan->nticks * sizeof(uint32_t));
+    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dCsW, (size_t)fin_blocks(ctx->n, 1) * kp * sizeof(double));
+    if (e == cudaSuccess) e = nmfb_malloc(ctx, (void **)&plan->dCsH, (size_t)fin_blocks(ctx->m, 1) * kp * sizeof(double));
     if (e != cudaSuccess) return nmfb_fail(ctx, NMFB_ENOMEM, "fused split buffers: %s", cudaGetErrorString(e));
-    NMFB_CUDA_TRY(ctx, cudaMemsetAsync(plan->dTick, 0, plan->nticks * sizeof(uint32_t), ctx->own_stream));
     // Maps over one factor's split copies: Y (the other factor, `rows` rows).
     auto const y_maps = [&](FusedMaps &mp, const float *sp, const SplitLayout &L, uint32_t rows) -> int {
         int r;
@@ -1031,8 +977,8 @@ int nmfb_fused_release(nmfb_ctx *ctx)
     if (plan->dErr) nmfb_free(ctx, plan->dErr);
     if (plan->dSplitW) nmfb_free(ctx, plan->dSplitW);
     if (plan->dSplitH) nmfb_free(ctx, plan->dSplitH);
-    if (plan->dCs) nmfb_free(ctx, plan->dCs);
-    if (plan->dTick) nmfb_free(ctx, plan->dTick);
+    if (plan->dCsW) nmfb_free(ctx, plan->dCsW);
+    if (plan->dCsH) nmfb_free(ctx, plan->dCsH);
     free(plan);
     ctx->tmaps = nullptr;
     return NMFB_OK;
@@ -1066,9 +1012,8 @@ int nmfb_fused_error(nmfb_ctx *ctx, uint32_t *code)
     NMFB_CUDA_TRY(ctx, cudaMemcpyAsync(code, plan->dErr, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
     NMFB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     if (*code) {
-        // an aborted launch may have left retirement counters and factor copies behind
+        // an aborted launch leaves factor copies behind that match no factor
         NMFB_CUDA_TRY(ctx, cudaMemsetAsync(plan->dErr, 0, sizeof(uint32_t), ctx->stream));
-        NMFB_CUDA_TRY(ctx, cudaMemsetAsync(plan->dTick, 0, plan->nticks * sizeof(uint32_t), ctx->stream));
         ctx->fz_ok[0] = ctx->fz_ok[1] = 0;
         NMFB_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
     }
