@@ -172,5 +172,13 @@ int nmfb_bf16_update_H(nmfb_ctx *ctx, int adjust);
 int nmfb_bf16_update_W(nmfb_ctx *ctx, int adjust);
 int nmfb_bf16_ready_W(nmfb_ctx *ctx);
 
+// ---- consensus.cu ---------------------------------------------------------
+size_t nmfb_summary_doubles(uint32_t m);
+size_t nmfb_summary_ints(uint32_t m);
+cudaError_t nmfb_launch_consensus(const uint32_t *const *labels, const uint32_t *sel, uint32_t nsel, uint32_t m,
+                                  uint32_t *C, cudaStream_t stream);
+cudaError_t nmfb_launch_cophenetic(const uint32_t *C, uint32_t m, uint32_t nruns, double *dbl, uint32_t *ints,
+                                   double **result, cudaStream_t stream);
+
 // Max number of reduction splits used by any arm (sizes dPart).
 #define NMFB_MAX_SPLIT 64
