@@ -13,8 +13,8 @@
 // part of the library's device image: every GPU that loads the library holds
 // it until the process exits.  Layout (offsets in bytes from the 256-aligned
 // base):
-//   [0, 32 KiB)            colpart: NA_MAX_SPLITS x 64 doubles, per-split column
-//                          sums of W
+//   [0, 32 KiB)            colpart: nsplit x k doubles (at most 4096), per-split
+//                          column sums of W
 //   [32 KiB, 16 MiB)       part:    nsplit x m x k floats, per-split partial
 //                          sums of Q^T W (Q = V ./ (W H^T))
 // Every scratch word a call reads is written earlier in the same call (each
@@ -36,6 +36,7 @@
 // variant of the engine's own update_H; results agree with nmfb_update_H to
 // FP32 rounding, not bit for bit.
 #include "../../include/nmfb200.h"
+#include "fused_common.cuh"
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -44,29 +45,59 @@
 namespace {
 
 constexpr size_t NA_SCRATCH_BYTES = (size_t)NMFB_NOALLOC_SCRATCH_BYTES;
-constexpr uint32_t NA_MAX_SPLITS = 64;
 constexpr uint32_t NA_KMAX = 64;
-constexpr size_t NA_COLPART_BYTES = (size_t)NA_MAX_SPLITS * NA_KMAX * sizeof(double);   // 32 KiB
+constexpr uint32_t NA_COLPARTS = 4096;
+constexpr size_t NA_COLPART_BYTES = (size_t)NA_COLPARTS * sizeof(double);   // 32 KiB
 constexpr size_t NA_PART_FLOATS = (NA_SCRATCH_BYTES - NA_COLPART_BYTES) / sizeof(float);
 static_assert(NA_PART_FLOATS == (size_t)NMFB_NOALLOC_MAX_MK, "header limit and scratch layout disagree");
 
-constexpr int NA_THREADS = 256;   // one column j of V (one sample) per thread
+constexpr int NA_THREADS = 128;   // one column j of V (one sample) per thread
 constexpr int NA_WT = 32;         // rows of W staged in shared memory per step
+constexpr int NA_VG = 4;          // rows of V a thread has in flight ahead of the ones it works on
+constexpr int NA_FIN = 256;       // threads of a k_na_finish CTA
 constexpr int NA_MAX_DEV = 64;
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[NA_SCRATCH_BYTES];
 
-// CTA (x, s) covers samples j in [256x, 256x+256) and rows i of split s.
+// Two FP32 values in a register pair; fma.rn.f32x2 is two FMAs in one instruction.
+typedef unsigned long long pair_t;
+__device__ __forceinline__ pair_t pair_of(float lo, float hi)
+{
+    pair_t d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 halves(pair_t p)
+{
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
+    return f;
+}
+__device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c)
+{
+    pair_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// CTA (x, s) covers samples j in [NT x, NT x + NT) and rows i of split s.
 // part[s][j][c] = sum_{i in split s} V[i][j] / (W_i . H_j) * W[i][c];
 // CTAs with x == 0 also write colpart[s][c] = sum_{i in split s} W[i][c] (FP64).
+// Bound by FP32 issue: KB packed FMAs (KB = k rounded up to 4), a division and
+// KB / 4 broadcast loads an element.  V's next rows and the next tile of W are
+// loaded ahead (a thread that loaded each V where it was used, with k padded to
+// 32, took 162 us for 20000 x 1000 at k = 20).
 template <int KB>
-__global__ void __launch_bounds__(NA_THREADS) k_na_partials(const float *__restrict__ V, size_t ldv,
-                                                            const float *__restrict__ W, size_t ldw,
-                                                            const float *__restrict__ H, size_t ldh, uint32_t n,
-                                                            uint32_t m, uint32_t k, uint32_t rows_per_split,
-                                                            float *__restrict__ part, double *__restrict__ colpart)
+__global__ void __launch_bounds__(NA_THREADS, KB <= 32 ? 4 : 2)
+    k_na_partials(const float *__restrict__ V, size_t ldv, const float *__restrict__ W, size_t ldw,
+                  const float *__restrict__ H, size_t ldh, uint32_t n, uint32_t m, uint32_t k, uint32_t rows_per_split,
+                  float *__restrict__ part, double *__restrict__ colpart)
 {
-    __shared__ float sW[NA_WT][KB];
+    static_assert(KB % 4 == 0, "rows of W as 16-byte vectors");
+    constexpr int K2 = KB / 2, PER = NA_WT * KB / NA_THREADS;   // floats of a W tile per thread
+    constexpr int SEG = NA_THREADS / KB;                        // row lanes of the column sums
+    __shared__ __align__(16) float sW[2][NA_WT][KB];
+    __shared__ double sC[SEG][KB];
     uint32_t const tid = threadIdx.x;
     uint32_t const j = blockIdx.x * NA_THREADS + tid;
     uint32_t const s = blockIdx.y;
@@ -76,61 +107,121 @@ __global__ void __launch_bounds__(NA_THREADS) k_na_partials(const float *__restr
     uint32_t const r0 = r0_wide < n ? (uint32_t)r0_wide : n;
     uint32_t const r1 = (uint64_t)r0 + rows_per_split < n ? r0 + rows_per_split : n;
 
-    float h[KB], acc[KB];
+    pair_t h[K2], acc[K2];
 #pragma unroll
-    for (int c = 0; c < KB; c++) {
-        h[c] = (active && (uint32_t)c < k) ? H[(size_t)j * ldh + c] : 0.0f;
-        acc[c] = 0.0f;
+    for (int c = 0; c < K2; c++) {
+        h[c] = pair_of((active && 2u * c < k) ? H[(size_t)j * ldh + 2 * c] : 0.0f,
+                       (active && 2u * c + 1 < k) ? H[(size_t)j * ldh + 2 * c + 1] : 0.0f);
+        acc[c] = 0;
     }
     double cs = 0.0;
-    for (uint32_t i0 = r0; i0 < r1; i0 += NA_WT) {
-        uint32_t const rows = min((uint32_t)NA_WT, r1 - i0);
-        __syncthreads();
-        for (uint32_t e = tid; e < (uint32_t)(NA_WT * KB); e += NA_THREADS) {
-            uint32_t const r = e / KB, c = e % KB;
-            sW[r][c] = (r < rows && c < k) ? W[(size_t)(i0 + r) * ldw + c] : 0.0f;
+    uint32_t const cc = tid % KB, seg = tid / KB;
+    float wreg[PER];
+    auto const load_w = [&](uint32_t i0) {
+#pragma unroll
+        for (int e = 0; e < PER; e++) {
+            uint32_t const r = (tid + e * NA_THREADS) / KB, c = (tid + e * NA_THREADS) % KB;
+            wreg[e] = (i0 + r < r1 && c < k) ? W[(size_t)(i0 + r) * ldw + c] : 0.0f;
         }
-        __syncthreads();
-        if (colsum_cta && tid < (uint32_t)KB)
-            for (uint32_t r = 0; r < rows; r++) cs += (double)sW[r][tid];
-        if (active) {
-            for (uint32_t r = 0; r < rows; r++) {
-                float wh = 0.0f;
+    };
+    auto const store_w = [&](uint32_t b) {
 #pragma unroll
-                for (int c = 0; c < KB; c++) wh = fmaf(sW[r][c], h[c], wh);
-                float const q = V[(size_t)(i0 + r) * ldv + j] / wh;
+        for (int e = 0; e < PER; e++) (&sW[b][0][0])[tid + e * NA_THREADS] = wreg[e];
+    };
+    float v[NA_VG], vn[NA_VG];
+    auto const load_v = [&](uint32_t i0) {
 #pragma unroll
-                for (int c = 0; c < KB; c++) acc[c] = fmaf(q, sW[r][c], acc[c]);
+        for (int r = 0; r < NA_VG; r++) vn[r] = (active && i0 + r < r1) ? V[(size_t)(i0 + r) * ldv + j] : 0.0f;
+    };
+    load_w(r0);
+    load_v(r0);
+    uint32_t b = 0;
+    for (uint32_t i0 = r0; i0 < r1; i0 += NA_WT, b ^= 1u) {
+        uint32_t const rows = min((uint32_t)NA_WT, r1 - i0);
+        store_w(b);
+        __syncthreads();   // (a buffer is rewritten two tiles on: past this barrier of the next tile)
+        if (i0 + NA_WT < r1) load_w(i0 + NA_WT);
+        if (colsum_cta && seg < (uint32_t)SEG)
+            for (uint32_t r = seg; r < rows; r += SEG) cs += (double)sW[b][r][cc];
+        for (uint32_t g = 0; g < rows; g += NA_VG) {
+#pragma unroll
+            for (int r = 0; r < NA_VG; r++) v[r] = vn[r];
+            load_v(i0 + g + NA_VG);
+#pragma unroll
+            for (int r = 0; r < NA_VG; r++) {
+                if (g + r >= rows) break;   // (uniform)
+                pair_t w[K2];
+#pragma unroll
+                for (int q = 0; q < KB / 4; q++) {
+                    ulonglong2 const x = reinterpret_cast<const ulonglong2 *>(&sW[b][g + r][0])[q];
+                    w[2 * q] = x.x;
+                    w[2 * q + 1] = x.y;
+                }
+                pair_t sum = 0;
+#pragma unroll
+                for (int c = 0; c < K2; c++) sum = fma2(w[c], h[c], sum);
+                float2 const wh = halves(sum);
+                float const q = v[r] / (wh.x + wh.y);
+                pair_t const q2 = pair_of(q, q);
+#pragma unroll
+                for (int c = 0; c < K2; c++) acc[c] = fma2(q2, w[c], acc[c]);
             }
         }
     }
     if (active) {
         float *dst = part + ((size_t)s * m + j) * k;
 #pragma unroll
-        for (int c = 0; c < KB; c++)
-            if ((uint32_t)c < k) dst[c] = acc[c];
+        for (int c = 0; c < K2; c++) {
+            float2 const a = halves(acc[c]);
+            if (2u * c < k) dst[2 * c] = a.x;
+            if (2u * c + 1 < k) dst[2 * c + 1] = a.y;
+        }
     }
-    if (colsum_cta && tid < k) colpart[(size_t)s * NA_KMAX + tid] = cs;
+    if (colsum_cta) {   // the row lanes in order
+        if (seg < (uint32_t)SEG) sC[seg][cc] = cs;
+        __syncthreads();
+        if (tid < k) {
+            double t = 0.0;
+            for (int l = 0; l < SEG; l++) t += sC[l][tid];
+            colpart[(size_t)s * k + tid] = t;
+        }
+    }
 }
 
-// H[j][c] = (H[j][c] * sum_s part[s][j][c]) / (float)sum_s colpart[s][c],
-// both sums in split order.
-__global__ void __launch_bounds__(NA_THREADS) k_na_finish(float *__restrict__ H, size_t ldh, uint32_t m, uint32_t k,
-                                                          uint32_t nsplit, const float *__restrict__ part,
-                                                          const double *__restrict__ colpart)
+// H[j][c] = (H[j][c] * sum_s part[s][j][c]) / (float)sum_s colpart[s][c], the
+// partials in split order; the column sums once per CTA, by eight lanes a column
+// (splits l, l + 8, ... in order, then a shuffle tree).
+__global__ void __launch_bounds__(NA_FIN) k_na_finish(float *__restrict__ H, size_t ldh, uint32_t m, uint32_t k,
+                                                      uint32_t nsplit, const float *part, const double *colpart)
 {
+    nmfb_tc::chain_wait();
+    __shared__ float sA[NA_KMAX];
+    for (uint32_t c0 = 0; c0 < k; c0 += NA_FIN / 8) {
+        uint32_t const c = c0 + threadIdx.x / 8;
+        double a = 0.0;
+        if (c < k)
+            for (uint32_t q = threadIdx.x % 8; q < nsplit; q += 8) a += __ldcg(colpart + (size_t)q * k + c);
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+        if (c < k && threadIdx.x % 8 == 0) sA[c] = (float)a;
+    }
+    __syncthreads();
     size_t const total = (size_t)m * k;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (size_t)gridDim.x * blockDim.x) {
         uint32_t const j = (uint32_t)(idx / k), c = (uint32_t)(idx % k);
-        float s = 0.0f;
-        double a = 0.0;
-        for (uint32_t q = 0; q < nsplit; q++) {
-            s += part[(size_t)q * total + idx];
-            a += colpart[(size_t)q * NA_KMAX + c];
-        }
         float *hp = H + (size_t)j * ldh + c;
-        *hp = __fdiv_rn(*hp * s, (float)a);
+        float const h = *hp;
+        float s = 0.0f;
+        for (uint32_t q = 0; q < nsplit; q += 8) {
+            float p[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) p[i] = q + i < nsplit ? __ldcg(part + (size_t)(q + i) * total + idx) : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (q + i < nsplit) s += p[i];
+        }
+        *hp = __fdiv_rn(h * s, sA[c]);
     }
 }
 
@@ -226,13 +317,13 @@ extern "C" int nmfb_update_H_noalloc(const float *V, size_t ldv, const float *W,
     float *part = reinterpret_cast<float *>(slot.scratch + NA_COLPART_BYTES);
     cudaStream_t const st = static_cast<cudaStream_t>(stream);
 
-    // Splits over the rows of V: enough CTAs for ~4 per SM, limited by the
-    // scratch (nsplit * m * k floats), by NA_MAX_SPLITS and by n.
+    // Splits over the rows of V: four CTAs per SM in one wave, limited by the
+    // scratch (nsplit * m * k floats, nsplit * k column sums) and by n.
     uint32_t const xblocks = (m + NA_THREADS - 1) / NA_THREADS;
-    uint64_t want = ((uint64_t)4 * slot.sm_count + xblocks - 1) / xblocks;
+    uint64_t want = (uint64_t)4 * slot.sm_count / xblocks;
     uint64_t const fit = (uint64_t)NA_PART_FLOATS / ((uint64_t)m * k);
     if (want > fit) want = fit;
-    if (want > NA_MAX_SPLITS) want = NA_MAX_SPLITS;
+    if (want > NA_COLPARTS / k) want = NA_COLPARTS / k;
     if (want > n) want = n;
     if (want < 1) want = 1;
     uint32_t const rps = (uint32_t)((n + want - 1) / want);
@@ -240,19 +331,24 @@ extern "C" int nmfb_update_H_noalloc(const float *V, size_t ldv, const float *W,
 
     dim3 const grid(xblocks, nsplit);
     cudaError_t e;
-    if (k <= 16)
-        e = launch_partials<16>(grid, st, V, ldv, W, ldw, H, ldh, n, m, k, rps, part, colpart);
-    else if (k <= 32)
-        e = launch_partials<32>(grid, st, V, ldv, W, ldw, H, ldh, n, m, k, rps, part, colpart);
-    else
-        e = launch_partials<64>(grid, st, V, ldv, W, ldw, H, ldh, n, m, k, rps, part, colpart);
+    switch ((k + 3) / 4) {
+#define NA_CASE(Q) \
+    case Q: e = launch_partials<4 * Q>(grid, st, V, ldv, W, ldw, H, ldh, n, m, k, rps, part, colpart); break;
+        NA_CASE(1) NA_CASE(2) NA_CASE(3) NA_CASE(4) NA_CASE(5) NA_CASE(6) NA_CASE(7) NA_CASE(8)
+        NA_CASE(9) NA_CASE(10) NA_CASE(11) NA_CASE(12) NA_CASE(13) NA_CASE(14) NA_CASE(15)
+#undef NA_CASE
+    default: e = launch_partials<64>(grid, st, V, ldv, W, ldw, H, ldh, n, m, k, rps, part, colpart); break;
+    }
     if (e != cudaSuccess) return NMFB_ECUDA;
 
     uint64_t const total = (uint64_t)m * k;
-    uint64_t blocks = (total + NA_THREADS - 1) / NA_THREADS;
+    uint64_t blocks = (total + NA_FIN - 1) / NA_FIN;
     uint64_t const cap = (uint64_t)8 * slot.sm_count;
     if (blocks > cap) blocks = cap;
-    k_na_finish<<<(unsigned)blocks, NA_THREADS, 0, st>>>(H, ldh, m, k, nsplit, part, colpart);
-    if (cudaGetLastError() != cudaSuccess) return NMFB_ECUDA;
+    if (nmfb_tc::launch_chained(k_na_finish, dim3((unsigned)blocks), NA_FIN, 0, st, H, ldh, m, k, nsplit,
+                                (const float *)part, (const double *)colpart) != cudaSuccess) {
+        cudaGetLastError();
+        return NMFB_ECUDA;
+    }
     return NMFB_OK;
 }
