@@ -362,12 +362,24 @@ int nmfb_batch_get_WH(nmfb_batch *b, uint32_t p, float *W, size_t ldw, float *H,
     uint32_t const k = b->ranks[p], ks = ks_of(k);
     if ((W && ldw < k) || (H && ldh < k)) return bfail(b, NMFB_EINVAL, "leading dimension below k");
     BTRY(b, cudaSetDevice(b->device));
-    if (W)
-        BTRY(b, cudaMemcpy2D(W, ldw * sizeof(float), b->dW + b->woff[p], ks * sizeof(float), k * sizeof(float), b->n,
-                             cudaMemcpyDeviceToHost));
-    if (H)
-        BTRY(b, cudaMemcpy2D(H, ldh * sizeof(float), b->dH + b->hoff[p], ks * sizeof(float), k * sizeof(float), b->m,
-                             cudaMemcpyDeviceToHost));
+    // Through a page-locked staging buffer in one DMA each (a pitched copy into
+    // pageable memory moves one short row at a time).
+    auto const fetch = [&](float *dst, size_t ld, const float *src, uint32_t rows) -> cudaError_t {
+        size_t const bytes = (size_t)rows * ks * sizeof(float);
+        float *const stage = (float *)nmfb_stage_get(bytes);
+        if (!stage)
+            return cudaMemcpy2D(dst, ld * sizeof(float), src, ks * sizeof(float), k * sizeof(float), rows,
+                                cudaMemcpyDeviceToHost);
+        cudaError_t e = cudaMemcpyAsync(stage, src, bytes, cudaMemcpyDeviceToHost, b->stream);
+        cudaError_t const es = cudaStreamSynchronize(b->stream);
+        if (e == cudaSuccess) e = es;
+        if (e == cudaSuccess)
+            for (uint32_t r = 0; r < rows; r++) memcpy(dst + (size_t)r * ld, stage + (size_t)r * ks, k * sizeof(float));
+        nmfb_stage_put(stage);
+        return e;
+    };
+    if (W) BTRY(b, fetch(W, ldw, b->dW + b->woff[p], b->n));
+    if (H) BTRY(b, fetch(H, ldh, b->dH + b->hoff[p], b->m));
     return NMFB_OK;
 }
 
