@@ -78,13 +78,13 @@ __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.laun
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... P, class... A>
-cudaError_t launch_chained(void (*kern)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t stream, A &&...args)
+cudaError_t launch_chained(void (*kern)(P...), dim3 grid, uint32_t block, size_t smem, cudaStream_t stream, A &&...args)
 {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid, 1, 1);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

@@ -36,32 +36,32 @@ __device__ __forceinline__ float adjust_value(float v) { return fmaxf(v, FLT_MIN
 // Column sums: block b reduces rows [r0, r1) of X (rows x kp) into part[b][*];
 // the last block to retire sums the block partials (FP64) in a fixed order:
 // thread group g (of blockDim / kp) sums blocks g, g + groups, ... in order,
-// then the groups are added in order.  Many short blocks with four loads in
-// flight per thread keep the reads bandwidth-bound rather than latency-bound.
-__global__ void k_colsum(const float *__restrict__ X, uint32_t rows, uint32_t kp, double *__restrict__ part,
-                         float *__restrict__ acc, uint32_t *__restrict__ ticket, const ConvState *st)
+// then the groups are added in order.  Latency-bound: blocks of 1024 threads,
+// so that few blocks (and with them a short last sum) cover the rows, and four
+// rows in flight per thread (256-thread blocks of 32 rows: 20 us at 8000 x 128).
+constexpr int CS_NT = 1024;
+__global__ void __launch_bounds__(CS_NT) k_colsum(const float *__restrict__ X, uint32_t rows, uint32_t kp,
+                                                  double *__restrict__ part, float *__restrict__ acc,
+                                                  uint32_t *__restrict__ ticket, const ConvState *st)
 {
     if (halted(st)) return;
-    __shared__ double red[256];
+    __shared__ double red[CS_NT];
     __shared__ bool is_last;
-    uint32_t const lanes = blockDim.x / kp;  // row lanes per block
+    uint32_t const lanes = CS_NT / kp;  // row lanes per block
     uint32_t const c = threadIdx.x % kp;
     uint32_t const rl = threadIdx.x / kp;
     uint32_t const per = (rows + gridDim.x - 1) / gridDim.x;
-    uint32_t const r0 = blockIdx.x * per;
+    uint32_t const r0 = min(rows, blockIdx.x * per);
     uint32_t const r1 = min(rows, r0 + per);
     double s = 0.0;
     if (rl < lanes) {
-        uint32_t r = r0 + rl;
-        for (; r + 3 * lanes < r1; r += 4 * lanes) {
-            float const a0 = X[(size_t)r * kp + c], a1 = X[(size_t)(r + lanes) * kp + c];
-            float const a2 = X[(size_t)(r + 2 * lanes) * kp + c], a3 = X[(size_t)(r + 3 * lanes) * kp + c];
-            s += (double)a0;
-            s += (double)a1;
-            s += (double)a2;
-            s += (double)a3;
+        for (uint32_t r = r0 + rl; r < r1; r += 4 * lanes) {
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) v[i] = r + i * lanes < r1 ? X[(size_t)(r + i * lanes) * kp + c] : 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) s += (double)v[i];
         }
-        for (; r < r1; r += lanes) s += (double)X[(size_t)r * kp + c];
     }
     red[threadIdx.x] = s;
     __syncthreads();
@@ -78,15 +78,20 @@ __global__ void k_colsum(const float *__restrict__ X, uint32_t rows, uint32_t kp
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    uint32_t const groups = lanes;
     double t = 0.0;
-    if (rl < groups)
-        for (uint32_t b = rl; b < gridDim.x; b += groups) t += __ldcg(&part[(size_t)b * kp + c]);
+    if (rl < lanes)
+        for (uint32_t b = rl; b < gridDim.x; b += 8 * lanes) {
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = b + i * lanes < gridDim.x ? __ldcg(&part[(size_t)(b + i * lanes) * kp + c]) : 0.0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) t += v[i];
+        }
     red[threadIdx.x] = t;
     __syncthreads();
     if (threadIdx.x < kp) {
         double u = 0.0;
-        for (uint32_t g = 0; g < groups; g++) u += red[g * kp + threadIdx.x];
+        for (uint32_t g = 0; g < lanes; g++) u += red[g * kp + threadIdx.x];
         acc[threadIdx.x] = (float)u;
     }
     if (threadIdx.x == 0) *ticket = 0u;
@@ -115,7 +120,14 @@ __global__ void __launch_bounds__(256) k_factor(int mode, float *__restrict__ X,
         if (c < k) {
             if (mode == FU_MULDIV) {
                 float s = 0.0f;
-                for (uint32_t q = 0; q < nsplit; q++) s += part[q * split_stride + idx];
+                for (uint32_t q = 0; q < nsplit; q += 8) {   // eight splits' loads in flight, added in split order
+                    float p[8];
+#pragma unroll
+                    for (int i = 0; i < 8; i++) p[i] = q + i < nsplit ? part[(q + i) * split_stride + idx] : 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 8; i++)
+                        if (q + i < nsplit) s += p[i];
+                }
                 v = __fdiv_rn(X[idx] * s, acc[c]);
                 if (adjust) v = adjust_value(v);
             } else {
@@ -369,11 +381,12 @@ inline unsigned grid_for(size_t items, unsigned block, unsigned cap)
 // ---------------------------------------------------------------------------
 int nmfb_colsum(nmfb_ctx *ctx, const float *X, uint32_t rows, float *acc, int which)
 {
-    unsigned const block = 256;
-    unsigned grid = (rows + 31) / 32;        // ~32 rows per block; at most 1024 block partials
+    // four rows per thread where that leaves at most a block per SM (1024 partials fit)
+    unsigned const rows_per = 4 * (CS_NT / ctx->kp);
+    unsigned grid = (rows + rows_per - 1) / rows_per;
+    if (grid > (unsigned)ctx->sm_count) grid = (unsigned)ctx->sm_count;
     if (grid > 1024u) grid = 1024u;
-    if (grid < 1) grid = 1;
-    k_colsum<<<grid, block, 0, ctx->stream>>>(X, rows, ctx->kp, ctx->dColPart + (size_t)which * 1024 * ctx->kp, acc,
+    k_colsum<<<grid, CS_NT, 0, ctx->stream>>>(X, rows, ctx->kp, ctx->dColPart + (size_t)which * 1024 * ctx->kp, acc,
                                              ctx->dTickets + which, ctx->dState);
     NMFB_LAUNCH_CHECK(ctx);
     return NMFB_OK;

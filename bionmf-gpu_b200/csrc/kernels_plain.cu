@@ -1,168 +1,225 @@
-// kernels_plain.cu -- the unfused FP32 SIMT arm (NMFB_ARM_PLAIN).
+// kernels_plain.cu -- the unfused FP32 SIMT arm (NMFB_ARM_PLAIN), the arm of
+// ranks above 64 and of the blockwise mode.
 //
-// It keeps the reference's five-step structure of a half-iteration
+// It keeps the structure of the reference's half-iteration
 // (src/NMF_routines.c:376-525 / 1014-1164), with the n x m quotient
 // materialised in HBM, but with hand-written kernels instead of cuBLAS:
 //   1. acc  = colsum(W or H)                 (k_colsum, kernels_common.cu)
-//   2. WH   = W * H^T        -> n x m         (k_gemm_nt)
-//   3. WH   = V ./ WH                         (k_div)
-//   4. Xaux = reduce(WH, other factor)        (k_gemm_red, split over the reduction)
-//   5. X    = X .* Xaux ./ acc                (k_muldiv, kernels_common.cu)
-// It is the measured "plain" baseline that the fused arm is compared against.
+//   2. Q    = V ./ (W * H^T)    -> n x m      (k_quot)
+//   3. Xaux = reduce(Q, other factor)         (k_red, split over the reduction)
+//   4. X    = X .* Xaux ./ acc                (k_factor, kernels_common.cu)
+// Both contractions are bound by FP32 issue: 2 n m k flops each, 72 TFLOP/s.
 #include "nmfb_internal.cuh"
+#include "fused_common.cuh"
 
 using nmfb::ConvState;
+using nmfb_tc::chain_next;
+using nmfb_tc::chain_wait;
+using nmfb_tc::launch_chained;
 
 namespace {
 
 __device__ __forceinline__ bool halted(const ConvState *st) { return st && *(volatile const uint32_t *)&st->converged; }
 
-// C[i][j] = sum_c A[i][c] * B[j][c]; A: ra x kp, B: rb x kp (row-major), C: ra x ldc.
-// 64 x 64 output tile per block, 256 threads, 4 x 4 outputs per thread.
-__global__ void __launch_bounds__(256) k_gemm_nt(const float *__restrict__ A, const float *__restrict__ B,
-                                                 float *__restrict__ Cm, uint32_t ra, uint32_t rb, uint32_t kp,
-                                                 size_t ldc, const ConvState *st)
+// Both kernels: a 128 x 64 output tile per CTA of 128 threads, 8 x 8 outputs per
+// thread (rows 4 ty + {0..3} and 64 + 4 ty + .., columns 4 tx + .. and 32 + 4 tx +
+// ..: every shared load is 16 bytes wide, conflict-free or broadcast, and feeds 16
+// FMAs), 16 steps of the reduction staged at a time, the next 16 in registers
+// meanwhile.
+constexpr int TM = 128, TN = 64, TK = 16;
+
+struct Tile {
+    float a[2][TK][TM + 4];
+    float b[2][TK][TN + 4];
+};
+
+__device__ __forceinline__ void tile_fma(const float (&a)[TK][TM + 4], const float (&b)[TK][TN + 4], uint32_t tx,
+                                         uint32_t ty, float (&acc)[8][8])
 {
-    if (halted(st)) return;
-    __shared__ float As[16][64 + 4];
-    __shared__ float Bs[16][64 + 4];
-    uint32_t const tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    uint32_t const i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (uint32_t c0 = 0; c0 < kp; c0 += 16) {
-        for (uint32_t e = threadIdx.x; e < 64 * 16; e += 256) {
-            uint32_t const r = e / 16, c = e % 16;
-            uint32_t const ia = i0 + r, jb = j0 + r;
-            As[c][r] = (ia < ra) ? A[(size_t)ia * kp + c0 + c] : 0.0f;
-            Bs[c][r] = (jb < rb) ? B[(size_t)jb * kp + c0 + c] : 0.0f;
-        }
-        __syncthreads();
 #pragma unroll
-        for (uint32_t c = 0; c < 16; c++) {
-            float a[4], b[4];
+    for (int kk = 0; kk < TK; kk++) {
+        float4 const a0 = *reinterpret_cast<const float4 *>(&a[kk][4 * ty]);
+        float4 const a1 = *reinterpret_cast<const float4 *>(&a[kk][64 + 4 * ty]);
+        float4 const b0 = *reinterpret_cast<const float4 *>(&b[kk][4 * tx]);
+        float4 const b1 = *reinterpret_cast<const float4 *>(&b[kk][32 + 4 * tx]);
+        float const av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        float const bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-            for (int q = 0; q < 4; q++) { a[q] = As[c][ty * 4 + q]; b[q] = Bs[c][tx * 4 + q]; }
+        for (int p = 0; p < 8; p++)
 #pragma unroll
-            for (int p = 0; p < 4; p++)
-#pragma unroll
-                for (int q = 0; q < 4; q++) acc[p][q] = fmaf(a[p], b[q], acc[p][q]);
-        }
-        __syncthreads();
+            for (int q = 0; q < 8; q++) acc[p][q] = fmaf(av[p], bv[q], acc[p][q]);
     }
+}
+
+// Q = V ./ (W H^T) over n x m (matrix_div_sub in division mode; the reference uses
+// fdividef, src/GPU_kernels.cu:1687-1695), the quotient in the epilogue of the
+// product: no pass over V and W H^T of its own.  W: n x kp, H: m x kp (padding
+// columns zero), V and Q: leading dimension ld, a multiple of 32; padding columns
+// are neither used nor written.
+__global__ void __launch_bounds__(128, 4) k_quot(const float *__restrict__ V, const float *W, const float *H, float *Q,
+                                                 uint32_t n, uint32_t m, uint32_t kp, uint32_t k, size_t ld,
+                                                 const ConvState *st)
+{
+    chain_next();
+    chain_wait();
+    if (halted(st)) return;
+    __shared__ __align__(16) Tile s;
+    uint32_t const tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
+    uint32_t const i0 = blockIdx.y * TM, j0 = blockIdx.x * TN;
+    // staging: thread t holds row t of W (16 columns) and half of row t % 64 of H
+    bool const ina = i0 + tid < n, inb = j0 + tid % TN < m;
+    const float *pa = W + (size_t)(i0 + tid) * kp;
+    const float *pb = H + (size_t)(j0 + tid % TN) * kp + tid / TN * 8;
+    float4 ra[4], rb[2];
+    float4 const zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    auto const load = [&](uint32_t c0) {
 #pragma unroll
-    for (int p = 0; p < 4; p++) {
-        uint32_t const i = i0 + ty * 4 + p;
-        if (i >= ra) continue;
+        for (int q = 0; q < 4; q++) ra[q] = ina ? __ldcg(reinterpret_cast<const float4 *>(pa + c0) + q) : zero;
+#pragma unroll
+        for (int q = 0; q < 2; q++) rb[q] = inb ? __ldcg(reinterpret_cast<const float4 *>(pb + c0) + q) : zero;
+    };
+    auto const store = [&](uint32_t buf) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            uint32_t const j = j0 + tx * 4 + q;
-            if (j < rb) Cm[(size_t)i * ldc + j] = acc[p][q];
+            s.a[buf][4 * q + 0][tid] = ra[q].x;
+            s.a[buf][4 * q + 1][tid] = ra[q].y;
+            s.a[buf][4 * q + 2][tid] = ra[q].z;
+            s.a[buf][4 * q + 3][tid] = ra[q].w;
         }
+        uint32_t const r = tid % TN, c = tid / TN * 8;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            s.b[buf][c + 4 * q + 0][r] = rb[q].x;
+            s.b[buf][c + 4 * q + 1][r] = rb[q].y;
+            s.b[buf][c + 4 * q + 2][r] = rb[q].z;
+            s.b[buf][c + 4 * q + 3][r] = rb[q].w;
+        }
+    };
+    float acc[8][8] = {};
+    uint32_t const steps = (k + TK - 1) / TK;   // (kp is a multiple of 16)
+    load(0);
+    // V's tile into L2 while the product runs: each line once, by one of its eight threads
+    if (tx == 0)
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            uint32_t const i = i0 + (p < 4 ? 0u : 64u) + 4 * ty + (p & 3);
+#pragma unroll
+            for (uint32_t j = j0; j < j0 + TN; j += 32)
+                if (i < n && j < m) asm volatile("prefetch.global.L2 [%0];" ::"l"(V + (size_t)i * ld + j));
+        }
+    store(0);
+    __syncthreads();
+    for (uint32_t t = 0; t < steps; t++) {
+        if (t + 1 < steps) load((t + 1) * TK);
+        tile_fma(s.a[t & 1], s.b[t & 1], tx, ty, acc);
+        if (t + 1 < steps) store((t + 1) & 1);
+        __syncthreads();
     }
-}
-
-// WH = V ./ WH over the n x m region (matrix_div_sub in division mode; the
-// reference uses fdividef, src/GPU_kernels.cu:1687-1695).  Rows over
-// blockIdx.y, columns in float4 chunks over blockIdx.x (rows start on
-// 128-byte boundaries: ld is a multiple of 32); a ragged tail of m % 4 columns
-// element by element.  Padding columns are neither read nor written.
-__global__ void k_div(const float *__restrict__ V, float *__restrict__ WH, uint32_t n, uint32_t m, size_t ld,
-                      const ConvState *st)
-{
-    if (halted(st)) return;
-    uint32_t const m4 = m / 4;
-    for (uint32_t i = blockIdx.y; i < n; i += gridDim.y) {
-        const float4 *v4 = reinterpret_cast<const float4 *>(V + (size_t)i * ld);
-        float4 *w4 = reinterpret_cast<float4 *>(WH + (size_t)i * ld);
-        for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < m4; q += gridDim.x * blockDim.x) {
-            float4 const a = v4[q];
-            float4 b = w4[q];
-            b.x = __fdividef(a.x, b.x);
-            b.y = __fdividef(a.y, b.y);
-            b.z = __fdividef(a.z, b.z);
-            b.w = __fdividef(a.w, b.w);
-            w4[q] = b;
-        }
-        if (blockIdx.x == 0)
-            for (uint32_t j = 4 * m4 + threadIdx.x; j < m; j += blockDim.x) {
-                size_t const o = (size_t)i * ld + j;
-                WH[o] = __fdividef(V[o], WH[o]);
+#pragma unroll
+    for (int p = 0; p < 8; p++) {
+        uint32_t const i = i0 + (p < 4 ? 0u : 64u) + 4 * ty + (p & 3);
+        if (i >= n) continue;
+#pragma unroll
+        for (int q = 0; q < 8; q += 4) {
+            uint32_t const j = j0 + (q < 4 ? 0u : 32u) + 4 * tx;
+            if (j >= m) continue;
+            size_t const o = (size_t)i * ld + j;
+            float4 const v = __ldcs(reinterpret_cast<const float4 *>(V + o));   // (a float4 from below m lies in the row)
+            float4 const r = make_float4(__fdividef(v.x, acc[p][q]), __fdividef(v.y, acc[p][q + 1]),
+                                         __fdividef(v.z, acc[p][q + 2]), __fdividef(v.w, acc[p][q + 3]));
+            if (j + 4 <= m) {
+                *reinterpret_cast<float4 *>(Q + o) = r;
+            } else {
+                Q[o] = r.x;
+                if (j + 1 < m) Q[o + 1] = r.y;
+                if (j + 2 < m) Q[o + 2] = r.z;
             }
+        }
     }
 }
 
-// Launch shape of k_div for `rows` rows: enough column threads for a row's
-// float4 chunks, rows spread over blockIdx.y up to 64K and ~16 CTAs per SM.
-dim3 div_grid(const nmfb_ctx *ctx, uint32_t rows)
+// Out[o][c] = sum_r Q(o, r) * F[r][c] for r in this CTA's reduction chunk.
+// Q(o, r) = Qm[o][r] when !TRANS, Qm[r][o] when TRANS (Qm has leading dim ldq, a
+// multiple of 32).  F: nred x kp.  Partial results go to part[chunk][o][c] (o <
+// nout, c < kp).  grid: row tiles x chunks x column tiles.
+template <bool TRANS>
+__global__ void __launch_bounds__(128, 4) k_red(const float *Qm, size_t ldq, const float *F, uint32_t nout, uint32_t nred,
+                                                uint32_t kp, uint32_t chunk, float *part, const ConvState *st)
 {
-    uint32_t const gx = (ctx->m / 4 + 255) / 256 > 0 ? (ctx->m / 4 + 255) / 256 : 1;
-    uint32_t gy = (16u * (uint32_t)ctx->sm_count + gx - 1) / gx;
-    if (gy > rows) gy = rows;
-    if (gy > 65535u) gy = 65535u;
-    if (gy == 0) gy = 1;
-    return dim3(gx, gy);
-}
-
-// Out[o][c] = sum_r Q(o, r) * F[r][c] for r in this block's reduction chunk.
-// Q(o, r) = Qm[o][r] when !transQ, Qm[r][o] when transQ (Qm has leading dim ldq).
-// F: nred x kp.  Partial results go to part[chunk][o][c] (o < nout, c < kp).
-// Block: 64 outputs x up to 64 columns per pass; 256 threads, 4 x 4 per thread.
-__global__ void __launch_bounds__(256) k_gemm_red(const float *__restrict__ Qm, size_t ldq, int transQ,
-                                                  const float *__restrict__ F, uint32_t nout, uint32_t nred,
-                                                  uint32_t kp, uint32_t chunk, float *__restrict__ part,
-                                                  const ConvState *st)
-{
+    chain_next();
+    chain_wait();
     if (halted(st)) return;
-    __shared__ float Qs[32][64 + 1];
-    __shared__ float Fs[32][64 + 1];
-    uint32_t const o0 = blockIdx.x * 64;
-    uint32_t const r_begin = blockIdx.y * chunk;
-    uint32_t const r_end = min(nred, r_begin + chunk);
-    uint32_t const osub = threadIdx.x / 16, csub = threadIdx.x % 16;
+    __shared__ __align__(16) Tile s;
+    uint32_t const tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
+    uint32_t const o0 = blockIdx.x * TM, c0 = blockIdx.z * TN;
+    uint32_t const r_begin = blockIdx.y * chunk, r_end = min(nred, r_begin + chunk);
+    float4 ra[4], rb[2];
+    float4 const zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    // staging: TRANS: thread t holds row t / 8 of the 16, outputs 16 (t % 8) ..; else the 16
+    // steps of output t.  F: row t / 8, columns 8 (t % 8) ...
+    auto const load = [&](uint32_t r0) {
+        if (TRANS) {
+            uint32_t const r = r0 + tid / 8, o = o0 + tid % 8 * 16;
+#pragma unroll
+            for (int q = 0; q < 4; q++)   // (a float4 from below nout lies in the row; outputs past nout are not kept)
+                ra[q] = r < r_end && o + 4 * q < nout ? __ldcg(reinterpret_cast<const float4 *>(Qm + (size_t)r * ldq + o) + q)
+                                                      : zero;
+        } else {
+            uint32_t const o = o0 + tid;
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                uint32_t const r = r0 + 4 * q;
+                float4 v = o < nout && r < r_end ? __ldcg(reinterpret_cast<const float4 *>(Qm + (size_t)o * ldq + r)) : zero;
+                if (r + 1 >= r_end) v.y = 0.0f;   // past the reduction: the row's padding holds anything
+                if (r + 2 >= r_end) v.z = 0.0f;
+                if (r + 3 >= r_end) v.w = 0.0f;
+                ra[q] = v;
+            }
+        }
+        uint32_t const r = r0 + tid / 8, c = c0 + tid % 8 * 8;
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            rb[q] = r < r_end && c + 4 * q < kp ? __ldcg(reinterpret_cast<const float4 *>(F + (size_t)r * kp + c) + q) : zero;
+    };
+    auto const store = [&](uint32_t buf) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (TRANS) {
+                *reinterpret_cast<float4 *>(&s.a[buf][tid / 8][tid % 8 * 16 + 4 * q]) = ra[q];
+            } else {
+                s.a[buf][4 * q + 0][tid] = ra[q].x;
+                s.a[buf][4 * q + 1][tid] = ra[q].y;
+                s.a[buf][4 * q + 2][tid] = ra[q].z;
+                s.a[buf][4 * q + 3][tid] = ra[q].w;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; q++) *reinterpret_cast<float4 *>(&s.b[buf][tid / 8][tid % 8 * 8 + 4 * q]) = rb[q];
+    };
+    float acc[8][8] = {};
+    uint32_t const steps = r_end > r_begin ? (r_end - r_begin + TK - 1) / TK : 0;
+    if (steps) {
+        load(r_begin);
+        store(0);
+    }
+    __syncthreads();
+    for (uint32_t t = 0; t < steps; t++) {
+        if (t + 1 < steps) load(r_begin + (t + 1) * TK);
+        tile_fma(s.a[t & 1], s.b[t & 1], tx, ty, acc);
+        if (t + 1 < steps) store((t + 1) & 1);
+        __syncthreads();
+    }
     float *outp = part + (size_t)blockIdx.y * nout * kp;
-    for (uint32_t cg = 0; cg < kp; cg += 64) {
-        uint32_t const kc = min(64u, kp - cg);
-        float acc[4][4] = {};
-        for (uint32_t r0 = r_begin; r0 < r_end; r0 += 32) {
-            for (uint32_t e = threadIdx.x; e < 32 * 64; e += 256) {
-                uint32_t r, o;
-                if (transQ) { r = e / 64; o = e % 64; }  // contiguous along o
-                else { o = e / 32; r = e % 32; }        // contiguous along r
-                uint32_t const gr = r0 + r, go = o0 + o;
-                float q = 0.0f;
-                if (gr < r_end && go < nout)
-                    q = transQ ? Qm[(size_t)gr * ldq + go] : Qm[(size_t)go * ldq + gr];
-                Qs[r][o] = q;
-            }
-            for (uint32_t e = threadIdx.x; e < 32 * 64; e += 256) {
-                uint32_t const r = e / 64, c = e % 64;
-                uint32_t const gr = r0 + r;
-                Fs[r][c] = (gr < r_end && c < kc) ? F[(size_t)gr * kp + cg + c] : 0.0f;
-            }
-            __syncthreads();
-#pragma unroll 8
-            for (uint32_t r = 0; r < 32; r++) {
-                float q[4], f[4];
 #pragma unroll
-                for (int p = 0; p < 4; p++) q[p] = Qs[r][osub * 4 + p];
+    for (int p = 0; p < 8; p++) {
+        uint32_t const o = o0 + (p < 4 ? 0u : 64u) + 4 * ty + (p & 3);
+        if (o >= nout) continue;
 #pragma unroll
-                for (int s = 0; s < 4; s++) f[s] = Fs[r][csub + 16 * s];
-#pragma unroll
-                for (int p = 0; p < 4; p++)
-#pragma unroll
-                    for (int s = 0; s < 4; s++) acc[p][s] = fmaf(q[p], f[s], acc[p][s]);
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int p = 0; p < 4; p++) {
-            uint32_t const o = o0 + osub * 4 + p;
-            if (o >= nout) continue;
-#pragma unroll
-            for (int s = 0; s < 4; s++) {
-                uint32_t const c = csub + 16 * s;
-                if (c < kc) outp[(size_t)o * kp + cg + c] = acc[p][s];
-            }
+        for (int q = 0; q < 8; q += 4) {
+            uint32_t const c = c0 + (q < 4 ? 0u : 32u) + 4 * tx;
+            if (c < kp)
+                *reinterpret_cast<float4 *>(outp + (size_t)o * kp + c) =
+                    make_float4(acc[p][q], acc[p][q + 1], acc[p][q + 2], acc[p][q + 3]);
         }
     }
 }
@@ -171,17 +228,34 @@ struct RedPlan {
     uint32_t nsplit, chunk;
 };
 
+// Splits of the reduction: about eight CTAs per SM, in chunks of whole staging steps.
 RedPlan plan_split(nmfb_ctx *ctx, uint32_t nout, uint32_t nred)
 {
-    uint32_t const oblocks = (nout + 63) / 64;
-    uint32_t want = (8u * (uint32_t)ctx->sm_count + oblocks - 1) / oblocks;   // ~8 CTAs per SM of work
+    uint32_t const tiles = (nout + TM - 1) / TM * ((ctx->k + TN - 1) / TN);
+    uint32_t want = (8u * (uint32_t)ctx->sm_count + tiles - 1) / tiles;
     if (want < 1) want = 1;
     if (want > NMFB_MAX_SPLIT) want = NMFB_MAX_SPLIT;
+    // (the partials of all splits fit the context's buffer)
+    size_t const fit = ctx->part_items / ((size_t)nout * ctx->kp);
+    if (want > fit) want = fit > 0 ? (uint32_t)fit : 1u;
     uint32_t chunk = (nred + want - 1) / want;
-    chunk = ((chunk + 31) / 32) * 32;
-    if (chunk == 0) chunk = 32;
+    chunk = (chunk + TK - 1) / TK * TK;
+    if (chunk == 0) chunk = TK;
     uint32_t const nsplit = (nred + chunk - 1) / chunk;
     return {nsplit, chunk};
+}
+
+int launch_red(nmfb_ctx *ctx, const float *Q, bool trans, const float *F, uint32_t nout, uint32_t nred, uint32_t *nsplit)
+{
+    RedPlan const p = plan_split(ctx, nout, nred);
+    if ((size_t)p.nsplit * nout * ctx->kp > ctx->part_items)
+        return nmfb_fail(ctx, NMFB_EINVAL, "partial buffer too small (%u splits of %u rows)", p.nsplit, nout);
+    dim3 const g((nout + TM - 1) / TM, p.nsplit, (ctx->k + TN - 1) / TN);
+    NMFB_CUDA_TRY(ctx, launch_chained(trans ? k_red<true> : k_red<false>, g, 128, 0, ctx->stream, Q, ctx->ldv, F, nout, nred,
+                                      ctx->kp, p.chunk, ctx->dPart, ctx->dState));
+    NMFB_LAUNCH_CHECK(ctx);
+    *nsplit = p.nsplit;
+    return NMFB_OK;
 }
 
 int plain_half(nmfb_ctx *ctx, bool is_H, int adjust)
@@ -196,44 +270,28 @@ int plain_half(nmfb_ctx *ctx, bool is_H, int adjust)
     int rc = nmfb_prof_begin(ctx, whole);
     if (rc) return rc;
     if ((rc = nmfb_colsum(ctx, Y, yrows, acc, is_H ? 0 : 1))) return rc;
-    // 2. WH = W * H^T (n x m)
-    dim3 g((ctx->m + 63) / 64, (ctx->n + 63) / 64);
-    k_gemm_nt<<<g, 256, 0, ctx->stream>>>(ctx->dW, ctx->dH, ctx->dWH, ctx->n, ctx->m, ctx->kp, ctx->ldv, ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    // 3. WH = V ./ WH
-    k_div<<<div_grid(ctx, ctx->n), 256, 0, ctx->stream>>>(ctx->dV, ctx->dWH, ctx->n, ctx->m, ctx->ldv, ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    // 4. Xaux = Q^T Y (update_H) or Q Y (update_W), split over the reduction.
-    RedPlan const p = plan_split(ctx, xrows, yrows);
-    if ((size_t)p.nsplit * xrows * ctx->kp > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "partial buffer too small (%u splits of %u rows)", p.nsplit, xrows);
-    dim3 rg((xrows + 63) / 64, p.nsplit);
+    // 2. Q = V ./ (W * H^T) (n x m)
+    if ((rc = nmfb_plain_quot(ctx, ctx->dV, ctx->dW, ctx->n, ctx->dWH))) return rc;
+    // 3. Xaux = Q^T Y (update_H) or Q Y (update_W), split over the reduction.
     if ((rc = nmfb_prof_begin(ctx, main))) return rc;
-    k_gemm_red<<<rg, 256, 0, ctx->stream>>>(ctx->dWH, ctx->ldv, is_H ? 1 : 0, Y, xrows, yrows, ctx->kp, p.chunk,
-                                           ctx->dPart, ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
+    uint32_t nsplit = 0;
+    if ((rc = launch_red(ctx, ctx->dWH, is_H, Y, xrows, yrows, &nsplit))) return rc;
     if ((rc = nmfb_prof_end(ctx, main))) return rc;
-    // 5. X = X .* Xaux ./ acc  (+ EPS adjust on test iterations)
-    rc = nmfb_muldiv(ctx, X, xrows, ctx->dPart, p.nsplit, (size_t)xrows * ctx->kp, acc, adjust);
+    // 4. X = X .* Xaux ./ acc  (+ EPS adjust on test iterations)
+    rc = nmfb_muldiv(ctx, X, xrows, ctx->dPart, nsplit, (size_t)xrows * ctx->kp, acc, adjust);
     if (rc) return rc;
     return nmfb_prof_end(ctx, whole);
 }
 
 }  // namespace
 
-// Row-block building blocks for the streamed mode (stream.cu): the same
-// kernels on `rows` rows of W and a rows x ldv block of V / WH.
-int nmfb_plain_wh(nmfb_ctx *ctx, const float *W, uint32_t rows, float *WH)
+// Building blocks, also of the streamed mode (stream.cu): the same kernels on
+// `rows` rows of W and a rows x ldv block of V.
+int nmfb_plain_quot(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, float *Q)
 {
-    dim3 g((ctx->m + 63) / 64, (rows + 63) / 64);
-    k_gemm_nt<<<g, 256, 0, ctx->stream>>>(W, ctx->dH, WH, rows, ctx->m, ctx->kp, ctx->ldv, ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    return NMFB_OK;
-}
-
-int nmfb_plain_div(nmfb_ctx *ctx, const float *V, float *WH, uint32_t rows)
-{
-    k_div<<<div_grid(ctx, rows), 256, 0, ctx->stream>>>(V, WH, rows, ctx->m, ctx->ldv, ctx->dState);
+    dim3 const g((ctx->m + TN - 1) / TN, (rows + TM - 1) / TM);
+    NMFB_CUDA_TRY(ctx, launch_chained(k_quot, g, 128, 0, ctx->stream, V, W, ctx->dH, Q, rows, ctx->m, ctx->kp, ctx->k,
+                                      ctx->ldv, ctx->dState));
     NMFB_LAUNCH_CHECK(ctx);
     return NMFB_OK;
 }
@@ -241,15 +299,7 @@ int nmfb_plain_div(nmfb_ctx *ctx, const float *V, float *WH, uint32_t rows)
 int nmfb_plain_red(nmfb_ctx *ctx, const float *Q, int transQ, const float *F, uint32_t nout, uint32_t nred,
                    uint32_t *nsplit)
 {
-    RedPlan const p = plan_split(ctx, nout, nred);
-    if ((size_t)p.nsplit * nout * ctx->kp > ctx->part_items)
-        return nmfb_fail(ctx, NMFB_EINVAL, "partial buffer too small (%u splits of %u rows)", p.nsplit, nout);
-    dim3 rg((nout + 63) / 64, p.nsplit);
-    k_gemm_red<<<rg, 256, 0, ctx->stream>>>(Q, ctx->ldv, transQ, F, nout, nred, ctx->kp, p.chunk, ctx->dPart,
-                                           ctx->dState);
-    NMFB_LAUNCH_CHECK(ctx);
-    *nsplit = p.nsplit;
-    return NMFB_OK;
+    return launch_red(ctx, Q, transQ != 0, F, nout, nred, nsplit);
 }
 
 int nmfb_plain_update_H(nmfb_ctx *ctx, int adjust) { return plain_half(ctx, true, adjust); }

@@ -142,8 +142,7 @@ int nmfb_objectives_rows(nmfb_ctx *ctx, const float *V, const float *W, uint32_t
 // ---- kernels_plain.cu -----------------------------------------------------
 int nmfb_plain_update_H(nmfb_ctx *ctx, int adjust);
 int nmfb_plain_update_W(nmfb_ctx *ctx, int adjust);
-int nmfb_plain_wh(nmfb_ctx *ctx, const float *W, uint32_t rows, float *WH);
-int nmfb_plain_div(nmfb_ctx *ctx, const float *V, float *WH, uint32_t rows);
+int nmfb_plain_quot(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, float *Q);
 int nmfb_plain_red(nmfb_ctx *ctx, const float *Q, int transQ, const float *F, uint32_t nout, uint32_t nred,
                    uint32_t *nsplit);
 

@@ -202,8 +202,7 @@ int nmfb_stream_update_H(nmfb_ctx *ctx, int adjust)
     if (grid > 8u * (unsigned)ctx->sm_count) grid = 8u * (unsigned)ctx->sm_count;
     rc = for_blocks(ctx, p, [&](uint32_t b, uint32_t i0, uint32_t nb, const float *Vb) -> int {
         const float *Wb = ctx->dW + (size_t)i0 * ctx->kp;
-        int r = nmfb_plain_wh(ctx, Wb, nb, p->dWHb);
-        if (!r) r = nmfb_plain_div(ctx, Vb, p->dWHb, nb);
+        int r = nmfb_plain_quot(ctx, Vb, Wb, nb, p->dWHb);
         uint32_t ns = 0;
         if (!r) r = nmfb_plain_red(ctx, p->dWHb, 1, Wb, ctx->m, nb, &ns);
         if (r) return r;
@@ -230,15 +229,13 @@ int nmfb_stream_update_W(nmfb_ctx *ctx, int adjust)
     p->haux_ready = 0;
     rc = for_blocks(ctx, p, [&](uint32_t b, uint32_t i0, uint32_t nb, const float *Vb) -> int {
         float *Wb = ctx->dW + (size_t)i0 * ctx->kp;
-        int r = nmfb_plain_wh(ctx, Wb, nb, p->dWHb);
-        if (!r) r = nmfb_plain_div(ctx, Vb, p->dWHb, nb);
+        int r = nmfb_plain_quot(ctx, Vb, Wb, nb, p->dWHb);
         uint32_t ns = 0;
         if (!r) r = nmfb_plain_red(ctx, p->dWHb, 0, ctx->dH, nb, ctx->m, &ns);
         if (!r) r = nmfb_muldiv(ctx, Wb, nb, ctx->dPart, ns, (size_t)nb * ctx->kp, ctx->dAccH, adjust);
         if (r || !fold) return r;
         // next update_H's term of this block, with the new W rows
-        r = nmfb_plain_wh(ctx, Wb, nb, p->dWHb);
-        if (!r) r = nmfb_plain_div(ctx, Vb, p->dWHb, nb);
+        r = nmfb_plain_quot(ctx, Vb, Wb, nb, p->dWHb);
         if (!r) r = nmfb_plain_red(ctx, p->dWHb, 1, Wb, ctx->m, nb, &ns);
         if (r) return r;
         k_accum<<<grid, 256, 0, ctx->stream>>>(p->dAux, ctx->dPart, ns, total, total, b == 0, ctx->dState);
