@@ -88,6 +88,8 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
     if (a.st && *(volatile const uint32_t *)&a.st->converged) return;
     __shared__ double ws[NW * KP];
     __shared__ float sx[KP * 33];                // x of one 32-row set, column-major (padded)
+    __shared__ float sacc[KP];                   // accY, once per CTA: it is read through L2, where one line
+                                                 // asked for by every thread is a hot spot (53 us at 50000 x 64)
     uint32_t const tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
     uint32_t const row = tid / TPR, c0 = (tid % TPR) * 4;
     uint32_t const blk = blockIdx.x;
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
     static_assert(BO % ((int)FIN_RB * RPT) == 0, "row sets of a CTA in one row block");
     uint32_t const ob = blk * (FIN_RB * RPT) / BO;
     bool const update = a.part != nullptr;
+    if (update && tid < (uint32_t)KP) sacc[tid] = __ldcg(a.accY + tid);
     uint32_t const nslot = update ? a.ts.nslot(ob) : 0;
     for (uint32_t q = 0; q < nslot; q += QB) {
         float4 v[RPT][QB];
@@ -133,6 +136,7 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
                 }
     }
     double csum[4] = {0.0, 0.0, 0.0, 0.0};   // this thread's rows of its columns, in row-set order
+    __syncthreads();   // sacc
 #pragma unroll
     for (int r = 0; r < RPT; r++) {
         if (in[r]) {
@@ -142,7 +146,7 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
                 uint32_t const cc = c0 + i;
                 float v = 0.0f;
                 if (cc < a.k) {
-                    v = update ? __fdiv_rn(xs[i] * x[r][i], __ldcg(a.accY + cc)) : xs[i];
+                    v = update ? __fdiv_rn(xs[i] * x[r][i], sacc[cc]) : xs[i];
                     if (a.adjust) v = fmaxf(v, FLT_MIN);
                 }
                 x[r][i] = v;
