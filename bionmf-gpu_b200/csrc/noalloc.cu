@@ -80,6 +80,13 @@ __device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c)
     return d;
 }
 
+__device__ __forceinline__ pair_t add2(pair_t a, pair_t b)
+{
+    pair_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 // CTA (x, s) covers samples j in [NT x, NT x + NT) and rows i of split s.
 // part[s][j][c] = sum_{i in split s} V[i][j] / (W_i . H_j) * W[i][c];
 // CTAs with x == 0 also write colpart[s][c] = sum_{i in split s} W[i][c] (FP64).
@@ -94,6 +101,7 @@ __global__ void __launch_bounds__(NA_THREADS, KB <= 32 ? 4 : 2)
                   float *__restrict__ part, double *__restrict__ colpart)
 {
     static_assert(KB % 4 == 0, "rows of W as 16-byte vectors");
+    constexpr bool TILE = KB <= 32;
     constexpr int K2 = KB / 2, PER = NA_WT * KB / NA_THREADS;   // floats of a W tile per thread
     constexpr int SEG = NA_THREADS / KB;                        // row lanes of the column sums
     __shared__ __align__(16) float sW[2][NA_WT][KB];
@@ -141,6 +149,12 @@ __global__ void __launch_bounds__(NA_THREADS, KB <= 32 ? 4 : 2)
         store_w(b);
         __syncthreads();   // (a buffer is rewritten two tiles on: past this barrier of the next tile)
         if (i0 + NA_WT < r1) load_w(i0 + NA_WT);
+        // up to rank 32 a tile is summed by itself first (shorter FP32 chains); above, the
+        // sums fill the registers and the splits are shorter instead
+        pair_t tl[TILE ? K2 : 1];
+        if (TILE)
+#pragma unroll
+            for (int c = 0; c < K2; c++) tl[c] = 0;
         if (colsum_cta && seg < (uint32_t)SEG)
             for (uint32_t r = seg; r < rows; r += SEG) cs += (double)sW[b][r][cc];
         for (uint32_t g = 0; g < rows; g += NA_VG) {
@@ -164,9 +178,17 @@ __global__ void __launch_bounds__(NA_THREADS, KB <= 32 ? 4 : 2)
                 float const q = v[r] / (wh.x + wh.y);
                 pair_t const q2 = pair_of(q, q);
 #pragma unroll
-                for (int c = 0; c < K2; c++) acc[c] = fma2(q2, w[c], acc[c]);
+                for (int c = 0; c < K2; c++) {
+                    if (TILE)
+                        tl[c] = fma2(q2, w[c], tl[c]);
+                    else
+                        acc[c] = fma2(q2, w[c], acc[c]);
+                }
             }
         }
+        if (TILE)
+#pragma unroll
+            for (int c = 0; c < K2; c++) acc[c] = add2(acc[c], tl[c]);
     }
     if (active) {
         float *dst = part + ((size_t)s * m + j) * k;
@@ -188,40 +210,54 @@ __global__ void __launch_bounds__(NA_THREADS, KB <= 32 ? 4 : 2)
     }
 }
 
-// H[j][c] = (H[j][c] * sum_s part[s][j][c]) / (float)sum_s colpart[s][c], the
-// partials in split order; the column sums once per CTA, by eight lanes a column
-// (splits l, l + 8, ... in order, then a shuffle tree).
+// H[j][c] = (H[j][c] * sum_s part[s][j][c]) / (float)sum_s colpart[s][c].  A CTA
+// takes NA_FIN / lanes entries; group l of its threads adds an entry's splits l, l +
+// lanes, ... eight loads at a time, then the groups are added in order.  Latency-
+// bound: `lanes` (1, 2, 4 or 8) grows with the splits.  The column sums once per CTA,
+// by eight lanes a column (splits l, l + 8, ... in order, then a shuffle tree).
 __global__ void __launch_bounds__(NA_FIN) k_na_finish(float *__restrict__ H, size_t ldh, uint32_t m, uint32_t k,
-                                                      uint32_t nsplit, const float *part, const double *colpart)
+                                                      uint32_t nsplit, uint32_t lanes, const float *part,
+                                                      const double *colpart)
 {
     nmfb_tc::chain_wait();
     __shared__ float sA[NA_KMAX];
+    __shared__ float sS[NA_FIN];
     for (uint32_t c0 = 0; c0 < k; c0 += NA_FIN / 8) {
         uint32_t const c = c0 + threadIdx.x / 8;
         double a = 0.0;
         if (c < k)
-            for (uint32_t q = threadIdx.x % 8; q < nsplit; q += 8) a += __ldcg(colpart + (size_t)q * k + c);
+            for (uint32_t q = threadIdx.x % 8; q < nsplit; q += 64) {
+                double v[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++) v[i] = q + 8 * i < nsplit ? __ldcg(colpart + (size_t)(q + 8 * i) * k + c) : 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) a += v[i];
+            }
 #pragma unroll
         for (int off = 4; off > 0; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
         if (c < k && threadIdx.x % 8 == 0) sA[c] = (float)a;
     }
-    __syncthreads();
     size_t const total = (size_t)m * k;
-    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (size_t)gridDim.x * blockDim.x) {
-        uint32_t const j = (uint32_t)(idx / k), c = (uint32_t)(idx % k);
-        float *hp = H + (size_t)j * ldh + c;
-        float const h = *hp;
+    uint32_t const per = NA_FIN / lanes, e = threadIdx.x % per, l = threadIdx.x / per;
+    for (size_t i0 = (size_t)blockIdx.x * per; i0 < total; i0 += (size_t)gridDim.x * per) {
+        size_t const idx = i0 + e;
         float s = 0.0f;
-        for (uint32_t q = 0; q < nsplit; q += 8) {
-            float p[8];
+        if (idx < total)
+            for (uint32_t q = l; q < nsplit; q += 8 * lanes) {
+                float p[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) p[i] = q + i < nsplit ? __ldcg(part + (size_t)(q + i) * total + idx) : 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (q + i < nsplit) s += p[i];
+                for (int i = 0; i < 8; i++) p[i] = q + i * lanes < nsplit ? __ldcg(part + (size_t)(q + i * lanes) * total + idx) : 0.0f;
+                s += ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+            }
+        __syncthreads();   // sA (first pass); the previous pass's readers of sS
+        sS[threadIdx.x] = s;
+        __syncthreads();
+        if (l == 0 && idx < total) {
+            for (uint32_t g = 1; g < lanes; g++) s += sS[g * per + e];
+            uint32_t const j = (uint32_t)(idx / k), c = (uint32_t)(idx % k);
+            float *hp = H + (size_t)j * ldh + c;
+            *hp = __fdiv_rn(*hp * s, sA[c]);
         }
-        *hp = __fdiv_rn(h * s, sA[c]);
     }
 }
 
@@ -317,13 +353,15 @@ extern "C" int nmfb_update_H_noalloc(const float *V, size_t ldv, const float *W,
     float *part = reinterpret_cast<float *>(slot.scratch + NA_COLPART_BYTES);
     cudaStream_t const st = static_cast<cudaStream_t>(stream);
 
-    // Splits over the rows of V: four CTAs per SM in one wave, limited by the
-    // scratch (nsplit * m * k floats, nsplit * k column sums) and by n.
+    // Splits over the rows of V: four CTAs per SM in one wave (above rank 32, where two
+    // fit, twice as many shorter ones), limited by the scratch (nsplit * m * k floats,
+    // nsplit * k column sums) and by n.
     uint32_t const xblocks = (m + NA_THREADS - 1) / NA_THREADS;
-    uint64_t want = (uint64_t)4 * slot.sm_count / xblocks;
+    uint64_t want = (uint64_t)(k <= 32 ? 4 : 8) * slot.sm_count / xblocks;
     uint64_t const fit = (uint64_t)NA_PART_FLOATS / ((uint64_t)m * k);
     if (want > fit) want = fit;
     if (want > NA_COLPARTS / k) want = NA_COLPARTS / k;
+    if (want > n / 16) want = n / 16;   // (a split of fewer rows costs k_na_finish more than it saves here)
     if (want > n) want = n;
     if (want < 1) want = 1;
     uint32_t const rps = (uint32_t)((n + want - 1) / want);
@@ -342,10 +380,11 @@ extern "C" int nmfb_update_H_noalloc(const float *V, size_t ldv, const float *W,
     if (e != cudaSuccess) return NMFB_ECUDA;
 
     uint64_t const total = (uint64_t)m * k;
-    uint64_t blocks = (total + NA_FIN - 1) / NA_FIN;
+    uint32_t const lanes = nsplit >= 48 ? 8u : nsplit >= 24 ? 4u : nsplit >= 12 ? 2u : 1u;
+    uint64_t blocks = (total * lanes + NA_FIN - 1) / NA_FIN;
     uint64_t const cap = (uint64_t)8 * slot.sm_count;
     if (blocks > cap) blocks = cap;
-    if (nmfb_tc::launch_chained(k_na_finish, dim3((unsigned)blocks), NA_FIN, 0, st, H, ldh, m, k, nsplit,
+    if (nmfb_tc::launch_chained(k_na_finish, dim3((unsigned)blocks), NA_FIN, 0, st, H, ldh, m, k, nsplit, lanes,
                                 (const float *)part, (const double *)colpart) != cudaSuccess) {
         cudaGetLastError();
         return NMFB_ECUDA;
