@@ -280,6 +280,7 @@ int do_update_H(nmfb_ctx *ctx, int adjust)
     if (ctx->splan) return nmfb_stream_update_H(ctx, adjust);
     if (ctx->arm == NMFB_ARM_PLAIN) return nmfb_plain_update_H(ctx, adjust);
     if (ctx->arm >= NMFB_ARM_BF16) return nmfb_bf16_update_H(ctx, adjust);
+    if (nmfb_small_fits(ctx)) return nmfb_small_update_H(ctx, adjust);
     return nmfb_fused_update_H(ctx, adjust);
 }
 
@@ -288,6 +289,7 @@ int do_update_W(nmfb_ctx *ctx, int adjust)
     if (ctx->splan) return nmfb_stream_update_W(ctx, adjust);
     if (ctx->arm == NMFB_ARM_PLAIN) return nmfb_plain_update_W(ctx, adjust);
     if (ctx->arm >= NMFB_ARM_BF16) return nmfb_bf16_update_W(ctx, adjust);
+    if (nmfb_small_fits(ctx)) return nmfb_small_update_W(ctx, adjust);
     return nmfb_fused_update_W(ctx, adjust);
 }
 
@@ -608,7 +610,9 @@ static int launch_block(nmfb_ctx *ctx, uint32_t J)
     static int const use_graphs = getenv("NMFB_NO_GRAPHS") == nullptr;
     if (!use_graphs || ctx->prof_on || ctx->splan) return enqueue_block(ctx, J);
     // the graph holds no preparation launch: make W's split copies current first
-    int const rc0 = (ctx->arm == NMFB_ARM_FUSED || ctx->arm == NMFB_ARM_FUSED_TF32) ? nmfb_fused_ready_W(ctx)
+    bool const small = nmfb_small_fits(ctx);
+    int const rc0 = small                                                              ? NMFB_OK
+                    : (ctx->arm == NMFB_ARM_FUSED || ctx->arm == NMFB_ARM_FUSED_TF32) ? nmfb_fused_ready_W(ctx)
                     : ctx->arm >= NMFB_ARM_BF16                                    ? nmfb_bf16_ready_W(ctx)
                                                                                    : NMFB_OK;
     if (rc0) return rc0;
@@ -642,7 +646,7 @@ static int launch_block(nmfb_ctx *ctx, uint32_t J)
     }
     NMFB_CUDA_TRY(ctx, cudaGraphLaunch(ctx->blk_exec, ctx->stream));
     ctx->launches += ctx->blk_kernels;
-    ctx->fz_ok[0] = 1;   // the block ends with update_W's epilogue and the test's adjust of H
+    ctx->fz_ok[0] = !small;   // the block ends with update_W's epilogue and the test's adjust of H
     ctx->fz_ok[1] = 0;
     return NMFB_OK;
 }

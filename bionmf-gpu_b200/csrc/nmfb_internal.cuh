@@ -59,10 +59,11 @@ struct nmfb_ctx {
     // Fused arms: the split copies and column sums of W ([0]) and of H ([1]) match
     // the factor (written by the previous half-iteration's epilogue).  Trusted
     // only inside one nmfb_run or step call; every entry point starts from 0.
+    // (Small matrices: [0] = the next update_H's sums are there, see small.cu.)
     int fz_ok[2];
-    // Inside nmfb_run: the blockwise mode may fold the next update_H's pass over
-    // V into update_W's pass (the factors change only through the run's own
-    // updates there).
+    // Inside nmfb_run: the blockwise mode and the small matrices' kernels may fold
+    // the next update_H's pass over V into update_W's pass (the factors change only
+    // through the run's own updates there).
     int in_run;
 
     uint64_t launches;
@@ -170,6 +171,11 @@ int nmfb_bf16_release(nmfb_ctx *ctx);
 int nmfb_bf16_update_H(nmfb_ctx *ctx, int adjust);
 int nmfb_bf16_update_W(nmfb_ctx *ctx, int adjust);
 int nmfb_bf16_ready_W(nmfb_ctx *ctx);
+
+// ---- small.cu -------------------------------------------------------------
+bool nmfb_small_fits(const nmfb_ctx *ctx);
+int nmfb_small_update_H(nmfb_ctx *ctx, int adjust);
+int nmfb_small_update_W(nmfb_ctx *ctx, int adjust);
 
 // ---- consensus.cu ---------------------------------------------------------
 size_t nmfb_summary_doubles(uint32_t m);
