@@ -16,7 +16,8 @@
 //   [0, 32 KiB)            colpart: nsplit x k doubles (at most 4096), per-split
 //                          column sums of W
 //   [32 KiB, 16 MiB)       part:    nsplit x m x k floats, per-split partial
-//                          sums of Q^T W (Q = V ./ (W H^T))
+//                          sums of Q^T W (Q = V ./ (W H^T)); behind them colpart,
+//                          where it does not fit the first 32 KiB
 // Every scratch word a call reads is written earlier in the same call (each
 // (split, row, factor) slot by exactly one CTA), so nothing carries over from
 // the previous call and nothing has to be cleared.  All calls share the one
@@ -360,12 +361,34 @@ extern "C" int nmfb_update_H_noalloc(const float *V, size_t ldv, const float *W,
     uint64_t want = (uint64_t)(k <= 32 ? 4 : 8) * slot.sm_count / xblocks;
     uint64_t const fit = (uint64_t)NA_PART_FLOATS / ((uint64_t)m * k);
     if (want > fit) want = fit;
-    if (want > NA_COLPARTS / k) want = NA_COLPARTS / k;
+    // Column sums that do not fit their own part go behind the partials: at most two CTAs
+    // per SM then, and at least k rows to a split, or the partials cost more than V (of
+    // 263 splits at 4209 x 415 k = 35: 68 us, of 120 41).
+    uint64_t const own = NA_COLPARTS / k;
+    if (want > own) {
+        uint64_t more = (NA_PART_FLOATS * sizeof(float) - 8) / ((uint64_t)m * k * sizeof(float) + k * sizeof(double));
+        if (more > 2u * slot.sm_count) more = 2u * slot.sm_count;
+        if (more > n / k) more = n / k;
+        if (want > more) want = more > own ? more : own;
+    }
     if (want > n / 16) want = n / 16;   // (a split of fewer rows costs k_na_finish more than it saves here)
+    // Whole waves where the last one is nearly empty (6182 x 812 k = 59: 609 CTAs 109 us, 588
+    // 102), and as few as give a split 4 k rows: below that the partials' traffic and their
+    // addition cost more than a wave's balance (one wave: 76 us; 585 x 1766 k = 62 71 -> 37).
+    // Longer splits keep their part of a wave: 50000 x 2000 k = 40 742 us in 2.8 waves, 959 in 2.
+    uint64_t const slots = (uint64_t)(k <= 32 ? 4 : 2) * slot.sm_count, ctas = want * xblocks;
+    if (ctas > slots && (ctas % slots < slots / 4 || n / want < 4 * k)) {
+        uint64_t waves = ctas / slots;
+        while (waves > 1 && (uint64_t)n * xblocks < 4 * k * waves * slots) waves--;
+        want = waves * slots / xblocks;
+    }
     if (want > n) want = n;
     if (want < 1) want = 1;
     uint32_t const rps = (uint32_t)((n + want - 1) / want);
     uint32_t const nsplit = (uint32_t)((n + rps - 1) / rps);
+
+    if ((uint64_t)nsplit * k > NA_COLPARTS)
+        colpart = reinterpret_cast<double *>(part + ((size_t)nsplit * m * k + 1) / 2 * 2);
 
     dim3 const grid(xblocks, nsplit);
     cudaError_t e;
