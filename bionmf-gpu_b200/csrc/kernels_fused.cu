@@ -26,8 +26,8 @@
 //              the tensor core's FP32 sums short) and writes the split's
 //              partial; k_finish (one CTA per 32 rows) sums the splits, applies
 //              X = X .* Xaux ./ colsum(Y) (and the EPS adjust when asked), and
-//              writes X's split copies and column sums for the next
-//              half-iteration: two launches per half-iteration.
+//              writes X's split copies for the next half-iteration, whose V producers
+//              sum its columns: two launches per half-iteration.
 //
 // Precision of the two contractions: x y = xh yh + xh yl + xl y with xh, yh
 // TF32.  The large term xh yh (and, in MMA2, rh yl) is an exact TF32 product
@@ -63,14 +63,6 @@ using nmfb::ConvState;
 using namespace nmfb_tc;
 
 namespace {
-
-// Two floats to a BF16 pair (round to nearest even), `first` in the low half.
-__device__ __forceinline__ uint32_t bf16x2_rn(float first, float second)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(second), "f"(first));
-    return r;
-}
 
 // Swizzle of a K-major operand whose rows are `bytes` long: the UMMA layout code
 // and the tensor-map mode (rows of 32 / 64 / 128 bytes).
@@ -550,7 +542,7 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                 }
                 if (NTERMS == 3) {
 #pragma unroll
-                    for (int j = 0; j < 8; j++) pl[j] = bf16x2_rn(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+                    for (int j = 0; j < 8; j++) pl[j] = fin_bf16x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
                 }
                 if (ch == CW / 16 - 1) DBG_PH(5, t);
                 // this team's bf16(Rl) buffer: MMA2 of the team's previous tile has read it
@@ -631,11 +623,11 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                     }
                 } else if (NTERMS == 3) {
 #pragma unroll
-                    for (int c = 0; c < 8; c++) b8[c] = bf16x2_rn(tf32_rna(x[2 * c]), tf32_rna(x[2 * c + 1]));
+                    for (int c = 0; c < 8; c++) b8[c] = fin_bf16x2(tf32_rna(x[2 * c]), tf32_rna(x[2 * c + 1]));
                     tmem_st8(xc + KP + c0 / 2, b8);
 #pragma unroll
                     for (int c = 0; c < 8; c++)
-                        b8[c] = bf16x2_rn(x[2 * c] - tf32_rna(x[2 * c]), x[2 * c + 1] - tf32_rna(x[2 * c + 1]));
+                        b8[c] = fin_bf16x2(x[2 * c] - tf32_rna(x[2 * c]), x[2 * c + 1] - tf32_rna(x[2 * c + 1]));
                     tmem_st8(xc + KP + KP / 2 + c0 / 2, b8);
                 }
             }
