@@ -90,13 +90,17 @@ struct GeoB {
     static constexpr int Y1STAGE = (MODE >= 1 ? 2 : 1) * YBYTES;   // Yh (| Yl)
     static constexpr int Y2STAGE = YTROWS * 128;            // Y^T
     static constexpr int VBYTES = BO * BR * 4;
-    static constexpr int Y1ST = 3, Y2ST = 2;
+    static constexpr int Y1ST = (KP == 64 && MODE == 2) ? 2 : 3, Y2ST = 2;   // (2: room for a fourth V stage)
     static constexpr uint32_t NDB = 4;                      // D buffers in TMEM; R takes D's place
     static constexpr int FIXED = 1024 + 512;
     static constexpr int XALL = (MODE >= 1 ? 2 : 1) * XBYTES, YALL = Y1ST * Y1STAGE + Y2ST * Y2STAGE;
     static constexpr int VAVAIL = (SMEM_LIMIT - FIXED - XALL - YALL) / VBYTES;
     static constexpr int VST = VAVAIL > 6 ? 6 : VAVAIL;
     static_assert(VST >= 3, "shared-memory ring too small");
+    // A team takes every other tile, so with an odd ring its uses of a V stage are two phases
+    // apart and their parities the same: waiting for tile t it must not meet the stage before
+    // tile t - VST (the other team's) has landed in it. D(t) is there only once R(t - NDB) was.
+    static_assert(VST % 2 == 0 || VST >= (int)NDB, "vfull's parity would be ambiguous");
     static constexpr int SMEM = FIXED + XALL + YALL + VST * VBYTES;
     static constexpr int NR = (KP == 64) ? 8 : 16;          // R warps
     static constexpr int NA = (KP == 64) ? 2 : 1;           // accumulator warps: sets of four, KP / NA columns each

@@ -134,6 +134,9 @@ struct Geo {
     static constexpr uint32_t ACC = 2 * KP;                // TMEM columns of one per-tile accumulator
     static constexpr uint32_t NACC = (KP == 64) ? 1 : 2;   // accumulators
     static constexpr uint32_t NDB = (KP == 16) ? 4 : 3;    // D buffers (MMA1 runs NDB tiles ahead)
+    // (a team takes every other tile: with an odd ring its uses of a V stage are two phases apart,
+    // and D(t) has to imply that tile t - VST, the other team's, has landed)
+    static_assert(VST % 2 == 0 || VST >= (int)NDB, "vfull's parity would be ambiguous");
     static constexpr uint32_t DA0 = NACC * ACC;            // D[b] (then Rh[b]) at DA0 + b BR
     static constexpr uint32_t NRL = (KP == 16) ? NDB : 2;  // bf16(Rl) buffers (2: one per R team)
     static_assert(NRL == NDB || (NRL == 2 && Y2ST == 2), "the R teams wait on y2empty for their Rl buffer");

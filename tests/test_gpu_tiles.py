@@ -51,3 +51,26 @@ def test_update_against_fp64(pkg, arm, n, m, k, sms):
             e.update_W()
             want = _updates(V.T, H1, W)
             assert np.abs(e.W / want - 1).max() <= TOL[arm]
+
+
+@pytest.mark.parametrize("arm,k", [("bf16x3", 40), ("bf16x3", 32), ("split_bf16", 64), ("fused", 50), ("fused", 20), ("bf16", 64)])
+def test_long_runs_end_alike(pkg, arm, k):
+    """Many tiles per CTA with loads that land out of order (V larger than L2): the R
+    teams' uses of a V stage must not run into one another, run after run."""
+    import torch
+
+    n, m = 30001, 3001
+    g = torch.Generator(device="cuda").manual_seed(k)
+    V = torch.poisson(torch.full((n, m), 6.0, device="cuda"), generator=g)
+    torch.cuda.synchronize()
+    rng = np.random.default_rng(k)
+    W, H = (rng.random((r, k), np.float32) + np.float32(0.05) for r in (n, m))
+    with pkg.NMF(n, m, k, arm=arm) as e:
+        e.set_V_device(V.data_ptr(), m)
+        first = None
+        for _ in range(8):
+            e.set_WH(W, H)
+            assert e.run(40, 10, 10 ** 6) == (40, False)
+            got = e.W, e.H
+            first = first or got
+            assert all(np.array_equal(a, b) for a, b in zip(got, first))
