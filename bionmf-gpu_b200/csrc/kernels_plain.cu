@@ -27,6 +27,7 @@ __device__ __forceinline__ bool halted(const ConvState *st) { return st && *(vol
 // FMAs), 16 steps of the reduction staged at a time, the next 16 in registers
 // meanwhile.
 constexpr int TM = 128, TN = 64, TK = 16;
+constexpr uint32_t RED_CHAIN = 512;   // longest FP32 chain of k_red, in steps of the reduction
 
 struct Tile {
     float a[2][TK][TM + 4];
@@ -142,9 +143,14 @@ __global__ void __launch_bounds__(128, 4) k_quot(const float *__restrict__ V, co
 // Q(o, r) = Qm[o][r] when !TRANS, Qm[r][o] when TRANS (Qm has leading dim ldq, a
 // multiple of 32).  F: nred x kp.  Partial results go to part[chunk][o][c] (o <
 // nout, c < kp).  grid: row tiles x chunks x column tiles.
-template <bool TRANS>
+// A chunk longer than `piece` (LONG) is summed piece by piece, each added to the CTA's
+// own partial (the registers are full, and the partial lies in L2): FP32 chains of at most
+// RED_CHAIN terms.  In one chain, update_W at 60000 x 5000 k = 256 (5000 terms) was off by
+// 17 * 2^-24 rms, now 2; the run takes 164 ms for 10 iterations, with half the splits and
+// long chains 172.
+template <bool TRANS, bool LONG>
 __global__ void __launch_bounds__(128, 4) k_red(const float *Qm, size_t ldq, const float *F, uint32_t nout, uint32_t nred,
-                                                uint32_t kp, uint32_t chunk, float *part, const ConvState *st)
+                                                uint32_t kp, uint32_t chunk, uint32_t piece, float *part, const ConvState *st)
 {
     chain_next();
     chain_wait();
@@ -203,36 +209,56 @@ __global__ void __launch_bounds__(128, 4) k_red(const float *Qm, size_t ldq, con
         store(0);
     }
     __syncthreads();
+    float *const outp = part + (size_t)blockIdx.y * nout * kp;
+    auto const put = [&](bool add) {   // acc to the partial, or added to it
+#pragma unroll
+        for (int p = 0; p < 8; p++) {
+            uint32_t const o = o0 + (p < 4 ? 0u : 64u) + 4 * ty + (p & 3);
+            if (o >= nout) continue;
+#pragma unroll
+            for (int q = 0; q < 8; q += 4) {
+                uint32_t const c = c0 + (q < 4 ? 0u : 32u) + 4 * tx;
+                if (c >= kp) continue;
+                float4 *const d = reinterpret_cast<float4 *>(outp + (size_t)o * kp + c);
+                float4 x = make_float4(acc[p][q], acc[p][q + 1], acc[p][q + 2], acc[p][q + 3]);
+                if (add) {
+                    float4 const y = *d;
+                    x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+                }
+                *d = x;
+            }
+        }
+    };
+    uint32_t done = 0;   // steps already in the partial (LONG)
     for (uint32_t t = 0; t < steps; t++) {
+        if (LONG && t - done == piece / TK) {
+            put(done > 0);
+            done = t;
+#pragma unroll
+            for (int p = 0; p < 8; p++)
+#pragma unroll
+                for (int q = 0; q < 8; q++) acc[p][q] = 0.0f;
+        }
         if (t + 1 < steps) load(r_begin + (t + 1) * TK);
         tile_fma(s.a[t & 1], s.b[t & 1], tx, ty, acc);
         if (t + 1 < steps) store((t + 1) & 1);
         __syncthreads();
     }
-    float *outp = part + (size_t)blockIdx.y * nout * kp;
-#pragma unroll
-    for (int p = 0; p < 8; p++) {
-        uint32_t const o = o0 + (p < 4 ? 0u : 64u) + 4 * ty + (p & 3);
-        if (o >= nout) continue;
-#pragma unroll
-        for (int q = 0; q < 8; q += 4) {
-            uint32_t const c = c0 + (q < 4 ? 0u : 32u) + 4 * tx;
-            if (c < kp)
-                *reinterpret_cast<float4 *>(outp + (size_t)o * kp + c) =
-                    make_float4(acc[p][q], acc[p][q + 1], acc[p][q + 2], acc[p][q + 3]);
-        }
-    }
+    put(LONG && done > 0);
 }
 
 struct RedPlan {
-    uint32_t nsplit, chunk;
+    uint32_t nsplit, chunk, piece;
 };
 
-// Splits of the reduction: about eight CTAs per SM, in chunks of whole staging steps.
+// Splits of the reduction: about eight CTAs per SM (above rank 128 more, or the chains of
+// additions get longer with the rank), none longer than RED_CHAIN where the partials
+// have room, in chunks of whole staging steps.
 RedPlan plan_split(nmfb_ctx *ctx, uint32_t nout, uint32_t nred)
 {
-    uint32_t const tiles = (nout + TM - 1) / TM * ((ctx->k + TN - 1) / TN);
+    uint32_t const ctiles = (ctx->k + TN - 1) / TN, tiles = (nout + TM - 1) / TM * (ctiles < 2 ? ctiles : 2);
     uint32_t want = (8u * (uint32_t)ctx->sm_count + tiles - 1) / tiles;
+    if (want < (nred + RED_CHAIN - 1) / RED_CHAIN) want = (nred + RED_CHAIN - 1) / RED_CHAIN;
     if (want < 1) want = 1;
     if (want > NMFB_MAX_SPLIT) want = NMFB_MAX_SPLIT;
     // (the partials of all splits fit the context's buffer)
@@ -242,7 +268,9 @@ RedPlan plan_split(nmfb_ctx *ctx, uint32_t nout, uint32_t nred)
     chunk = (chunk + TK - 1) / TK * TK;
     if (chunk == 0) chunk = TK;
     uint32_t const nsplit = (nred + chunk - 1) / chunk;
-    return {nsplit, chunk};
+    uint32_t const pieces = (chunk + RED_CHAIN - 1) / RED_CHAIN;   // of equal length
+    uint32_t const piece = ((chunk + pieces - 1) / pieces + TK - 1) / TK * TK;
+    return {nsplit, chunk, piece};
 }
 
 int launch_red(nmfb_ctx *ctx, const float *Q, bool trans, const float *F, uint32_t nout, uint32_t nred, uint32_t *nsplit)
@@ -251,8 +279,10 @@ int launch_red(nmfb_ctx *ctx, const float *Q, bool trans, const float *F, uint32
     if ((size_t)p.nsplit * nout * ctx->kp > ctx->part_items)
         return nmfb_fail(ctx, NMFB_EINVAL, "partial buffer too small (%u splits of %u rows)", p.nsplit, nout);
     dim3 const g((nout + TM - 1) / TM, p.nsplit, (ctx->k + TN - 1) / TN);
-    NMFB_CUDA_TRY(ctx, launch_chained(trans ? k_red<true> : k_red<false>, g, 128, 0, ctx->stream, Q, ctx->ldv, F, nout, nred,
-                                      ctx->kp, p.chunk, ctx->dPart, ctx->dState));
+    auto const kern = p.chunk > p.piece ? (trans ? k_red<true, true> : k_red<false, true>)
+                                          : (trans ? k_red<true, false> : k_red<false, false>);
+    NMFB_CUDA_TRY(ctx, launch_chained(kern, g, 128, 0, ctx->stream, Q, ctx->ldv, F, nout, nred, ctx->kp, p.chunk, p.piece, ctx->dPart,
+                                      ctx->dState));
     NMFB_LAUNCH_CHECK(ctx);
     *nsplit = p.nsplit;
     return NMFB_OK;
