@@ -103,8 +103,8 @@ __global__ void __launch_bounds__(CS_NT) k_colsum(const float *__restrict__ X, u
 //                   src/GPU_kernels.cu:2013-2019: product first, then the division),
 //                   followed by the EPS adjust when `adjust` is set;
 //   mode FU_ADJUST: v = fmaxf(X[r][c], FLT_MIN)                   (matrix_adjust).
-// Padding columns c >= k are kept at 0.  The split partials are summed in
-// split order, so the result does not depend on scheduling.
+// Padding columns c >= k are kept at 0.  The split partials are summed in a
+// fixed order (eight at a time), so the result does not depend on scheduling.
 enum { FU_MULDIV = 1, FU_ADJUST = 2 };
 
 __global__ void __launch_bounds__(256) k_factor(int mode, float *__restrict__ X, uint32_t rows, uint32_t kp, uint32_t k,
@@ -120,14 +120,7 @@ __global__ void __launch_bounds__(256) k_factor(int mode, float *__restrict__ X,
         if (c < k) {
             if (mode == FU_MULDIV) {
                 float s = 0.0f;
-                for (uint32_t q = 0; q < nsplit; q += 8) {   // eight splits' loads in flight, added in split order
-                    float p[8];
-#pragma unroll
-                    for (int i = 0; i < 8; i++) p[i] = q + i < nsplit ? part[(q + i) * split_stride + idx] : 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 8; i++)
-                        if (q + i < nsplit) s += p[i];
-                }
+                for (uint32_t q = 0; q < nsplit; q += 8) s += nmfb_add8(part + idx, split_stride, q, nsplit);
                 v = __fdiv_rn(X[idx] * s, acc[c]);
                 if (adjust) v = adjust_value(v);
             } else {

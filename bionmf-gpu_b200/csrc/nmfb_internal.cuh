@@ -129,6 +129,17 @@ int nmfb_fail(nmfb_ctx *ctx, int code, const char *fmt, ...);
 extern "C" int nmfb_prof_begin(nmfb_ctx *ctx, int cls);
 extern "C" int nmfb_prof_end(nmfb_ctx *ctx, int cls);
 
+// Sum of the split partials q .. q + 7 (below n) of one entry: eight loads in flight,
+// added as a tree.  One after another, 63 partials of 16 terms each (1000 x 97 k = 65)
+// had an rms error of 2.1 * 2^-24 of the update, as a tree 1.1.
+__device__ __forceinline__ float nmfb_add8(const float *part, size_t stride, uint32_t q, uint32_t n)
+{
+    float p[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) p[i] = q + i < n ? part[(q + i) * stride] : 0.0f;
+    return ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7]));
+}
+
 // ---- kernels_common.cu ----------------------------------------------------
 int nmfb_colsum(nmfb_ctx *ctx, const float *X, uint32_t rows, float *acc, int which);
 int nmfb_muldiv(nmfb_ctx *ctx, float *X, uint32_t rows, const float *part, uint32_t nsplit,

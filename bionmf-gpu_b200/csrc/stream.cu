@@ -53,9 +53,9 @@ __global__ void k_accum(float *__restrict__ aux, const float *__restrict__ part,
 {
     if (st && *(volatile const uint32_t *)&st->converged) return;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        float s = first ? 0.0f : aux[e];
-        for (uint32_t q = 0; q < nsplit; q++) s += part[q * stride + e];
-        aux[e] = s;
+        float s = 0.0f;   // this block's term, then one addition to the blocks' before
+        for (uint32_t q = 0; q < nsplit; q += 8) s += nmfb_add8(part + e, stride, q, nsplit);
+        aux[e] = first ? s : aux[e] + s;
     }
 }
 

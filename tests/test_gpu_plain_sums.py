@@ -48,3 +48,22 @@ def test_long_reductions_against_fp64(pkg, n, m, k):
         want = torch.cat([Wd[i:i + rows] * ((V[i:i + rows].double() / (Wd[i:i + rows] @ Hd.T)) @ Hd)
                           for i in range(0, n, rows)]) / Hd.sum(0)
         assert rms(e.W, want) <= RMS
+
+
+@pytest.mark.parametrize("n,m,k", [(1000, 97, 65), (8000, 1000, 100), (16000, 130, 70)])
+def test_many_partials_against_fp64(pkg, n, m, k):
+    """update_H from 63 or 64 splits of a few hundred rows at most: by the rule above their chains
+    cost (N/3)/64 < 2, and adding them in eights (7 roundings in a tree of 3, then P/8 in turn)
+    (P/8)/3 + 1 with product, division and column sum 3: rms <= sqrt((2 + 3.7 + 3) / 3) = 1.7,
+    one after another 64/3 -> 2.9."""
+    rng = np.random.default_rng(k)
+    V = rng.poisson(6.0, (n, m)).astype(np.float32)
+    W, H = (rng.random((r, k), np.float32) + np.float32(0.05) for r in (n, m))
+    with pkg.NMF(n, m, k, arm="plain") as e:
+        e.set_V(V)
+        e.set_WH(W, H)
+        e.update_H()
+        got = e.H
+    Wd, Hd = W.astype(np.float64), H.astype(np.float64)
+    want = Hd * ((V / (Wd @ Hd.T)).T @ Wd) / Wd.sum(0)
+    assert np.sqrt(np.mean((got / want - 1) ** 2)) <= 1.7 * 2.0 ** -24
