@@ -254,35 +254,50 @@ __global__ void k_conv_compare(const uint32_t *__restrict__ labels, uint32_t *__
 //
 // Bound by the FP64 pipe (64 FMA per cycle and SM): k multiply-adds an element
 // for WH and, for the divergence, a division and a logarithm (about 45 more).
-// A CTA takes 64 x 64 tiles of V in turn; 32 columns at a time of the tile's
-// rows of W and H are converted to FP64 once, in shared memory, and each
-// thread forms 4 x 4 elements of WH from them, so an element costs half a
-// shared load per multiply-add and no conversion.  (One thread per element
+// A CTA takes tiles of V in turn (OBJ_CX threads across, 256 / OBJ_CX down); up to 32
+// columns at a time of the tile's rows of W and H are converted to FP64 once, in shared
+// memory, and each thread forms 4 x 4 elements of WH from them, so an element costs half
+// a shared load per multiply-add and no conversion.  (One thread per element
 // with both rows read and converted from global memory was bound by the
 // conversions and by the division of the element index: 1344 us for
 // 12007 x 1501 at k = 20.)  WHAT selects the
 // sums: OBJ_DOTS leaves out the division and the logarithm.  Thread, CTA and
 // grid sums have fixed orders.
 enum { OBJ_DOTS = 1, OBJ_KL = 2 };
-constexpr int OBJ_T = 64;    // tile edge
+// Threads across a tile: 64 columns, or the 4 to 32 that a narrower V has.  Up to 16
+// columns the few threads that share a row of W read it themselves (H stays in shared
+// memory, k <= m <= 16).  With 64-column tiles 1000000 x 2 k = 2 took 269 us (divergence)
+// and 126 (dots), 200000 x 5 k = 3 109 and 49; now 59 and 50, 48 and 35 (a call).
+__host__ __device__ constexpr int obj_cx(uint32_t m) { return m <= 4 ? 1 : m <= 8 ? 2 : m <= 16 ? 4 : m <= 32 ? 8 : 16; }
+constexpr int obj_cols(int cx) { return 4 * cx; }
+constexpr int obj_rows(int cx) { return 4 * (256 / cx); }
 constexpr int OBJ_KC = 32;   // rank columns per shared-memory chunk
 
-template <int WHAT>
+template <int WHAT, int CX>
 __global__ void __launch_bounds__(256) k_objective(const float *__restrict__ V, size_t ldv, const float *__restrict__ W,
                                                    const float *__restrict__ H, uint32_t n, uint32_t m, uint32_t kp,
                                                    uint32_t k, double *__restrict__ part, double *__restrict__ out,
                                                    uint32_t *__restrict__ ticket)
 {
-    __shared__ __align__(16) double sW[OBJ_KC][OBJ_T + 2];   // [column][row]; 16-byte rows for the paired loads
-    __shared__ __align__(16) double sH[OBJ_KC][OBJ_T + 2];
+    constexpr int TR = obj_rows(CX), TC = obj_cols(CX);
+    constexpr bool NARROW = CX <= 4;
+    __shared__ __align__(16) double sW[NARROW ? 1 : OBJ_KC][NARROW ? 2 : TR + 2];   // [column][row]; 16-byte rows for the paired loads
+    __shared__ __align__(16) double sH[NARROW ? TC : OBJ_KC][TC + 2];
     __shared__ double red[3][8];
     __shared__ bool is_last;
-    uint32_t const tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-    uint32_t const tcols = (m + OBJ_T - 1) / OBJ_T, trows = (n + OBJ_T - 1) / OBJ_T;
+    uint32_t const tid = threadIdx.x, tx = tid % CX, ty = tid / CX;
+    uint32_t const tcols = (m + TC - 1) / TC, trows = (n + TR - 1) / TR;
     uint64_t const tiles = (uint64_t)tcols * trows;
     double sv = 0.0, sd = 0.0, kl = 0.0;
+    if (NARROW) {
+        for (uint32_t e = tid; e < TC * TC; e += 256) {
+            uint32_t const r = e / TC, c = e % TC;
+            sH[c][r] = r < m && c < k ? (double)H[(size_t)r * kp + c] : 0.0;
+        }
+        __syncthreads();
+    }
     for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        uint32_t const i0 = (uint32_t)(t / tcols) * OBJ_T, j0 = (uint32_t)(t % tcols) * OBJ_T;
+        uint32_t const i0 = (uint32_t)(t / tcols) * TR, j0 = (uint32_t)(t % tcols) * TC;
         // this thread's 4 x 4 elements of V; the leading dimension is a multiple of 32, so a
         // float4 starting below m lies in its row
         float4 v[4];
@@ -293,13 +308,35 @@ __global__ void __launch_bounds__(256) k_objective(const float *__restrict__ V, 
                                     : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
         double wh[4][4] = {};
-        for (uint32_t c0 = 0; c0 < k; c0 += OBJ_KC) {
+        if constexpr (NARROW) {   // (W's padding columns are 0)
+            for (uint32_t c0 = 0; c0 < k; c0 += 4) {
+                float4 w[4];
+#pragma unroll
+                for (int p = 0; p < 4; p++) {
+                    uint32_t const i = min(i0 + ty * 4 + p, n - 1);
+                    w[p] = *reinterpret_cast<const float4 *>(W + (size_t)i * kp + c0);
+                }
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    double h[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) h[q] = sH[c0 + c][tx * 4 + q];
+#pragma unroll
+                    for (int p = 0; p < 4; p++) {
+                        double const x = c == 0 ? w[p].x : c == 1 ? w[p].y : c == 2 ? w[p].z : w[p].w;
+#pragma unroll
+                        for (int q = 0; q < 4; q++) wh[p][q] += x * h[q];
+                    }
+                }
+            }
+        }
+        for (uint32_t c0 = 0; !NARROW && c0 < k; c0 += OBJ_KC) {
             uint32_t const kc = min((uint32_t)OBJ_KC, k - c0);
             __syncthreads();   // the previous chunk's readers are done
-            for (uint32_t e = tid; e < OBJ_T * kc; e += 256) {
+            for (uint32_t e = tid; e < TR * kc; e += 256) {
                 uint32_t const r = e / kc, c = e % kc;
                 sW[c][r] = i0 + r < n ? (double)W[(size_t)(i0 + r) * kp + c0 + c] : 0.0;
-                sH[c][r] = j0 + r < m ? (double)H[(size_t)(j0 + r) * kp + c0 + c] : 0.0;
+                if (TC >= TR || r < TC) sH[c][r] = j0 + r < m ? (double)H[(size_t)(j0 + r) * kp + c0 + c] : 0.0;
             }
             __syncthreads();
 #pragma unroll 4
@@ -465,15 +502,26 @@ int nmfb_reset_conv(nmfb_ctx *ctx, uint32_t stop_threshold)
     return NMFB_OK;
 }
 
+template <int CX>
+static auto objective_kernel(int what)
+{
+    return what == OBJ_DOTS ? k_objective<OBJ_DOTS, CX> : what == OBJ_KL ? k_objective<OBJ_KL, CX>
+                                                                         : k_objective<OBJ_DOTS | OBJ_KL, CX>;
+}
+
 static int objectives_rows(nmfb_ctx *ctx, const float *V, const float *W, uint32_t rows, int what, double out[3])
 {
-    // four CTAs per SM by registers and shared memory; dObj holds the partials of 1024
-    uint64_t const tiles = (uint64_t)((ctx->m + OBJ_T - 1) / OBJ_T) * ((rows + OBJ_T - 1) / OBJ_T);
+    // two CTAs per SM by registers (82 to 126 a thread), in two waves; dObj holds the partials of 1024
+    int const cx = obj_cx(ctx->m);
+    uint64_t const tr = obj_rows(cx), tc = obj_cols(cx), tiles = ((ctx->m + tc - 1) / tc) * ((rows + tr - 1) / tr);
     uint64_t grid = 4u * (uint64_t)ctx->sm_count;
     if (grid > tiles) grid = tiles;
     if (grid > 1024) grid = 1024;
-    auto const kern = what == OBJ_DOTS ? k_objective<OBJ_DOTS> : what == OBJ_KL ? k_objective<OBJ_KL>
-                                                                                : k_objective<OBJ_DOTS | OBJ_KL>;
+    auto const kern = cx == 1   ? objective_kernel<1>(what)
+                      : cx == 2 ? objective_kernel<2>(what)
+                      : cx == 4 ? objective_kernel<4>(what)
+                      : cx == 8 ? objective_kernel<8>(what)
+                                : objective_kernel<16>(what);
     kern<<<(unsigned)grid, 256, 0, ctx->stream>>>(V, ctx->ldv, W, ctx->dH, rows, ctx->m, ctx->kp, ctx->k, ctx->dObj,
                                                  ctx->dObj + 3 * 1024, ctx->dObjTicket);
     NMFB_LAUNCH_CHECK(ctx);
