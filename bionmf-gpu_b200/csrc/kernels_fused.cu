@@ -58,6 +58,7 @@
 #include <cuda_bf16.h>
 #include <float.h>
 #include <cudaTypedefs.h>
+#include <type_traits>
 
 using nmfb::ConvState;
 using namespace nmfb_tc;
@@ -400,32 +401,54 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                 uint32_t const oy = s * (G::Y1STAGE >> 4);
                 bool const last = c1 + 1 == TB;   // the row block's last tile
                 if (elect_one()) {
-                    // MMA1, K = KP: D = the small terms, then += Xh Yh^T (TF32, k-steps of 8 per
-                    // column block).  Small terms: [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T
-                    // (K = 2 KP, k-steps of 16: the first KP / 16 read bf16(Yl), the rest bf16(Y)),
-                    // or Xh Yl^T + Xl Yh^T in TF32.
+                    // MMA1, K = KP: D = Xh Yh^T (TF32, k-steps of 8 per column block) and the small
+                    // terms [bf16(Xh) | bf16(Xl)] [bf16(Yl) ; bf16(Y)]^T (K = 2 KP, k-steps of 16:
+                    // the first KP / 16 read bf16(Yl), the rest bf16(Y)), or Xh Yl^T + Xl Yh^T in TF32.
+                    // Each MMA truncates its FP32 sums, so D comes out a little small, R = V / D
+                    // large and MMA2's sum small again: the two offset each other.  MMA2 has
+                    // more steps, so up to rank 32 the small terms come last here, where a step
+                    // truncates most, and at 64 first: rms error of one update / 2^-24 with
+                    // them first / last 3.8 / 2.2 (20000 x 1000 k = 16), 3.5 / 2.1
+                    // (12007 x 1501 k = 20), 3.0 / 2.0 (60000 x 5000 k = 32) and
+                    // 1.8 / 3.8 (40009 x 3001 k = 50).
                     constexpr int KPB = G::CB / 8;     // k-steps per swizzle column block
-                    if (NTERMS == 3 && G::LO32) {
-                        mma_ts<false>(dcol, xh, desc_at(dYB0, oy), IDESC1);
-                        mma_ts<true>(dcol, xh + KP, desc_at(dY0, oy), IDESC1);
+                    auto const main_term = [&](auto sum) {   // sum: added to D
 #pragma unroll
-                        for (int ks = 1; ks < KP / 8; ks++) {
-                            mma_ts<true>(dcol, xh + ks * 8, desc_at(dYB0, oy + ks * 2), IDESC1);
-                            mma_ts<true>(dcol, xh + KP + ks * 8, desc_at(dY0, oy + ks * 2), IDESC1);
+                        for (int ks = 0; ks < KP / 8; ks++) {
+                            uint64_t const b = desc_at(dY0, oy + (((ks / KPB) * G::YBLK + (ks % KPB) * 32) >> 4));
+                            if (ks == 0)
+                                mma_ts<decltype(sum)::value>(dcol, xh, b, IDESC1);
+                            else
+                                mma_ts<true>(dcol, xh + ks * 8, b, IDESC1);
                         }
-                    } else if (NTERMS == 3) {
-                        mma_ts_bf16<false>(dcol, xh + KP, desc_at(dYB0, oy), IDESC1B);
+                    };
+                    auto const small_terms = [&](auto sum) {
+                        if constexpr (G::LO32) {
+                            mma_ts<decltype(sum)::value>(dcol, xh, desc_at(dYB0, oy), IDESC1);
+                            mma_ts<true>(dcol, xh + KP, desc_at(dY0, oy), IDESC1);
 #pragma unroll
-                        for (int j = 1; j < KP / 8; j++)
-                            mma_ts_bf16<true>(dcol, xh + KP + j * 8,
-                                              desc_at(dYB0, oy + (((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4)),
-                                              IDESC1B);
+                            for (int ks = 1; ks < KP / 8; ks++) {
+                                mma_ts<true>(dcol, xh + ks * 8, desc_at(dYB0, oy + ks * 2), IDESC1);
+                                mma_ts<true>(dcol, xh + KP + ks * 8, desc_at(dY0, oy + ks * 2), IDESC1);
+                            }
+                        } else {
+                            mma_ts_bf16<decltype(sum)::value>(dcol, xh + KP, desc_at(dYB0, oy), IDESC1B);
+#pragma unroll
+                            for (int j = 1; j < KP / 8; j++)
+                                mma_ts_bf16<true>(dcol, xh + KP + j * 8,
+                                                  desc_at(dYB0, oy + (((j / (KP / 16)) * G::YBB + (j % (KP / 16)) * 32) >> 4)),
+                                                  IDESC1B);
+                        }
+                    };
+                    if constexpr (NTERMS != 3) {
+                        main_term(std::false_type());
+                    } else if constexpr (KP == 64) {
+                        small_terms(std::false_type());
+                        main_term(std::true_type());
+                    } else {
+                        main_term(std::false_type());
+                        small_terms(std::true_type());
                     }
-                    mma_ts<NTERMS == 3>(dcol, xh, desc_at(dY0, oy), IDESC1);
-#pragma unroll
-                    for (int ks = 1; ks < KP / 8; ks++)
-                        mma_ts<true>(dcol, xh + ks * 8, desc_at(dY0, oy + (((ks / KPB) * G::YBLK + (ks % KPB) * 32) >> 4)),
-                                     IDESC1);
                     tc_commit(&dfull[db]);
                     tc_commit(&y1empty[s]);
                     if (last) tc_commit(&xfree[xs % G::NXB]);
