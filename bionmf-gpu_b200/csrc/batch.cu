@@ -9,6 +9,7 @@
 #include <stdarg.h>
 #include <stdlib.h>
 #include <algorithm>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -33,8 +34,9 @@ struct nmfb_batch {
     Problem *dProbs;
     uint32_t *dOrder, *dQueue;
     uint32_t **dLabelPtrs;
-    uint32_t *dCounts;                    // workspaces of nmfb_batch_consensus
+    uint32_t *dCounts;                    // workspaces of nmfb_batch_consensus, held under summary_lock
     double *dSummary;
+    std::mutex summary_lock;
     int v_set, wh_set;
     cudaEvent_t ev0, ev1;
     float last_ms;
@@ -395,7 +397,9 @@ int nmfb_batch_consensus(nmfb_batch *b, uint32_t k, uint32_t *counts, uint32_t *
     uint32_t const m = b->m;
     size_t const mm = (size_t)m * m;
     // Workspaces, allocated on the first call that needs them and kept: the counts with
-    // the selection, and the linkage's.
+    // the selection, and the linkage's.  One call at a time has them, until its results
+    // are on the host.
+    std::lock_guard<std::mutex> const held(b->summary_lock);
     cudaError_t e = cudaSuccess;
     if (!b->dCounts) e = cudaMalloc(&b->dCounts, (mm + b->nprob) * sizeof(uint32_t));
     if (e == cudaSuccess && cophenetic && !b->dSummary)

@@ -266,7 +266,8 @@ int nmfb_batch_get_WH(nmfb_batch *b, uint32_t p, float *W, size_t ldw, float *H,
 /* Consensus of the problems of rank k: counts (m x m, may be NULL) = number of
  * those runs that co-cluster each sample pair; *nruns = their number;
  * *cophenetic (may be NULL) = cophenetic correlation of average-linkage
- * clustering of 1 - counts / nruns. */
+ * clustering of 1 - counts / nruns.  Several threads may ask one batch at the
+ * same time (their calls follow one another). */
 int nmfb_batch_consensus(nmfb_batch *b, uint32_t k, uint32_t *counts, uint32_t *nruns, double *cophenetic);
 
 /* ---------------------------------------------------------------------------
