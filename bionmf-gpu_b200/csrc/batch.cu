@@ -364,20 +364,34 @@ int nmfb_batch_get_WH(nmfb_batch *b, uint32_t p, float *W, size_t ldw, float *H,
     uint32_t const k = b->ranks[p], ks = ks_of(k);
     if ((W && ldw < k) || (H && ldh < k)) return bfail(b, NMFB_EINVAL, "leading dimension below k");
     BTRY(b, cudaSetDevice(b->device));
-    // Through a page-locked staging buffer in one DMA each (a pitched copy into
-    // pageable memory moves one short row at a time).
+    // Through page-locked staging buffers of at most 8 MB, one DMA each, the next while
+    // this one's rows are copied out (a pitched copy into pageable memory moves one short
+    // row at a time).
     auto const fetch = [&](float *dst, size_t ld, const float *src, uint32_t rows) -> cudaError_t {
-        size_t const bytes = (size_t)rows * ks * sizeof(float);
-        float *const stage = (float *)nmfb_stage_get(bytes);
-        if (!stage)
-            return cudaMemcpy2D(dst, ld * sizeof(float), src, ks * sizeof(float), k * sizeof(float), rows,
-                                cudaMemcpyDeviceToHost);
-        cudaError_t e = cudaMemcpyAsync(stage, src, bytes, cudaMemcpyDeviceToHost, b->stream);
-        cudaError_t const es = cudaStreamSynchronize(b->stream);
-        if (e == cudaSuccess) e = es;
-        if (e == cudaSuccess)
-            for (uint32_t r = 0; r < rows; r++) memcpy(dst + (size_t)r * ld, stage + (size_t)r * ks, k * sizeof(float));
-        nmfb_stage_put(stage);
+        size_t const step = ks, row = step * sizeof(float), len = k * sizeof(float);
+        uint32_t const most = (uint32_t)((8u << 20) / row), chunk = rows < most ? rows : most;
+        float *stage[2] = {(float *)nmfb_stage_get(chunk * row), rows > chunk ? (float *)nmfb_stage_get(chunk * row) : nullptr};
+        cudaError_t e = cudaSuccess;
+        if (!stage[0] || (rows > chunk && !stage[1])) {
+            e = cudaMemcpy2D(dst, ld * sizeof(float), src, row, k * sizeof(float), rows, cudaMemcpyDeviceToHost);
+        } else {
+            auto const copy = [&](uint32_t r0, float *to) {
+                return cudaMemcpyAsync(to, src + (size_t)r0 * ks, std::min(chunk, rows - r0) * row, cudaMemcpyDeviceToHost, b->stream);
+            };
+            e = copy(0, stage[0]);
+            for (uint32_t r0 = 0, c = 0; r0 < rows; r0 += chunk, c ^= 1) {
+                cudaError_t const es = cudaStreamSynchronize(b->stream);   // this chunk is there, and no copy in flight
+                if (e == cudaSuccess) e = es;
+                if (e != cudaSuccess) break;
+                uint32_t const nr = std::min(chunk, rows - r0);
+                if (rows - r0 > nr) e = copy(r0 + nr, stage[c ^ 1]);
+                float *to = dst + (size_t)r0 * ld;
+                const float *from = stage[c];
+                for (uint32_t r = 0; r < nr; r++, to += ld, from += step) memcpy(to, from, len);
+            }
+        }
+        nmfb_stage_put(stage[0]);
+        nmfb_stage_put(stage[1]);
         return e;
     };
     if (W) BTRY(b, fetch(W, ldw, b->dW + b->woff[p], b->n));

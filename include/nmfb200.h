@@ -86,9 +86,11 @@ uint64_t nmfb_context_bytes(int device, uint32_t n, uint32_t m, uint32_t k, int 
 
 /* Context device memory comes from a library-owned stream-ordered pool per
  * device (cudaMallocFromPoolAsync), and page-locked host staging buffers (for
- * uploads and downloads, up to 8 MB each, one or two per call in flight) from
- * a process-wide pool, so contexts can be created, fed and destroyed while
- * others compute without synchronising the device.  Freed memory stays
+ * uploads and downloads, one or two per call in flight, of power-of-two sizes:
+ * up to 8 MB for V and for a batch's factors, a whole factor of a context, a
+ * whole request of the device queue) from a process-wide pool, so contexts can
+ * be created, fed and destroyed while others compute without synchronising the
+ * device.  Freed memory stays
  * cached in the pools for the next context; this returns the device pool's
  * memory to the driver (after synchronising the device) and frees the
  * staging buffers no call holds.  No counterpart in the reference. */
