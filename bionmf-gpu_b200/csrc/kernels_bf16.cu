@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
 #pragma unroll 1
             for (int ch = 0; ch < CW / 16; ch++) {
                 int const col0 = grp * CW + ch * 16;
-                uint32_t d[32];
+                uint32_t d[16];
                 float v[16];
                 tmem_ld16(lane_addr + G::DB0 + b * BR + col0, d);
                 if (HSIDE) {
@@ -481,11 +481,11 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
             tc_fence_after();
 #pragma unroll
             for (int c0 = 0; c0 < KC; c0 += 16) {
-                uint32_t a[32], a2[32];
+                uint32_t a[16], a2[16];
                 tmem_ld16(lane_addr + bp * G::ACCW + k0 + c0, a);
                 if (SPLIT2) tmem_ld16(lane_addr + bp * G::ACCW + KP + k0 + c0, a2);
-                tmem_wait_ld_dep16(a);
-                if (SPLIT2) tmem_wait_ld_dep16(a2);
+                tmem_wait_ld_dep(a);
+                if (SPLIT2) tmem_wait_ld_dep(a2);
 #pragma unroll
                 for (int c = 0; c < 16; c++)
                     sum[c0 + c] += SPLIT2 ? __uint_as_float(a[c]) + __uint_as_float(a2[c]) : __uint_as_float(a[c]);

@@ -512,8 +512,8 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
                 int const col0 = grp * CW + ch * 16;                          // first tile column of the chunk
                 uint32_t const dcol = G::DA0 + b * BR + col0;                 // its columns of D
                 uint32_t const rlcol = G::RL0 + (t % G::NRL) * (BR / 2) + (col0 / 16) * 8;  // and of bf16(Rl)
-                uint32_t d[32];   // D, then the TF32 hi part of R
-                uint32_t v[32];   // V, then the lo part of R
+                uint32_t d[16];   // D, then the TF32 hi part of R
+                uint32_t v[16];   // V, then the lo part of R
                 tmem_ld16(lane_addr + dcol, d);
                 if (HSIDE) {
                     // V tile [BR rows][128 cols], row-major; this thread's column = row.
@@ -696,11 +696,11 @@ __global__ void __launch_bounds__(Geo<KP>::NTHR, 1)
             // to the running one in one rounding.
 #pragma unroll
             for (int c0 = 0; c0 < KC; c0 += 16) {
-                uint32_t a[32], a2[32];
+                uint32_t a[16], a2[16];
                 tmem_ld16(lane_addr + bp * ACC_COLS + k0 + c0, a);
                 if (NTERMS == 3) tmem_ld16(lane_addr + bp * ACC_COLS + KP + k0 + c0, a2);
-                tmem_wait_ld_dep16(a);
-                if (NTERMS == 3) tmem_wait_ld_dep16(a2);
+                tmem_wait_ld_dep(a);
+                if (NTERMS == 3) tmem_wait_ld_dep(a2);
 #pragma unroll
                 for (int c = 0; c < 16; c++)
                     sum[c0 + c] += NTERMS == 3 ? __uint_as_float(a[c]) + __uint_as_float(a2[c]) : __uint_as_float(a[c]);
