@@ -18,6 +18,12 @@ using nmfb_tc::tf32_rna;
 
 constexpr uint32_t FIN_RB = 32;    // rows of X per k_finish CTA
 
+// How the half-iteration that updates W (or H) is dealt out.
+inline nmfb_tc::TileSplit plan_of(const nmfb_ctx *ctx, bool w)
+{
+    return nmfb_tc::plan_tiles(w ? ctx->n : ctx->m, w ? ctx->m : ctx->n, 64, (uint32_t)ctx->sm_count, ctx->part_items / ctx->kp);
+}
+
 // k_finish's launch shape for a factor of `rows` rows: KP / 4 threads per row
 // of a 32-row set, RPT row sets per CTA (each thread takes one row of each),
 // and enough CTAs to cover every 64-row block of the split copies (rows past

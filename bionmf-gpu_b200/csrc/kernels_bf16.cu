@@ -67,15 +67,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         : "memory");
 }
 
-// Two floats to a BF16 pair (round to nearest even); `first` in the low half,
-// i.e. at the lower address.
-__device__ __forceinline__ uint32_t pack_bf16x2(float first, float second)
-{
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(second), "f"(first));
-    return r;
-}
-
 // MODE 0: BF16 x BF16 in both contractions; 1: split-BF16 WH denominator;
 // 2: split-BF16 in both contractions.
 template <int KP, int MODE>
@@ -445,10 +436,10 @@ __global__ void __launch_bounds__(GeoB<KP, MODE>::NTHR, 1)
                     // R = V * (1/WH); a zero WH of the data behaves as in the reference's division.
                     float const r0 = v[c] * rcp_approx(__uint_as_float(d[c]));
                     float const r1 = v[c + 1] * rcp_approx(__uint_as_float(d[c + 1]));
-                    pk[c / 2] = pack_bf16x2(r0, r1);
+                    pk[c / 2] = fin_bf16x2(r0, r1);
                     if (SPLIT2) {
                         float const h0 = __uint_as_float(pk[c / 2] << 16), h1 = __uint_as_float(pk[c / 2] & 0xffff0000u);
-                        pl[c / 2] = pack_bf16x2(r0 - h0, r1 - h1);
+                        pl[c / 2] = fin_bf16x2(r0 - h0, r1 - h1);
                     }
                 }
                 // R over the 16 columns of D it came from: Rh packed in the first 8, Rl in the others.
@@ -579,25 +570,19 @@ int set_attrs_b(nmfb_ctx *ctx)
     return rc;
 }
 
-// How the half-iteration that updates W (or H) is dealt out.
-TileSplit plan_of_b(const nmfb_ctx *ctx, bool w)
-{
-    return plan_tiles(w ? ctx->n : ctx->m, w ? ctx->m : ctx->n, 64, (uint32_t)ctx->sm_count, ctx->part_items / ctx->kp);
-}
-
 template <bool HSIDE, int KP, int MODE>
 int launch_b(nmfb_ctx *ctx, const MapsB &maps, PlanB *plan)
 {
     using G = GeoB<KP, MODE>;
-    static_assert(G::BR == 64, "plan_of_b");
+    static_assert(G::BR == 64, "plan_of");
     ArgsB args;
     args.O = HSIDE ? ctx->m : ctx->n;
     args.R = HSIDE ? ctx->n : ctx->m;
-    args.ts = plan_of_b(ctx, !HSIDE);
+    args.ts = plan_of(ctx, !HSIDE);
     if ((size_t)args.ts.slots * args.O * KP > ctx->part_items)
         return nmfb_fail(ctx, NMFB_EINVAL, "bf16 arm: partial buffer too small (%u slots)", args.ts.slots);
     args.csy.cs = HSIDE ? plan->dCsW : plan->dCsH;
-    args.csy.nblk = fin_blocks(args.R, fin_rpt(plan_of_b(ctx, HSIDE).slots));
+    args.csy.nblk = fin_blocks(args.R, fin_rpt(plan_of(ctx, HSIDE).slots));
     args.csy.acc = HSIDE ? ctx->dAccW : ctx->dAccH;
     args.part = ctx->dPart;
     args.err = plan->dErr;
@@ -678,7 +663,7 @@ int launch_finish_b(nmfb_ctx *ctx, bool w, bool update, int adjust)
     fa.O = w ? ctx->n : ctx->m;
     __nv_bfloat16 *xs = w ? plan->wsplit : plan->hsplit;
     size_t const sz = (size_t)fa.O * KP;
-    fa.ts = plan_of_b(ctx, w);
+    fa.ts = plan_of(ctx, w);
     fa.k = ctx->k;
     fa.adjust = adjust;
     fa.part = update ? ctx->dPart : nullptr;

@@ -807,12 +807,6 @@ struct FusedPlan {
 #endif
 };
 
-// How the half-iteration that updates W (or H) is dealt out.
-TileSplit plan_of(const nmfb_ctx *ctx, bool w)
-{
-    return plan_tiles(w ? ctx->n : ctx->m, w ? ctx->m : ctx->n, 64, (uint32_t)ctx->sm_count, ctx->part_items / ctx->kp);
-}
-
 // k_finish on W (or H): its update from the partials, or, with update = false,
 // only its split copies and column-sum partials.
 template <int KP>
