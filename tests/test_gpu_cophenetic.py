@@ -1,6 +1,6 @@
 """GPU test of the consensus summary against a direct average linkage: many tied
 distances (few runs), no ties, two samples, one cluster, more samples than a
-block has threads per merge step.  The merges take the lowest pair of slots on
+merge step scans at a time.  The merges take the lowest pair of slots on
 ties and the heights are the same FP64 operations in the same order, so the
 correlation agrees to the rounding of its sums (at most m^2 terms: 1e-10).
 """

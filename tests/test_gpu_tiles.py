@@ -24,12 +24,12 @@ def _updates(V, W, H):
 @pytest.mark.parametrize("arm", ["fused", "bf16x3"])
 @pytest.mark.parametrize("n,m,k,sms", [
     (129, 65, 3, 0),        # two row blocks, ragged tiles on both sides
-    (129, 65, 30, 0),       # (the FP32 arm's tensor-core kernels from here on)
+    (129, 65, 30, 0),       # (the FP32 arm's tensor-core kernels)
     (2000, 33, 5, 0),       # one-tile row blocks (W side), one CTA each
-    (2000, 33, 27, 0),
+    (2000, 33, 27, 0),      # (the FP32 arm's tensor-core kernels from here on)
     (3000, 40, 16, 5),      # one-tile row blocks, several to a CTA
     (5000, 130, 20, 7),     # three-tile row blocks crossed by runs of every phase
-    (9000, 70, 33, 3),      # rank 64 instantiation: 32-column tiles, a single X buffer
+    (9000, 70, 33, 3),      # rank 64 instantiation: 64-column tiles, a single X buffer
     (700, 9000, 17, 2),     # long reductions: partials every 128 tiles
     (8320, 300, 2, 1),      # one CTA does everything
     (16400, 129, 64, 148),  # partial sums that end on a multiple of 128 tiles
