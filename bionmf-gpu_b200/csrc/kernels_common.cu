@@ -254,7 +254,7 @@ __global__ void k_conv_compare(const uint32_t *__restrict__ labels, uint32_t *__
 //
 // Bound by the FP64 pipe (64 FMA per cycle and SM): k multiply-adds an element
 // for WH and, for the divergence, a division and a logarithm (about 45 more).
-// A CTA takes tiles of V in turn (OBJ_CX threads across, 256 / OBJ_CX down); up to 32
+// A CTA takes tiles of V in turn (CX threads across, 256 / CX down); up to 32
 // columns at a time of the tile's rows of W and H are converted to FP64 once, in shared
 // memory, and each thread forms 4 x 4 elements of WH from them, so an element costs half
 // a shared load per multiply-add and no conversion.  (One thread per element

@@ -40,8 +40,11 @@ extern "C" {
 
 /* Update kernels ("arms").  All arms run the same method; they differ only
  * in how the two n x m x k contractions of a half-iteration are evaluated. */
-#define NMFB_ARM_FUSED 0  /* fused half-iteration (one launch): TF32 hi x (hi + lo) products plus the
-                           * lo x y term as a BF16 product, FP32 accumulation (FP32-accurate, ~2^-20 per product) */
+#define NMFB_ARM_FUSED 0  /* fused half-iteration on tensor cores: TF32 hi x (hi + lo) products plus the lo x y
+                           * term as a BF16 product (TF32 up to rank 16), FP32 accumulation (FP32-accurate, ~2^-20
+                           * per product).  Small matrices (rank <= 24, H of at most 8 KB, few rows per SM; the
+                           * rule stands in csrc/small.cu) run FP32 SIMT kernels without tensor cores or device
+                           * waits instead, two launches an iteration. */
 #define NMFB_ARM_PLAIN 1  /* unfused FP32 SIMT kernels mirroring the reference's 5 steps */
 #define NMFB_ARM_FUSED_TF32 2 /* fused, 1xTF32 denominator (reduced precision) */
 #define NMFB_ARM_BF16 3       /* fused, BF16 operands, FP32 accumulation (reduced precision) */
@@ -208,9 +211,16 @@ int nmfb_set_wait_limit(nmfb_ctx *ctx, uint64_t ns);
  * The fused arms split each half-iteration's reduction so that one wave of
  * CTAs fills that many SMs; a smaller figure leaves room for the kernels of
  * other contexts on other streams (many small solves served side by side)
- * and gives each CTA a longer run of tiles.  The split count, and with it the
- * summation order, depends on this figure and the sizes only.  No counterpart
- * in the reference, which runs one factorisation per process. */
+ * and gives each CTA a longer run of tiles.  A large context without a limit
+ * holds every SM for the whole of each of its main kernels, and others run in
+ * the gaps between them: beside a 60000 x 2000 k = 20 one, a 5000 x 38 k = 3
+ * context made 511 runs of 20 iterations a second, with the large one limited
+ * to 132 SMs 1665 and to 111 SMs 2770 (the large one 204, 189 and 173).
+ * The split count, and with it the summation order, depends on this figure and
+ * the sizes only, and so does whether a context counts as small (rows per SM):
+ * a limit can move it from the SIMT kernels of small matrices to the tensor
+ * cores, whose results agree to FP32 rounding.  No counterpart in the
+ * reference, which runs one factorisation per process. */
 int nmfb_set_sm_limit(nmfb_ctx *ctx, uint32_t sms);
 
 /* ---------------------------------------------------------------------------
