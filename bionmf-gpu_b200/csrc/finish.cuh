@@ -248,13 +248,15 @@ __global__ void __launch_bounds__(FIN_RB * KP / 4, 128 / KP) k_finish(const Fini
 // k_finish for the factor of a.O rows, with the row sets per thread that its
 // partial count calls for (the block count is fin_blocks(a.O, fin_rpt(a.ts.slots))).
 // Chained to the main kernel only where that has fewer than FIN_CHAIN_TILES tiles to
-// a CTA: a dependent launch waiting behind a long kernel keeps the kernels of other
-// streams from starting, whatever SMs are free (5000 x 38 k = 3 beside a 60000 x 2000
-// k = 20 context limited to 111 SMs: 370 runs of 20 iterations a second, ordinary 2790),
-// and its CTAs, placed early, wait beside the last main ones. Alone, us an iteration
-// chained / ordinary: 4 tiles (4700 x 1000 k = 12) 23.5 / 24.6, 8 (9400 x 1000 k = 12)
-// 32.6 / 31.9, 11 (20000 x 600) 43.0 / 39.9, 17 (20000 x 1000 k = 16) 51.9 / 49.0. What
-// precedes the copies of a factor that is not updated (a.part null) is a k_finish, too.
+// a CTA: a dependent launch that is let in early and waits behind a long kernel keeps
+// the kernels of other streams from starting, whatever SMs are free (5000 x 38 k = 3
+// beside a 60000 x 2000 k = 20 context limited to 111 SMs: 370 runs of 20 iterations a
+// second, ordinary 2770), and its CTAs, placed early, wait beside the last main ones.
+// Alone, us an iteration chained / ordinary: 4 tiles (4700 x 1000 k = 12) 23.5 / 24.6,
+// 8 (9400 x 1000 k = 12) 32.6 / 31.9, 11 (20000 x 600) 43.0 / 39.9, 17 (20000 x 1000
+// k = 16) 51.9 / 49.0.  The copies of a factor that is not updated (a.part null) follow a
+// k_finish, or work of the caller that lets nothing in early: chained (behind a 1 ms
+// kernel other streams run on).
 constexpr uint32_t FIN_CHAIN_TILES = 8;
 template <int KP, int BR, int LAYOUT>
 cudaError_t fin_launch(const FinishArgs &a, cudaStream_t s)

@@ -73,7 +73,8 @@ inline TileSplit plan_tiles(uint32_t O, uint32_t R, uint32_t br, uint32_t sms, s
 // global memory calls chain_wait first, and what the kernel just before wrote is
 // read through L2.  It hides a launch and the prologue
 // (barriers, tensor-memory allocation), about 2 us a launch.  Not for a launch behind
-// a long kernel: while it waits, other streams' kernels do not start (see fin_launch).
+// a long kernel that calls chain_next early: while it waits, other streams' kernels do
+// not start (see fin_launch).
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
