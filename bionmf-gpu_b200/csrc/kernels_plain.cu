@@ -280,9 +280,9 @@ int launch_red(nmfb_ctx *ctx, const float *Q, bool trans, const float *F, uint32
         return nmfb_fail(ctx, NMFB_EINVAL, "partial buffer too small (%u splits of %u rows)", p.nsplit, nout);
     dim3 const g((nout + TM - 1) / TM, p.nsplit, (ctx->k + TN - 1) / TN);
     auto const kern = p.chunk > p.piece ? (trans ? k_red<true, true> : k_red<false, true>)
-                                          : (trans ? k_red<true, false> : k_red<false, false>);
-    NMFB_CUDA_TRY(ctx, launch_chained(kern, g, 128, 0, ctx->stream, Q, ctx->ldv, F, nout, nred, ctx->kp, p.chunk, p.piece, ctx->dPart,
-                                      ctx->dState));
+                                        : (trans ? k_red<true, false> : k_red<false, false>);
+    NMFB_CUDA_TRY(ctx, launch_chained(kern, g, 128, 0, ctx->stream, Q, ctx->ldv, F, nout, nred, ctx->kp, p.chunk, p.piece,
+                                      ctx->dPart, ctx->dState));
     NMFB_LAUNCH_CHECK(ctx);
     *nsplit = p.nsplit;
     return NMFB_OK;
