@@ -422,9 +422,10 @@ uint64_t nmfb_context_bytes(int device, uint32_t n, uint32_t m, uint32_t k, int 
     } else if (arm == NMFB_ARM_PLAIN) {
         b += nv;                                                       // WH
     } else {
-        b += 4 + (2 * ((uint64_t)n + m) + ((n + 31) / 32 + (m + 31) / 32) * 64) * kp * 4;   // TF32 splits
-        if (arm >= NMFB_ARM_BF16)
-            b += (2 * ((uint64_t)n + m) + ((n + 63) / 64 + (m + 63) / 64) * 128) * kp * 2;  // BF16 splits
+        uint64_t const blk32 = (uint64_t)(n + 31) / 32 + (m + 31) / 32, blk64 = (uint64_t)(n + 63) / 64 + (m + 63) / 64;
+        uint64_t const sums = 2 * blk64 * kp * 8;                          // k_finish's column-sum partials
+        b += 4 + (2 * ((uint64_t)n + m) + blk32 * 64 + blk64 * 32) * kp * 4 + sums;   // TF32 splits
+        if (arm >= NMFB_ARM_BF16) b += (2 * ((uint64_t)n + m) + blk64 * 128) * kp * 2 + sums;   // BF16 splits
     }
     return b + 32ull * (2u << 20);   // allocation granularity slack for ~32 buffers
 }
